@@ -5,16 +5,16 @@
 //                    (1 B read + 1/8 B written per voxel, four bytes per SWAR step); the validating
 //                    form also checks the mask (values 0/1, both classes present) with
 //                    warp-aggregated counters.
-//   2. k_edt_zy    : one CTA per (32-wide z chunk, x plane, polarity), lanes = z columns.  For every
-//                    y line it finds the nearest site along z from the line's bit words (clz/ffs over
-//                    the chunk's own word, a ballot over the other words) into shared memory, then
-//                    runs the y pass g(y,z) = min_y' dz(y',z)^2 + (y-y')^2 as an exact lower
-//                    envelope (below), banded over the CTA's warps.  Writes int32 g (4 B/voxel).
+//   2. k_edt_zy    : one CTA per (32-wide z chunk, x plane, polarity).  A lane per y line fills the
+//                    chunk's squared z distances from the line's bit words into shared memory; then,
+//                    lanes = z columns, the y pass g(y,z) = min_y' dz(y',z)^2 + (y-y')^2 as an exact
+//                    minimum over groups of rows, most of them ruled out by a bound (below).  Writes
+//                    float32 g (integers below 2^22; 4 B/voxel); a plane without a site is filled.
 //   3. k_edt_x     : one CTA per (z chunk, y row, polarity): stages the nx x 32 column block of g in
-//                    shared memory with cp.async (coalesced 128 B rows, every load in flight at
-//                    once), runs the same envelope along x in place and writes the final int32
-//                    (4 B/voxel); the paired form runs both polarities, then k_edt_signed turns the
-//                    two squared distances into the correctly rounded signed float32.
+//                    shared memory with cp.async (every load in flight at once), runs the same pass
+//                    along x and writes the final int32 (4 B/voxel); the paired form runs both
+//                    polarities, then k_edt_signed turns the two squared distances into the correctly
+//                    rounded signed float32.
 // Global traffic per voxel and polarity: 1 (mask) + 4 + 4 (g round trip) + 4 (output) + 1/4 (bit
 // words, mostly L2) bytes -- the 13 B/voxel algorithmic figure.
 //
@@ -30,7 +30,7 @@
 
 namespace {
 
-constexpr int kMaxAxis = 512;            // hull entries pack a site index < 2^11 and c < 2^21; smem holds 512 x 32
+constexpr int kMaxAxis = 512;  // the reference's bound; 512 rows of a column block fit three CTAs per SM
 
 struct Counters {
     unsigned long long ones;     // mask bytes equal to 1
@@ -110,376 +110,393 @@ void launch_bits(int grid, cudaStream_t stream, const uint8_t* mask, uint32_t* b
 }
 
 // ------------------------------------------------------------------------------------------
-// Exact 1-D min-plus along a column, out(q) = min_s f(s) + (q - s)^2, by lower envelopes.
+// Exact 1-D min-plus along a column, out(q) = min_s f(s) + (q - s)^2, by pruned groups.
 //
-// Site s contributes the parabola P_s(q) = c_s - 2 q s + q^2 with c_s = f(s) + s^2, so out(q) is the
-// lower envelope of lines c_s - 2 q s plus q^2: the sites that matter are the vertices of the lower
-// convex hull of the points (s, c_s), and site b between a and u is never strictly lowest exactly
-// when (c_b - c_a)(u - b) >= (c_u - c_b)(b - a) -- an integer test, no division (the reference's
-// envelope intersects parabolas with floor division instead, edt_persistent_pair_v1/edt.cu:12-29).
-// Sites with no finite value (the sentinel) never win against a finite one and are left out.
+// A CTA owns 32 adjacent columns (lanes) over the whole axis, staged in shared memory as float32 rows
+// (every value is an integer below 2^22, so float32 holds it and every sum below exactly).  Rows are
+// taken kGroup at a time: `mins` keeps each group's smallest f per column and `low` over all columns,
+// and a warp works out kGroup consecutive outputs (a strip) of its 32 columns at once.  A group at
+// distance d (nearest row to nearest output) can lower an output of a column only where the column's
+// min f + d^2 lies below the largest of its outputs so far, so every other group is passed over and the
+// result is the full minimum.  The strip's own group comes first, the nearest kNear on each side next
+// (one test per column and a vote each); of the rest, lanes take a group each and test it with `low`
+// against the largest output of all columns, the lowest bound is evaluated first, and what remains
+// below the new largest output follows -- a site hundreds of rows away costs a few groups, not all
+// those in between.
 //
-// A CTA owns 32 adjacent columns (lanes) over the whole axis, staged in shared memory as rows of
-// 32 words (row r holds f(r) of the 32 columns: 128 B, conflict-free per lane); its kBandWarps
-// warps split the axis into bands:
-//   1. stage : f of the band's rows lands in the band's own rows of the array (cp.async from global
-//              memory in the x pass; computed from the bit words in the zy pass);
-//   2. build : each warp runs the hull stack over its band's rows, one stack per lane, in place --
-//              stack entry k overwrites row r0 + k, never beyond the row being read;
-//   3. merge : pairwise joins of band groups in log2(kBandWarps) rounds -- the bridge between two
-//              x-separated lower hulls trims a suffix of the left one and a prefix of the right one --
-//              leaving each band a contiguous surviving range [lo, hi];
-//   4. output: each warp finds the hull vertex covering its first target (band scan + binary search)
-//              and walks the hull forward over its targets, one compare per step.
-// Values are exact integers: c < 2^21 and |products| < 2^31 for axes up to 512.
+// Inside a group, output k and site i (both counted in their group, D = first output - first site) meet
+// at f + (D - i)^2 + 2 k (D - i) + k^2: per two sites one packed square and one FMA per output (FFMA2 on
+// the pair of sites), whose two results and the running value go through one three-operand minimum.
+// k^2 is added at the end.  76 instructions for 64 pairs; pairing the outputs instead of the sites,
+// which needs every site's terms twice, issued about 175.
+//
+// Sites without a finite value carry the sentinel, which a finite value always beats and which stays
+// the result where the whole column has none.
+//
+// Bound: instruction issue (70 % of the issue slots; the FMA and ALU pipes half busy each, DRAM a
+// fifth).  A lower envelope built as a hull per column (one push, its pops and one walk step per voxel,
+// band hulls joined pairwise) took 107 (x) and 149 (zy) warp instructions per 32 voxels of the 512^3
+// obstacle grid (2000 boxes, 8 % filled), its loops diverging over the lanes; here it is 74 and 92, and
+// the work depends on the data only through votes: x 637 -> 402 us, zy 858 -> 545 us, the transform
+// 1515 -> 979 us (30 % random voxels 1640 -> 772, one box edge or ball far from most voxels 0 - 40 %
+// less).  The hulls remain faster only where a smooth surface lies hundreds of voxels away from most of
+// the grid along its diagonal (a half-space x + y + z < 350 of 512^3: 984 against 1584 us).
 // ------------------------------------------------------------------------------------------
-constexpr int kBandWarps = 8;
-constexpr int kBandThreads = 32 * kBandWarps;
-constexpr int kNever = 1 << 30;  // c of a successor that never wins (every real c is < 2^21)
+constexpr int kWarps = 8;
+constexpr int kThreads = 32 * kWarps;
+constexpr int kGroup = 8;              // rows per group, outputs per strip
+constexpr int kNear = 2;               // groups on each side of a strip that are tested one by one
+constexpr int kMaxGroups = kMaxAxis / kGroup;  // 64: two per lane
+constexpr float kPadValue = 8.0e6f;    // rows past the axis and groups taken: above every bound
+constexpr float kFar = 2048.f;         // z distance on a side of a row without a site
+constexpr float kIntBias = 8388608.f;  // 2^23: adding it puts a non-negative integer into the mantissa bits
 
-__device__ __forceinline__ uint32_t pack_site(int v, int c) { return ((uint32_t)v << 21) | (uint32_t)c; }
-__device__ __forceinline__ int site_v(uint32_t e) { return (int)(e >> 21); }
-__device__ __forceinline__ int site_c(uint32_t e) { return (int)(e & 0x1fffffu); }
+__host__ __device__ __forceinline__ int groups_of(int n) { return (n + kGroup - 1) / kGroup; }
 
-// Middle site b of a < b < u is never strictly below both neighbours' parabolas.
-__device__ __forceinline__ bool hidden(uint32_t a, uint32_t b, uint32_t u) {
-    const int va = site_v(a), vb = site_v(b), vu = site_v(u);
-    const int ca = site_c(a), cb = site_c(b), cu = site_c(u);
-    return (cb - ca) * (vu - vb) >= (cu - cb) * (vb - va);
+// Shared memory of a pass over an axis of length n with rows of `ld` words: the rows, padded to whole
+// groups, then the groups' minima per column and over all columns.
+int pass_smem_bytes(int n, int ld) { return (groups_of(n) * (kGroup * ld + 32) + 2 * kNear * 32 + kMaxGroups) * 4; }
+
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float d;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+// Extremes over the warp of non-negative floats (their bits order as unsigned integers).
+__device__ __forceinline__ float warp_max(float v) {
+    return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));
+}
+__device__ __forceinline__ float warp_min(float v) {
+    return __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(v)));
 }
 
-// P_next(q) <= P_cur(q) for sites cur < next: the hull walk moves on.
-__device__ __forceinline__ bool next_wins(uint32_t cur, uint32_t nxt, int q) {
-    return site_c(nxt) - site_c(cur) <= 2 * q * (site_v(nxt) - site_v(cur));
-}
+// A strip's outputs of one column: a[k] is output k less k^2.
+struct Strip {
+    float a[kGroup];
 
-// Shared layout of a band pass over an axis of length n: hull[n][32] entries, then per band and
-// lane the entry count and the surviving range.
-struct BandSmem {
-    uint32_t* hull;
-    int* cnt;
-    int* lo;
-    int* hi;
-};
-
-__device__ __forceinline__ BandSmem band_smem(void* base, int n) {
-    BandSmem b;
-    b.hull = static_cast<uint32_t*>(base);
-    b.cnt = reinterpret_cast<int*>(b.hull + n * 32);
-    b.lo = b.cnt + kBandWarps * 32;
-    b.hi = b.lo + kBandWarps * 32;
-    return b;
-}
-
-__host__ __device__ __forceinline__ int band_rows(int n) { return (n + kBandWarps - 1) / kBandWarps; }
-
-int band_smem_bytes(int n) { return n * 32 * 4 + 3 * kBandWarps * 32 * 4; }
-
-// Hull stack of one lane over rows r0, r0 + 1, ... whose f values sit in the lane's column of
-// the staged rows; entries overwrite the rows from r0 on (entry k at row r0 + k).  Registers hold
-// the top entry (v1, c1) and its edge from the entry below (dv, dc), so the convexity test is one
-// multiply-compare and a pop needs one shared-memory load.
-struct InPlaceHull {
-    uint32_t* base;  // &hull[r0 * 32 + lane]
-    int r0;
-    int top;             // index of the top entry, -1 when empty
-    int v1, c1, dv, dc;  // top entry; top minus the entry below (valid when top >= 1)
-
-    __device__ __forceinline__ InPlaceHull(uint32_t* hull, int r0_, int lane)
-        : base(hull + r0_ * 32 + lane), r0(r0_), top(-1), v1(0), c1(0), dv(1), dc(0) {}
-
-    // rows [ra, rb) in increasing order; f >= sentinel is no site
-    __device__ __forceinline__ void rows(int ra, int rb, int32_t sentinel) {
-#pragma unroll 4
-        for (int v = ra; v < rb; ++v) {
-            const int f = (int)base[(v - r0) * 32];
-            if (f >= sentinel) continue;
-            const int c = f + v * v;
-            int ev = v - v1, ec = c - c1;
-            // the top is hidden between the entry below it and the new site
-            while (top >= 1 && dc * ev >= ec * dv) {
-                --top;
-                v1 -= dv;
-                c1 -= dc;
-                if (top >= 1) {
-                    const uint32_t e = base[(top - 1) * 32];
-                    dv = v1 - site_v(e);
-                    dc = c1 - site_c(e);
-                }
-                ev = v - v1;
-                ec = c - c1;
+    __device__ __forceinline__ float value(int k) const { return a[k] + (float)(k * k); }
+    __device__ __forceinline__ int integer(int k) const {  // value(k), exact: its bits above 2^23
+        return __float_as_int(a[k] + (kIntBias + (float)(k * k))) - 0x4b000000;
+    }
+    // the sites of one group: col points at its first row's value of this column, e = (D, D - 1),
+    // back2 = (-2, -2); output k + 1's terms are output k's plus 2 (D - i), so no constants are held
+    template <int LD, bool kFirst = false>
+    __device__ __forceinline__ void group(const float* __restrict__ col, float2 e, float2 back2) {
+#pragma unroll
+        for (int i = 0; i < kGroup; i += 2) {
+            const float2 step = __fadd2_rn(e, e);
+            float2 c = __ffma2_rn(e, e, make_float2(col[i * LD], col[(i + 1) * LD]));
+#pragma unroll
+            for (int k = 0; k < kGroup; ++k) {
+                a[k] = kFirst && i == 0 ? fminf(c.x, c.y) : min3(a[k], c.x, c.y);
+                if (k + 1 < kGroup) c = __fadd2_rn(c, step);
             }
-            ++top;
-            base[top * 32] = pack_site(v, c);
-            v1 = v;
-            c1 = c;
-            dv = ev;
-            dc = ec;
+            e = __fadd2_rn(e, back2);
         }
+    }
+    // Largest value of the strip (past the axis's end its outputs count too: a last strip may then look
+    // at a group more than it needs).
+    __device__ __forceinline__ float largest() const {
+        return max3(max3(value(0), value(1), value(2)), max3(value(3), value(4), value(5)), fmaxf(value(6), value(7)));
     }
 };
 
-__device__ __forceinline__ bool band_live(const BandSmem& sm, int b, int lane) {
-    return sm.hi[b * 32 + lane] >= sm.lo[b * 32 + lane];
-}
-
-// Phase 3: pairwise joins of band groups in log2(kBandWarps) rounds (warp j joins group j of the
-// round), each the bridge between two x-separated lower hulls: trim the left group's suffix and the
-// right group's prefix until the junction is convex.  Every band ends with a surviving range [lo, hi]
-// (empty when hi < lo); the ranges in band order are the column's lower hull.  Contains
-// __syncthreads(): every thread of the CTA calls it.
-__device__ void hull_merge(const BandSmem& sm, int n) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int rows = band_rows(n);
-    sm.lo[warp * 32 + lane] = 0;
-    sm.hi[warp * 32 + lane] = sm.cnt[warp * 32 + lane] - 1;
-    for (int half = 1; half < kBandWarps; half *= 2) {
-        __syncthreads();
-        const int a = warp * 2 * half, m = a + half, e = min(kBandWarps, a + 2 * half);
-        if (m < kBandWarps) {
-            int L = m - 1;
-            while (L >= a && !band_live(sm, L, lane)) --L;
-            int R = m;
-            while (R < e && !band_live(sm, R, lane)) ++R;
-            if (L >= a && R < e) {
-                // every step removes one entry: the loop ends within n steps
-                for (int step = 0; step <= n; ++step) {
-                    const int hiL = sm.hi[L * 32 + lane], loR = sm.lo[R * 32 + lane];
-                    const uint32_t e1 = sm.hull[(L * rows + hiL) * 32 + lane];
-                    const uint32_t r0 = sm.hull[(R * rows + loR) * 32 + lane];
-                    int pb = L, pi = hiL - 1;
-                    if (pi < sm.lo[L * 32 + lane]) {
-                        pb = L - 1;
-                        while (pb >= a && !band_live(sm, pb, lane)) --pb;
-                        pi = pb >= a ? sm.hi[pb * 32 + lane] : -1;
-                    }
-                    if (pb >= a && hidden(sm.hull[(pb * rows + pi) * 32 + lane], e1, r0)) {
-                        sm.hi[L * 32 + lane] = hiL - 1;
-                        if (hiL - 1 < sm.lo[L * 32 + lane]) L = pb;
-                        continue;
-                    }
-                    int sb = R, si = loR + 1;
-                    if (si > sm.hi[R * 32 + lane]) {
-                        sb = R + 1;
-                        while (sb < e && !band_live(sm, sb, lane)) ++sb;
-                        si = sb < e ? sm.lo[sb * 32 + lane] : -1;
-                    }
-                    if (sb < e && hidden(e1, r0, sm.hull[(sb * rows + si) * 32 + lane])) {
-                        sm.lo[R * 32 + lane] = loR + 1;
-                        if (loR + 1 > sm.hi[R * 32 + lane]) R = sb;
-                        continue;
-                    }
-                    break;
-                }
-            }
-        }
-    }
-    __syncthreads();
-}
-
-// Phase 4 for targets [q0, q1) of one warp: store(value) for q = q0, q0 + 1, ... in order; lanes
-// whose column has no site store `sentinel`.
-template <typename Store>
-__device__ __forceinline__ void hull_output(const BandSmem& sm, int n, int q0, int q1, int32_t sentinel, Store store) {
+// Minima of a warp's own groups [g0, g1).
+template <int LD>
+__device__ __forceinline__ void group_minima(const float* __restrict__ rows, float* __restrict__ mins,
+                                             float* __restrict__ low, int g0, int g1) {
     const int lane = threadIdx.x & 31;
-    const int rows = band_rows(n);
-    if (q0 >= q1) return;
-    int b = 0;
-    while (b < kBandWarps && !band_live(sm, b, lane)) ++b;
-    if (b == kBandWarps) {
-        for (int q = q0; q < q1; ++q) store(sentinel);
-        return;
-    }
-    // band holding the vertex that covers q0: the first band whose last surviving entry is not
-    // beaten at q0 by the next surviving band's first one
-    for (;;) {
-        int nb = b + 1;
-        while (nb < kBandWarps && !band_live(sm, nb, lane)) ++nb;
-        if (nb == kBandWarps) break;
-        if (!next_wins(sm.hull[(b * rows + sm.hi[b * 32 + lane]) * 32 + lane],
-                       sm.hull[(nb * rows + sm.lo[nb * 32 + lane]) * 32 + lane], q0))
-            break;
-        b = nb;
-    }
-    // binary search inside band b: the first index whose successor does not win at q0
-    int lo = sm.lo[b * 32 + lane], hi = sm.hi[b * 32 + lane];
-    {
-        const uint32_t* band = sm.hull + b * rows * 32 + lane;
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if (next_wins(band[mid * 32], band[(mid + 1) * 32], q0)) lo = mid + 1;
-            else hi = mid;
-        }
-    }
-    // walk: p points at the successor of the current vertex (vc, cc), dn = its v - vc and cn its
-    // c - cc; pend is the last surviving entry of p's band.  Past the last vertex the successor
-    // never wins (dn = 0, cn = kNever).
-    const uint32_t* p = sm.hull + (b * rows + lo) * 32 + lane;
-    const uint32_t* pend = sm.hull + (b * rows + sm.hi[b * 32 + lane]) * 32 + lane;
-    const uint32_t e = *p;
-    int vc = site_v(e), cc = site_c(e);
-    int dn = 0, cn = kNever;
-    auto fetch = [&]() {
-        if (p < pend) {
-            p += 32;
-        } else {
-            int k = b + 1;
-            while (k < kBandWarps && !band_live(sm, k, lane)) ++k;
-            if (k == kBandWarps) {
-                dn = 0;
-                cn = kNever;
-                return;
-            }
-            b = k;
-            p = sm.hull + (k * rows + sm.lo[k * 32 + lane]) * 32 + lane;
-            pend = sm.hull + (k * rows + sm.hi[k * 32 + lane]) * 32 + lane;
-        }
-        const uint32_t x = *p;
-        dn = site_v(x) - vc;
-        cn = site_c(x) - cc;
-    };
-    fetch();
-#pragma unroll 4
-    for (int q = q0; q < q1; ++q) {
-        const int q2 = 2 * q;
-        while (cn <= q2 * dn) {
-            vc += dn;
-            cc += cn;
-            fetch();
-        }
-        store(cc + q * (q - 2 * vc));
+    for (int g = g0; g < g1; ++g) {
+        const float* col = rows + g * kGroup * LD + lane;
+        float m = col[0];
+#pragma unroll
+        for (int i = 1; i + 1 < kGroup; i += 2) m = min3(m, col[i * LD], col[(i + 1) * LD]);
+        m = fminf(m, col[(kGroup - 1) * LD]);
+        mins[g * 32 + lane] = m;
+        m = warp_min(m);
+        if (lane == 0) low[g] = m;
     }
 }
 
-__device__ __forceinline__ void cp_async4(uint32_t* smem_dst, const int32_t* src) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem_dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(src) : "memory");
+// The strips [g0, g1) of one warp in ascending order, an axis of n rows: store(strip, g) for each, columns
+// inside the grid.  All rows and minima of the CTA are in place (the caller has synchronised); `mins`
+// holds kNear groups of kPadValue before the first and after the last group, which therefore fail every
+// test.  Columns outside the grid hold kPadValue in every row and take no part in the decisions.
+//
+// Far from every site the minimum lies groups away and moves less than a group per strip: a strip that
+// ended there hands the place to the next one, which begins with that group instead of its own.  The
+// site of an output never lies before the previous output's, so groups before the least such place of
+// the columns are left out, and groups beyond a column's own are tested at the strip's last output.
+template <int LD, typename Store>
+__device__ __forceinline__ void strips(const float* __restrict__ rows, const float* __restrict__ mins,
+                                       const float* __restrict__ low, int n, int g0, int g1, bool in, Store store) {
+    const int lane = threadIdx.x & 31;
+    const int ng = groups_of(n);
+    // packed constants, kept in registers (their values hidden from the compiler, which would rebuild
+    // each from immediates at every use)
+    float2 origin = make_float2(0.f, -1.f), back2 = make_float2(-2.f, -2.f);
+    float2 ahead = make_float2((float)kGroup, (float)kGroup), behind = make_float2(-(float)kGroup, -(float)kGroup);
+    asm volatile("" : "+f"(origin.x), "+f"(origin.y), "+f"(back2.x), "+f"(back2.y));
+    asm volatile("" : "+f"(ahead.x), "+f"(ahead.y), "+f"(behind.x), "+f"(behind.y));
+    int seed = 0;   // offset of the group to begin with
+    int least = 0;  // groups before it hold no minimum of this and later strips
+    for (int g = g0; g < g1; ++g) {
+        const float* const own = rows + g * kGroup * LD + lane;
+        const float* const near = mins + g * 32 + lane;
+        Strip s;
+        float most;  // largest output of this column
+        if (seed == 0) {
+            s.group<LD, true>(own, origin, back2);
+            most = in ? s.largest() : 0.f;
+            float2 left = origin, right = origin;
+#pragma unroll
+            for (int o = 1; o <= kNear; ++o) {
+                const float d = (float)(kGroup * o - (kGroup - 1));
+                left = __fadd2_rn(left, ahead);
+                right = __fadd2_rn(right, behind);
+                if (__any_sync(0xffffffffu, near[-o * 32] < most - d * d)) {
+                    s.group<LD>(own - o * kGroup * LD, left, back2);
+                    most = in ? s.largest() : 0.f;
+                }
+                if (__any_sync(0xffffffffu, near[o * 32] < most - d * d)) {
+                    s.group<LD>(own + o * kGroup * LD, right, back2);
+                    most = in ? s.largest() : 0.f;
+                }
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < kGroup; ++k) s.a[k] = kPadValue;
+            most = in ? kPadValue : 0.f;
+        }
+        constexpr float kReach = (float)(kGroup * kNear + 1);
+        if (seed != 0 || __any_sync(0xffffffffu, kReach * kReach < most)) {
+            float top = warp_max(most);  // of all columns
+            const int skip = seed == 0 ? kNear : -1;
+            int at = seed == 0 ? -kNear : ng;  // a group no later than the last output's minimum, as an offset
+            const int o0 = abs(lane - g), o1 = abs(lane + 32 - g);
+            const float d0 = fmaxf((float)(kGroup * o0 - (kGroup - 1)), 0.f), d1 = fmaxf((float)(kGroup * o1 - (kGroup - 1)), 0.f);
+            float b0 = o0 > skip && lane >= least && lane < ng ? fmaf(d0, d0, low[lane]) : kPadValue;
+            float b1 = o1 > skip && lane + 32 >= least && lane + 32 < ng ? fmaf(d1, d1, low[lane + 32]) : kPadValue;
+            int next = g + seed;
+            bool begin = seed != 0;
+            for (;;) {  // each turn takes one group out
+                int j = next;
+                if (!begin) {
+                    const float b = fminf(b0, b1), best = warp_min(b);
+                    if (!(best < top)) break;
+                    const int who = __ffs(__ballot_sync(0xffffffffu, b == best)) - 1;
+                    j = __shfl_sync(0xffffffffu, b0 <= b1 ? lane : lane + 32, who);
+                }
+                if (lane == j) b0 = kPadValue;
+                if (lane + 32 == j) b1 = kPadValue;
+                const int o = j - g;
+                const float D = (float)(-kGroup * o);
+                // distance to the nearest output, and from the last one where only that can gain
+                const float d = fmaxf(fabsf(D) - (float)(kGroup - 1), 0.f);
+                const float dl = o < 0 ? D : d;
+                const bool beyond = o > at;
+                const float e = beyond ? dl : d;
+                const float lim = beyond && in ? s.value(kGroup - 1) : most;
+                if (!begin && !__any_sync(0xffffffffu, near[o * 32] < fmaf(-e, e, lim))) continue;
+                begin = false;
+                const float was = s.a[kGroup - 1];
+                s.group<LD>(own + o * (kGroup * LD), make_float2(D, D - 1.f), back2);
+                if (s.a[kGroup - 1] < was) at = o;
+                most = in ? s.largest() : 0.f;
+                top = warp_max(most);
+            }
+            least = g + __reduce_min_sync(0xffffffffu, in ? at : ng);
+            seed = __shfl_sync(0xffffffffu, at, 0) - 1;
+            if (seed >= -kNear - 1 && seed <= kNear) seed = 0;
+        }
+        if (in) store(s, g);
+    }
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
+// Outputs of strip g of an axis of n rows, `stride` elements apart from `out` (row 0) on.
+template <typename T>
+__device__ __forceinline__ void put(const Strip& s, T* __restrict__ out, int64_t stride, int n, int g) {
+    T* p = out + (int64_t)(g * kGroup) * stride;
+    const int valid = n - g * kGroup;
+    auto one = [&](int k) {
+        if (sizeof(T) == 4 && T(0.5f) == T(0)) *p = (T)s.integer(k);
+        else *p = (T)s.value(k);
+        p += stride;
+    };
+    if (valid >= kGroup) {
+#pragma unroll
+        for (int k = 0; k < kGroup; ++k) one(k);
+    } else {
+#pragma unroll
+        for (int k = 0; k < kGroup; ++k)
+            if (k < valid) one(k);
+    }
+}
+
+// The padding groups of `mins` (strips).
+__device__ __forceinline__ void pad_minima(float* __restrict__ mins, int ng) {
+    for (int i = threadIdx.x; i < kNear * 32; i += blockDim.x) {
+        mins[i - kNear * 32] = kPadValue;
+        mins[ng * 32 + i] = kPadValue;
+    }
+}
+
+// cp.async of `bytes` (4 or 16) to shared memory.
+template <int bytes>
+__device__ __forceinline__ void cp_async(float* smem_dst, const float* src) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem_dst);
+    if (bytes == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(src) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 // z pass (nearest set bit along z from the bit words) + y pass.  grid = (W, nx, polarities),
-// block = kBandThreads, dynamic smem = band_smem_bytes(ny).  Polarity p measures to set bits when
+// block = kThreads, dynamic smem = pass_smem_bytes(ny, kZyLd).  Polarity p measures to set bits when
 // (p ^ invert) == 0, to clear bits otherwise.
-__global__ void __launch_bounds__(kBandThreads) k_edt_zy(const uint32_t* __restrict__ bits, int32_t* __restrict__ g,
-                                                         int nx, int ny, int nz, int W, int invert, int32_t sentinel) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const BandSmem sm = band_smem(smem_raw, ny);
-    const int w = blockIdx.x, x = blockIdx.y, pol = blockIdx.z;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const bool flip = (pol ^ invert) != 0;
-    const int tail = nz & 31;
-    const uint32_t last_valid = tail ? ((1u << tail) - 1u) : 0xffffffffu;
-    const int z = 32 * w + lane;
-    const int rows = band_rows(ny);
-    const int y0 = warp * rows, y1 = min(ny, y0 + rows);
-    // 1. f(y) = squared distance to the nearest site along z, for each row of the band, into the
-    //    band's rows (sentinel where the row has no site)
-    uint32_t* const mine = sm.hull + y0 * 32 + lane;
-    const uint32_t* line = bits + ((int64_t)x * ny + y0) * W + lane;  // row y0's words, one per lane < W
-    const bool loads = lane < W;
-    const uint32_t below_mask = (1u << w) - 1u, above_mask = ~((2u << w) - 1u);
-    const uint32_t low_mask = 0xffffffffu >> (31 - lane), high_mask = 0xffffffffu << lane;
-    constexpr int kAhead = 8;  // rows of bit words in flight
-    uint32_t ring[kAhead];
+//
+// z: a lane owns a row.  It reads the row's words once, keeps the last nonzero word before and the
+// first one after its own, and fills the row's 32 distances by a forward and a backward count over the
+// own word's bits, two instructions a voxel each -- where a lane per voxel spent ballots, shuffles and
+// bit searches on every one.  Rows are 33 words apart so that these stores, one row per lane, and the
+// y pass's reads, one column per lane, are both free of bank conflicts.
+constexpr int kZyLd = 33;
+
+// Squared z distances of a row's 32 voxels to the set bits of `own` and to the nearest sites outside the
+// word, `from` and `to` voxels before its first and after its last neighbour.  Out of line: its counts
+// stay out of the registers of the y pass.
+__device__ __noinline__ void fill_row(float* __restrict__ row, uint32_t own, float from, float to) {
+    float up[32], d = from;
 #pragma unroll
-    for (int k = 0; k < kAhead; ++k) ring[k] = (loads && y0 + k < y1) ? line[k * W] : 0u;
-    for (int yb = y0; yb < y1; yb += kAhead) {
-#pragma unroll
-        for (int k = 0; k < kAhead; ++k) {
-            const int y = yb + k;
-            uint32_t word = ring[k];
-            ring[k] = (loads && y + kAhead < y1) ? line[(y + kAhead - y0) * W] : 0u;
-            if (y >= y1) break;
-            if (loads) {
-                if (flip) word = ~word;
-                if (lane == W - 1) word &= last_valid;
-            }
-            const uint32_t nonzero = __ballot_sync(0xffffffffu, word != 0);
-            int f = sentinel;
-            if (nonzero) {  // uniform across the warp
-                const uint32_t own = __shfl_sync(0xffffffffu, word, w);
-                const uint32_t below = nonzero & below_mask;
-                const uint32_t above = nonzero & above_mask;
-                const int pw = below ? 31 - __clz(below) : 0;
-                const int nw = above ? __ffs(above) - 1 : 0;
-                const uint32_t prev_word = __shfl_sync(0xffffffffu, word, pw);
-                const uint32_t next_word = __shfl_sync(0xffffffffu, word, nw);
-                const uint32_t low = own & low_mask;
-                const uint32_t high = own & high_mask;
-                int prev = -(1 << 20), next = 1 << 20;
-                if (low) prev = 32 * w + 31 - __clz(low);
-                else if (below) prev = 32 * pw + 31 - __clz(prev_word);
-                if (high) next = 32 * w + __ffs(high) - 1;
-                else if (above) next = 32 * nw + __ffs(next_word) - 1;
-                const int d = min(z - prev, next - z);
-                f = d * d;
-            }
-            mine[(y - y0) * 32] = (uint32_t)f;
-        }
+    for (int z = 0; z < 32; ++z) {
+        d = (own >> z) & 1u ? 0.f : d + 1.f;
+        up[z] = d;
     }
-    // 2. hull stack over the band, in place
-    InPlaceHull st(sm.hull, y0, lane);
-    st.rows(y0, y1, sentinel);
-    sm.cnt[warp * 32 + lane] = st.top + 1;
-    hull_merge(sm, ny);
-    if (z >= nz) return;
-    int32_t* out = g + (int64_t)pol * nx * ny * nz + ((int64_t)x * ny + y0) * nz + z;
-    hull_output(sm, ny, y0, y1, sentinel, [&](int32_t v) {
-        *out = v;
-        out += nz;
-    });
+    d = to;
+#pragma unroll
+    for (int z = 31; z >= 0; --z) {
+        d = (own >> z) & 1u ? 0.f : d + 1.f;
+        const float m = fminf(d, up[z]);
+        row[z] = m * m;
+    }
 }
 
-// x pass.  grid = (W, ny, polarities), block = kBandThreads, dynamic smem = band_smem_bytes(nx).
+__global__ void __launch_bounds__(kThreads, 3) k_edt_zy(const uint32_t* __restrict__ bits, float* __restrict__ g,
+                                                        int nx, int ny, int nz, int W, int invert, float sentinel) {
+    extern __shared__ __align__(16) float smem[];
+    const int w = blockIdx.x, x = blockIdx.y, pol = blockIdx.z;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int ng = groups_of(ny);
+    float* const rows = smem;
+    float* const mins = smem + ng * kGroup * kZyLd + kNear * 32;
+    float* const low = mins + (ng + kNear) * 32;
+    pad_minima(mins, ng);
+    const uint32_t flip = (pol ^ invert) != 0 ? 0xffffffffu : 0u;
+    const int tail = nz & 31;
+    const uint32_t last_valid = tail ? ((1u << tail) - 1u) : 0xffffffffu;
+    const int live = min(32, nz - 32 * w);  // columns of this chunk inside the grid
+    const int per = (ng + kWarps - 1) / kWarps;
+    const int g0 = min(ng, warp * per), g1 = min(ng, g0 + per);
+    // a plane without a site keeps the sentinel everywhere
+    const uint32_t* const plane = bits + (int64_t)x * ny * W;
+    bool some = false;
+    for (int k = threadIdx.x; k < ny * W; k += kThreads) {
+        uint32_t word = plane[k] ^ flip;
+        if (tail && k % W == W - 1) word &= last_valid;
+        some |= word != 0u;
+    }
+    float* const out = g + (int64_t)pol * nx * ny * nz + (int64_t)x * ny * nz + 32 * w + lane;
+    const bool in = lane < live;
+    if (!__syncthreads_or(some)) {
+        if (in)
+            for (int y = g0 * kGroup; y < min(ny, g1 * kGroup); ++y) out[(int64_t)y * nz] = sentinel;
+        return;
+    }
+    for (int y0 = g0 * kGroup; y0 < g1 * kGroup; y0 += 32) {
+        const int y = y0 + lane;
+        if (y >= g1 * kGroup) continue;
+        float* const row = rows + y * kZyLd;
+        if (y >= ny) {  // padding to a whole group
+#pragma unroll
+            for (int z = 0; z < 32; ++z) row[z] = kPadValue;
+            continue;
+        }
+        const uint32_t* const line = plane + y * W;
+        uint32_t before = 0u, after = 0u;
+        int bw = 0, aw = 0;
+        for (int k = 0; k < w; ++k) {
+            const uint32_t word = line[k] ^ flip;
+            if (word) { before = word; bw = k; }
+        }
+        const uint32_t own = (line[w] ^ flip) & (w == W - 1 ? last_valid : 0xffffffffu);
+        for (int k = W - 1; k > w; --k) {
+            const uint32_t word = (line[k] ^ flip) & (k == W - 1 ? last_valid : 0xffffffffu);
+            if (word) { after = word; aw = k; }
+        }
+        if (!(before | own | after)) {
+#pragma unroll
+            for (int z = 0; z < 32; ++z) row[z] = sentinel;
+        } else {
+            fill_row(row, own, before ? (float)(32 * (w - bw) - 1 - (31 - __clz(before))) : kFar,
+                     after ? (float)(32 * (aw - w) - 32 + __ffs(after) - 1) : kFar);
+        }
+        for (int z = live; z < 32; ++z) row[z] = kPadValue;
+    }
+    __syncwarp();
+    group_minima<kZyLd>(rows, mins, low, g0, g1);
+    __syncthreads();
+    strips<kZyLd>(rows, mins, low, ny, g0, g1, in, [&](const Strip& s, int gr) { put<float>(s, out, nz, ny, gr); });
+}
+
+// x pass.  grid = (W, ny, polarities), block = kThreads, dynamic smem = pass_smem_bytes(nx, 32).
 // Reads g (polarity-major, `size` voxels each) and writes out with the same layout; out may be g
-// itself (each CTA reads its whole column block before it writes any of it).
-__global__ void __launch_bounds__(kBandThreads) k_edt_x(const int32_t* g, int32_t* out, int nx, int ny, int nz,
-                                                        int32_t sentinel) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const BandSmem sm = band_smem(smem_raw, nx);
+// itself (each CTA reads its whole column block before it writes any of it).  kVec: rows of g are
+// 16-byte aligned (nz a multiple of 4 and g itself aligned), so one copy instruction moves four rows'
+// segments of the block instead of one.
+template <bool kVec>
+__global__ void __launch_bounds__(kThreads, 3) k_edt_x(const float* g, int32_t* out, int nx, int ny, int nz) {
+    extern __shared__ __align__(16) float smem[];
     const int w = blockIdx.x, y = blockIdx.y, pol = blockIdx.z;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int z = 32 * w + lane;
-    const bool live = z < nz;
-    const int64_t size = (int64_t)nx * ny * nz;
-    const int64_t col = (int64_t)pol * size + (int64_t)y * nz + z;
-    const int64_t stride = (int64_t)ny * nz;
-    const int rows = band_rows(nx);
-    const int x0 = warp * rows, x1 = min(nx, x0 + rows);
-    // 1. stage the band's column values into its rows, in four commit groups so that the hull
-    //    starts on the first quarter while the rest is in flight
-    constexpr int kGroups = 4;
-    const int chunk = (rows + kGroups - 1) / kGroups;
-    uint32_t* const mine = sm.hull + x0 * 32 + lane;
-    InPlaceHull st(sm.hull, x0, lane);
-    if (live) {
-        const int32_t* src = g + col + (int64_t)x0 * stride;
-#pragma unroll
-        for (int j = 0; j < kGroups; ++j) {
-            const int ka = j * chunk, kb = min(x1 - x0, ka + chunk);
-            for (int k = ka; k < kb; ++k) cp_async4(mine + k * 32, src + (int64_t)k * stride);
-            cp_async_commit();
+    const int ng = groups_of(nx);
+    float* const rows = smem;
+    float* const mins = smem + ng * kGroup * 32 + kNear * 32;
+    float* const low = mins + (ng + kNear) * 32;
+    pad_minima(mins, ng);
+    const int64_t size = (int64_t)nx * ny * nz, stride = (int64_t)ny * nz;
+    const int64_t col = (int64_t)pol * size + (int64_t)y * nz + 32 * w;
+    const int live = min(32, nz - 32 * w);
+    const int per = (ng + kWarps - 1) / kWarps;
+    const int g0 = min(ng, warp * per), g1 = min(ng, g0 + per);
+    const int x1 = min(nx, g1 * kGroup);
+    // the warp's rows, 4 a copy instruction (kVec) or one; columns outside the grid are filled
+    const int rstep = kVec ? 4 : 1, c = kVec ? 4 * (lane & 7) : lane;
+    const int xa = g0 * kGroup + (kVec ? lane >> 3 : 0);
+    if (c < live) {
+        const float* src = g + col + xa * stride + c;
+        float* to = rows + xa * 32 + c;
+#pragma unroll 4
+        for (int x = xa; x < x1; x += rstep) {
+            cp_async<kVec ? 16 : 4>(to, src);
+            src += rstep * stride;
+            to += rstep * 32;
         }
-        // 2. hull stack over the band, in place, one commit group at a time
-        cp_async_wait<kGroups - 1>();
-        st.rows(x0, min(x1, x0 + chunk), sentinel);
-        cp_async_wait<kGroups - 2>();
-        st.rows(min(x1, x0 + chunk), min(x1, x0 + 2 * chunk), sentinel);
-        cp_async_wait<kGroups - 3>();
-        st.rows(min(x1, x0 + 2 * chunk), min(x1, x0 + 3 * chunk), sentinel);
-        cp_async_wait<0>();
-        st.rows(min(x1, x0 + 3 * chunk), x1, sentinel);
+    } else {
+        for (int x = xa; x < x1; x += rstep)
+            for (int k = 0; k < (kVec ? 4 : 1); ++k) rows[x * 32 + c + k] = kPadValue;
     }
-    sm.cnt[warp * 32 + lane] = st.top + 1;
-    hull_merge(sm, nx);
-    if (!live) return;
-    int32_t* dst = out + col + (int64_t)x0 * stride;
-    hull_output(sm, nx, x0, x1, sentinel, [&](int32_t v) {
-        *dst = v;
-        dst += stride;
-    });
+    for (int x = max(nx, g0 * kGroup); x < g1 * kGroup; ++x) rows[x * 32 + lane] = kPadValue;
+    cp_async_wait_all();
+    __syncwarp();
+    group_minima<32>(rows, mins, low, g0, g1);
+    __syncthreads();
+    int32_t* const dst = out + col + lane;
+    const bool in = lane < live;
+    strips<32>(rows, mins, low, nx, g0, g1, in, [&](const Strip& s, int gr) { put<int32_t>(s, dst, stride, nx, gr); });
 }
 
 // Correctly rounded signed distance of one voxel from its two squared distances, the reference's
@@ -510,6 +527,15 @@ int32_t sentinel_of(int nx, int ny, int nz) {
 
 int words_of(int nz) { return (nz + 31) / 32; }
 
+void launch_x(const float* g, int32_t* out, int nx, int ny, int nz, int W, int npol, cudaStream_t stream) {
+    const dim3 grid(W, ny, npol);
+    const int smem = pass_smem_bytes(nx, 32);
+    if (nz % 4 == 0 && (reinterpret_cast<uintptr_t>(g) & 15) == 0)
+        k_edt_x<true><<<grid, kThreads, smem, stream>>>(g, out, nx, ny, nz);
+    else
+        k_edt_x<false><<<grid, kThreads, smem, stream>>>(g, out, nx, ny, nz);
+}
+
 // Scratch layout: [Counters (256 B)] [bit words] [g for up to two polarities].
 int64_t scratch_bytes(int nx, int ny, int nz, int npol) {
     const int64_t size = (int64_t)nx * ny * nz;
@@ -529,8 +555,10 @@ int configure_device() {
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return FB_RUNTIME;
     std::lock_guard<std::mutex> guard(g_configure_lock);
     if (g_configured[dev]) return FB_OK;
-    FB_CUDA(cudaFuncSetAttribute(k_edt_zy, cudaFuncAttributeMaxDynamicSharedMemorySize, band_smem_bytes(kMaxAxis)));
-    FB_CUDA(cudaFuncSetAttribute(k_edt_x, cudaFuncAttributeMaxDynamicSharedMemorySize, band_smem_bytes(kMaxAxis)));
+    const auto most = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    FB_CUDA(cudaFuncSetAttribute(k_edt_zy, most, pass_smem_bytes(kMaxAxis, kZyLd)));
+    FB_CUDA(cudaFuncSetAttribute(k_edt_x<true>, most, pass_smem_bytes(kMaxAxis, 32)));
+    FB_CUDA(cudaFuncSetAttribute(k_edt_x<false>, most, pass_smem_bytes(kMaxAxis, 32)));
     g_configured[dev] = true;
     return FB_OK;
 }
@@ -550,7 +578,7 @@ int enqueue(const uint8_t* d_mask, int nx, int ny, int nz, int paired, int sites
     char* base = static_cast<char*>(scratch);
     Counters* counters = reinterpret_cast<Counters*>(base);
     uint32_t* bits = reinterpret_cast<uint32_t*>(base + 256);
-    int32_t* g = reinterpret_cast<int32_t*>(base + 256 + ((lines * W * 4 + 255) / 256 * 256));
+    float* g = reinterpret_cast<float*>(base + 256 + ((lines * W * 4 + 255) / 256 * 256));
     if (count) FB_CUDA(cudaMemsetAsync(counters, 0, sizeof(Counters), stream));
     const int sms = fb_sm_count();
     const int64_t words = lines * W;
@@ -560,17 +588,18 @@ int enqueue(const uint8_t* d_mask, int nx, int ny, int nz, int paired, int sites
     const int32_t sentinel = sentinel_of(nx, ny, nz);
     // Single polarity measuring to zero bytes = the set bits flipped.
     const int invert = paired ? 0 : (sites_nonzero ? 0 : 1);
-    k_edt_zy<<<dim3(W, nx, npol), kBandThreads, band_smem_bytes(ny), stream>>>(bits, g, nx, ny, nz, W, invert, sentinel);
+    k_edt_zy<<<dim3(W, nx, npol), kThreads, pass_smem_bytes(ny, kZyLd), stream>>>(bits, g, nx, ny, nz, W, invert,
+                                                                                  (float)sentinel);
     FB_LAUNCH();
     if (paired) {
         // both polarities' x passes into the squared output (or in place), then the signed values
-        int32_t* sq = out_sq ? out_sq : g;
-        k_edt_x<<<dim3(W, ny, 2), kBandThreads, band_smem_bytes(nx), stream>>>(g, sq, nx, ny, nz, sentinel);
+        int32_t* sq = out_sq ? out_sq : reinterpret_cast<int32_t*>(g);
+        launch_x(g, sq, nx, ny, nz, W, 2, stream);
         FB_LAUNCH();
         const int grid = (int)std::min<int64_t>((size + 255) / 256, (int64_t)sms * 16);
         k_edt_signed<<<grid, 256, 0, stream>>>(sq, out_signed, size, pitch, (float)(0.5 * pitch));
     } else {
-        k_edt_x<<<dim3(W, ny, 1), kBandThreads, band_smem_bytes(nx), stream>>>(g, out_sq, nx, ny, nz, sentinel);
+        launch_x(g, out_sq, nx, ny, nz, W, 1, stream);
     }
     FB_LAUNCH();
     (void)size;

@@ -147,3 +147,35 @@ def test_handle_lifecycle(fe):
     h.close()
     with pytest.raises(RuntimeError):
         h.query(m, 1.0)
+
+
+def _far_mask(kind, shape):
+    """One site, a small ball, a slanted half-space or a few boxes: distances of up to the whole axis."""
+    x, y, z = np.ogrid[:shape[0], :shape[1], :shape[2]]
+    if kind == "voxel":
+        m = np.zeros(shape, bool)
+        m[shape[0] // 3, shape[1] // 2, shape[2] - 1] = True
+        return m
+    if kind == "ball":
+        r = min(shape) // 4 + 1
+        return (x - shape[0] // 2) ** 2 + (y - shape[1] // 3) ** 2 + (z - shape[2] // 2) ** 2 < r * r
+    if kind == "slant":
+        return 3 * x + 2 * y + z < shape[0] // 2 + 1
+    m = np.zeros(shape, bool)
+    m[: shape[0] // 5 + 1, : shape[1] // 7 + 1, :] = True
+    m[-1, shape[1] // 2:, : shape[2] // 2 + 1] = True
+    return m
+
+
+@pytest.mark.parametrize("shape", [(7, 8, 9), (8, 16, 31), (17, 33, 32), (63, 65, 33), (129, 255, 36), (257, 30, 50),
+                                   (31, 511, 34), (512, 40, 12), (200, 264, 64)])
+@pytest.mark.parametrize("kind", ["voxel", "ball", "slant", "boxes"])
+def test_strips_near_and_far_against_oracle(fe, shape, kind):
+    """Edges of the passes' groups of 8 rows and 32 columns, the 16-byte and 4-byte staging (the depth a
+    multiple of 4 or not), and sites many groups away, in both polarities: whole numbers, equal."""
+    import torch
+    m = _far_mask(kind, shape)
+    d = torch.from_numpy(m.view(np.uint8)).cuda()
+    for nonzero, binary in ((True, ~m), (False, m)):
+        got = fe.squared_distance_device(d, sites_nonzero=nonzero).cpu().numpy()
+        assert np.array_equal(got, oracle.edt_squared(binary)), (nonzero,)
