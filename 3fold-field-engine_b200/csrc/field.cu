@@ -13,6 +13,8 @@
 //                    corners in float32 in block-local coordinates, decides kind -1/0/+1 by the
 //                    reference rule, re-evaluating in float64 when a corner value lies within the
 //                    guard band of 0 or of the margin; the active blocks keep their lists.
+//   k_cull_program, k_classify_program, k_leaf_program  the same for general postfix programs, in
+//                    float64 throughout, on programs pruned per superblock and per block.
 //   k_compact        single-pass decoupled look-back scan: ascending active block ids + count.
 //   k_leaf<B>        warp per active block: block-level culling, float64 -> float32 localisation of
 //                    each surviving primitive, float32 evaluation of all B^3 voxels, float64 recheck
@@ -862,25 +864,212 @@ __global__ void __launch_bounds__(128, 6) k_classify_blocks(Geo G, const FbPrim*
                    t);
 }
 
-// General postfix programs: every corner of every block in float64, no culling.
-__global__ void __launch_bounds__(128) k_classify_program(Geo G, const FbPrim* __restrict__ prims,
-                                                          const FbInsn* __restrict__ prog, int n_prog,
-                                                          int32_t* __restrict__ kind, float* __restrict__ cma) {
-    const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+// ------------------------------------------------------------------------------------ general programs
+// The whole float64 program at every corner and voxel is bound by the float64 chains of operands that
+// never matter; pruned per superblock and per block a few of them are left, with the same bits.  An
+// assembly of 12 plates with 24 bores (71 instructions) on 192 x 160 x 121: classification 198 -> 60 us
+// (18 superblocks, 42 blocks and corners; 76 us when every block prunes the whole program itself),
+// leaves 610 -> 46 us.
+constexpr int kProgCap = 256;   // longest pruned program kept for a region
+constexpr int kProgWarps = 4;
+
+// Bounds of a primitive's float64 value over the ball (c, R): the value at the centre and the
+// Lipschitz bound, widened by 1e-10 of every magnitude that enters the evaluation (about 10^6 times
+// its float64 rounding) and rounded outwards to float32.
+__device__ __forceinline__ void prim_bounds_d(const FbPrim& P, const PrimF& F, const double* c, double R, float& lo,
+                                              float& hi) {
+    const double v = prim_world_d(P, c[0], c[1], c[2]);
+    double mag = R;
+    for (int r = 0; r < 3; ++r)
+        mag += fabs(P.A[4 * r] * c[0]) + fabs(P.A[4 * r + 1] * c[1]) + fabs(P.A[4 * r + 2] * c[2]) + fabs(P.A[4 * r + 3]);
+    for (int j = 0; j < 10; ++j) mag += fabs(P.p[j]);
+    const double lip = (double)F.lip;
+    const double r = lip * R + 1e-10 * (fmax(lip, fabs(P.s)) * mag + fabs(P.off) + fabs(v));
+    lo = __double2float_rd(v - r);
+    hi = __double2float_ru(v + r);
+}
+
+// Warp-cooperative pruning of a program (in == nullptr: the whole program of n_in instructions) for
+// the ball (c, R): the lanes bound 32 instructions' primitives at a time, then the warp walks them with
+// the stack of bounds held one entry per lane, cutting the operands that a hard or smooth min / max
+// provably ignores everywhere in the region (strictly beyond the blend width, where the smooth form
+// adds exactly zero).  `out` is the warp's shared buffer of kProgCap entries.  Returns the pruned
+// length, or -1 where the program is longer than that or malformed.  NaN bounds compare false: kept.
+__device__ int prune_program(const FbPrim* __restrict__ prims, const PrimF* __restrict__ primf,
+                             const FbInsn* __restrict__ prog, const uint32_t* __restrict__ in, int n_in,
+                             const double* c, double R, uint32_t* out) {
+    const int lane = threadIdx.x & 31;
+    float slo = 0.f, shi = 0.f;  // stack entry `lane`
+    int sst = 0;                 // where its instructions start in `out`
+    int sp = 0, n = 0;
+    for (int base = 0; base < n_in; base += 32) {
+        uint32_t ent = 0;
+        int op = OP_OFFSET;
+        float lo = 0.f, hi = 0.f;  // a push: its bounds; otherwise k rounded down and up
+        if (base + lane < n_in) {
+            ent = in ? in[base + lane] : (uint32_t)(base + lane) << 2;
+            const FbInsn I = prog[ent >> 2];
+            op = (ent & kProgNeg) ? -1 : I.op;
+            if (op == OP_PUSH) {
+                prim_bounds_d(prims[I.arg], primf[I.arg], c, R, lo, hi);
+            } else {
+                lo = __double2float_rd(I.k);
+                hi = __double2float_ru(I.k);
+            }
+        }
+        const int m = min(32, n_in - base);
+        for (int j = 0; j < m; ++j) {
+            const uint32_t e = __shfl_sync(0xffffffffu, ent, j);
+            const int o = __shfl_sync(0xffffffffu, op, j);
+            const float l = __shfl_sync(0xffffffffu, lo, j), h = __shfl_sync(0xffffffffu, hi, j);
+            if (n >= kProgCap) return -1;
+            if (o == OP_PUSH) {
+                if (sp >= 32) return -1;
+                if (lane == sp) { slo = l; shi = h; sst = n; }
+                if (lane == 0) out[n] = e;
+                ++sp;
+                ++n;
+                continue;
+            }
+            if (o == OP_OFFSET || o == -1) {
+                if (sp < 1) return -1;
+                if (lane == sp - 1) {
+                    const float a = slo, b = shi;
+                    slo = o == -1 ? -b : __fsub_rd(a, h);
+                    shi = o == -1 ? -a : __fsub_ru(b, l);
+                }
+                if (lane == 0) out[n] = e;
+                ++n;
+                continue;
+            }
+            if (sp < 2) return -1;
+            const float k = fmaxf(h, 0.f);
+            const float alo = __shfl_sync(0xffffffffu, slo, sp - 2), ahi = __shfl_sync(0xffffffffu, shi, sp - 2);
+            float blo = __shfl_sync(0xffffffffu, slo, sp - 1), bhi = __shfl_sync(0xffffffffu, shi, sp - 1);
+            const int a0 = __shfl_sync(0xffffffffu, sst, sp - 2), b0 = __shfl_sync(0xffffffffu, sst, sp - 1);
+            const bool uni = o == OP_UNION, neg = !uni && o != OP_INTERSECT;
+            if (neg) {
+                const float t = blo;
+                blo = -bhi;
+                bhi = -t;
+            }
+            const bool drop_b = uni ? blo > __fadd_ru(ahi, k) : bhi < __fsub_rd(alo, k);
+            const bool drop_a = uni ? alo > __fadd_ru(bhi, k) : ahi < __fsub_rd(blo, k);
+            float rlo = alo, rhi = ahi;
+            if (drop_b) {
+                n = b0;
+            } else if (drop_a) {
+                rlo = blo;
+                rhi = bhi;
+                const int len = n - b0;
+                __syncwarp();
+                for (int t = 0; t < len; t += 32) {
+                    const uint32_t w = t + lane < len ? out[b0 + t + lane] : 0u;
+                    __syncwarp();
+                    if (t + lane < len) out[a0 + t + lane] = w;
+                    __syncwarp();
+                }
+                n = a0 + len;
+                if (neg) {  // n <= its old value: below the capacity
+                    if (lane == 0) out[n] = e | kProgNeg;
+                    ++n;
+                }
+            } else {
+                rlo = uni ? __fsub_rd(fminf(alo, blo), 0.25f * k) : fmaxf(alo, blo);
+                rhi = uni ? fminf(ahi, bhi) : __fadd_ru(fmaxf(ahi, bhi), 0.25f * k);
+                // a NaN bound must stay one: fminf and fmaxf would hide it
+                if (!(alo <= ahi && blo <= bhi)) rlo = rhi = __int_as_float(0x7fc00000);
+                if (lane == 0) out[n] = e;
+                ++n;
+            }
+            --sp;
+            if (lane == sp - 1) { slo = rlo; shi = rhi; }
+        }
+    }
+    __syncwarp();
+    return sp == 1 ? n : -1;
+}
+
+// Warp per superblock: the program pruned to it, kept in its slot of the pool (len -1: the whole
+// program).
+__global__ void __launch_bounds__(32 * kProgWarps) k_cull_program(Geo G, const FbPrim* __restrict__ prims,
+                                                                  const PrimF* __restrict__ primf,
+                                                                  const FbInsn* __restrict__ prog, int n_prog,
+                                                                  uint32_t* __restrict__ pool, int64_t pool_base,
+                                                                  int cap, int64_t* __restrict__ off,
+                                                                  int32_t* __restrict__ len) {
+    __shared__ uint32_t s_out[kProgWarps][kProgCap];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t r = blockIdx.x * (int64_t)kProgWarps + warp;
+    if (r >= G.nsuper) return;
+    const int rz = (int)(r % G.nsz), ry = (int)((r / G.nsz) % G.nsy), rx = (int)(r / ((int64_t)G.nsz * G.nsy));
+    const double edge = (double)G.S * G.B, half = 0.5 * edge;
+    const double c[3] = {G.x0 + (rx * edge + half) * G.pitch, G.y0 + (ry * edge + half) * G.pitch,
+                         G.z0 + (rz * edge + half) * G.pitch};
+    const int n = prune_program(prims, primf, prog, nullptr, n_prog, c, 1.7320509 * half * G.pitch, s_out[warp]);
+    const bool kept = n >= 0 && n <= cap;
+    for (int i = lane; kept && i < n; i += 32) pool[pool_base + r * cap + i] = s_out[warp][i];
+    if (lane == 0) {
+        off[r] = pool_base + r * cap;
+        len[r] = kept ? n : -1;
+    }
+}
+
+// Warp per block of a general program: the superblock's program pruned further to the block, the 8
+// corners of it in float64 (lanes 0-7, the oracle's operations), the kind decided from them; an active
+// block's program is kept for the leaf pass (blk_len -1 where the pool is full).
+__global__ void __launch_bounds__(32 * kProgWarps) k_classify_program(
+    Geo G, const FbPrim* __restrict__ prims, const PrimF* __restrict__ primf, const FbInsn* __restrict__ prog,
+    int n_prog, const uint32_t* __restrict__ pool, const int64_t* __restrict__ sb_off,
+    const int32_t* __restrict__ sb_len, int32_t* __restrict__ kind, float* __restrict__ cma,
+    int32_t* __restrict__ blk_off, int32_t* __restrict__ blk_len, uint32_t* __restrict__ blk_pool, int64_t blk_cap,
+    int* __restrict__ cursor) {
+    __shared__ uint32_t s_out[kProgWarps][kProgCap];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t b = blockIdx.x * (int64_t)kProgWarps + warp;
     if (b >= G.nblocks) return;
     const int bk = (int)(b % G.nbz), bj = (int)((b / G.nbz) % G.nby), bi = (int)(b / ((int64_t)G.nbz * G.nby));
     const int B = G.B;
-    double mn = 1.0e30;
-    bool pos = false, neg = false;
-    for (int c = 0; c < 8; ++c) {
-        const double vd = program_eval_d(prims, prog, n_prog, vertex_d(G.x0, (int64_t)bi * B + (c & 1) * B, G.pitch),
-                                         vertex_d(G.y0, (int64_t)bj * B + ((c >> 1) & 1) * B, G.pitch),
-                                         vertex_d(G.z0, (int64_t)bk * B + ((c >> 2) & 1) * B, G.pitch));
-        mn = fmin(mn, fabs(vd));
-        if (vd >= 0.0) pos = true; else neg = true;
+    const int64_t s = ((int64_t)(bi / G.S) * G.nsy + bj / G.S) * G.nsz + bk / G.S;
+    const uint32_t* in = sb_len[s] >= 0 ? pool + sb_off[s] : nullptr;
+    const int n_in = in ? sb_len[s] : n_prog;
+    const double half = 0.5 * B;
+    const double ctr[3] = {G.x0 + (bi * B + half) * G.pitch, G.y0 + (bj * B + half) * G.pitch,
+                           G.z0 + (bk * B + half) * G.pitch};
+    const int n = prune_program(prims, primf, prog, in, n_in, ctr, 1.7320509 * half * G.pitch, s_out[warp]);
+    const uint32_t* list = n >= 0 ? s_out[warp] : in;
+    double v = 1.0e30;
+    bool neg = false;
+    if (lane < 8) {
+        const double x = vertex_d(G.x0, (int64_t)bi * B + (lane & 1) * B, G.pitch);
+        const double y = vertex_d(G.y0, (int64_t)bj * B + ((lane >> 1) & 1) * B, G.pitch);
+        const double z = vertex_d(G.z0, (int64_t)bk * B + ((lane >> 2) & 1) * B, G.pitch);
+        double vd;
+        program_group_d<1>(prims, primf, prog, list, n >= 0 ? n : n_in, &x, &y, &z, &vd);
+        neg = !(vd >= 0.0);
+        v = fmin(1.0e30, fabs(vd));
     }
-    kind[b] = (pos && neg) ? 0 : (mn <= (double)G.margin ? 0 : (neg ? -1 : 1));
-    cma[b] = (float)mn;
+    const unsigned negs = __ballot_sync(0xffffffffu, neg);
+    for (int o = 4; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
+    const int kd = __shfl_sync(0xffffffffu, (negs != 0u && negs != 0xffu) ? 0 : (v <= (double)G.margin ? 0 : (negs ? -1 : 1)), 0);
+    int at = 0;
+    if (lane == 0) {
+        kind[b] = kd;
+        cma[b] = (float)v;
+        // past the pool's end (or int32) nothing more is placed, so the cursor cannot wrap around
+        at = -1;
+        const int64_t limit = blk_cap < (int64_t(1) << 30) ? blk_cap : int64_t(1) << 30;
+        if (kd == 0 && n >= 0 && *(volatile int*)cursor < limit) at = atomicAdd(cursor, n);
+    }
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (kd == 0) {
+        const bool kept = n >= 0 && at >= 0 && (int64_t)at + n <= blk_cap;
+        for (int i = lane; kept && i < n; i += 32) blk_pool[at + i] = s_out[warp][i];
+        if (lane == 0) {
+            blk_off[b] = at;
+            blk_len[b] = kept ? n : -1;
+        }
+    }
 }
 
 // ------------------------------------------------------------------------------------ compaction
@@ -1817,33 +2006,56 @@ __global__ void __launch_bounds__(32 * kLeafWarps, 6) k_leaf(Geo G, const FbPrim
                              kind, blk_off, blk_len, blk_pool, blk_cap, s_prim[warp], s_list[warp], s_acc[warp]);
 }
 
-// Leaf tiles of a general postfix program: float64 per voxel, no culling.
+// Leaf tiles of a general postfix program: float64 per voxel, a warp per 32 V voxels of an active block
+// on the block's pruned program (the whole one where the classification kept none): an assembly's few
+// thousand active blocks then fill the GPU, and V voxels of a lane hide each other's float64 chains (the
+// assembly's leaves 125 us with a warp per block, 46 us with a warp per 128 voxels).
 template <int B>
 __global__ void __launch_bounds__(128) k_leaf_program(Geo G, const FbPrim* __restrict__ prims,
+                                                      const PrimF* __restrict__ primf,
                                                       const FbInsn* __restrict__ prog, int n_prog,
                                                       const int32_t* __restrict__ active,
                                                       const int32_t* __restrict__ count, int64_t capacity,
-                                                      float* __restrict__ tiles) {
-    constexpr int kVox = B * B * B;
+                                                      float* __restrict__ tiles, const int32_t* __restrict__ kind,
+                                                      const int32_t* __restrict__ blk_off,
+                                                      const int32_t* __restrict__ blk_len,
+                                                      const uint32_t* __restrict__ blk_pool, int64_t blk_cap) {
+    constexpr int kVox = B * B * B, V = B == 4 ? 2 : 4, kParts = kVox / (32 * V);
     const int lane = threadIdx.x & 31;
     const int64_t gwarp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    const int64_t n_active = min((int64_t)count[0], capacity);
-    for (int64_t a = gwarp; a < n_active; a += nwarps) {
-        const int64_t blk = active[a];
+    const int64_t n_items = min((int64_t)count[0], capacity) * kParts;
+    for (int64_t w = gwarp; w < n_items; w += nwarps) {
+        const int64_t a = w / kParts, blk = active[a];
+        const int v0 = (int)(w % kParts) * (32 * V) + lane;
         float* out = tiles + a * kVox;
         if (blk < 0 || blk >= G.nblocks) {
-            for (int v = lane; v < kVox; v += 32) out[v] = kBig;
+#pragma unroll
+            for (int k = 0; k < V; ++k) out[v0 + 32 * k] = kBig;
             continue;
         }
-        const int bk = (int)(blk % G.nbz), bj = (int)((blk / G.nbz) % G.nby), bi = (int)(blk / ((int64_t)G.nbz * G.nby));
-        for (int v = lane; v < kVox; v += 32) {
-            const int li = v / (B * B), lj = (v / B) % B, lk = v % B;
-            const double x = rn_add(G.x0, rn_mul((double)(bi * B + li), G.pitch));
-            const double y = rn_add(G.y0, rn_mul((double)(bj * B + lj), G.pitch));
-            const double z = rn_add(G.z0, rn_mul((double)(bk * B + lk), G.pitch));
-            out[v] = (float)program_eval_d(prims, prog, n_prog, x, y, z);
+        const uint32_t* list = nullptr;
+        int n = n_prog;
+        if (kind[blk] == 0) {  // only active blocks have a program of their own
+            const int64_t off = blk_off[blk];
+            const int len = blk_len[blk];
+            if (len >= 0 && off >= 0 && off + len <= blk_cap) {
+                list = blk_pool + off;
+                n = len;
+            }
         }
+        const int bk = (int)(blk % G.nbz), bj = (int)((blk / G.nbz) % G.nby), bi = (int)(blk / ((int64_t)G.nbz * G.nby));
+        double x[V], y[V], z[V], r[V];
+#pragma unroll
+        for (int k = 0; k < V; ++k) {
+            const int v = v0 + 32 * k, li = v / (B * B), lj = (v / B) % B, lk = v % B;
+            x[k] = rn_add(G.x0, rn_mul((double)(bi * B + li), G.pitch));
+            y[k] = rn_add(G.y0, rn_mul((double)(bj * B + lj), G.pitch));
+            z[k] = rn_add(G.z0, rn_mul((double)(bk * B + lk), G.pitch));
+        }
+        program_group_d<V>(prims, primf, prog, list, n, x, y, z, r);
+#pragma unroll
+        for (int k = 0; k < V; ++k) out[v0 + 32 * k] = (float)r[k];
     }
 }
 
@@ -2065,7 +2277,13 @@ int classify_impl(const FbGeom& g, const FbPrim* prims, int n_prims, const FbIns
             G, prims, S.primf, chain, S.pool, S.off + G.ncoarse, S.len + G.ncoarse, kind, cma, S.blk_off, S.blk_len,
             S.blk_pool, P.blk_cap, S.misc + 2);
     } else {
-        k_classify_program<<<fb_div_up(G.nblocks, 128), 128, 0, st>>>(G, prims, chain, n_chain, kind, cma);
+        k_cull_program<<<fb_div_up(G.nsuper, kProgWarps), 32 * kProgWarps, 0, st>>>(
+            G, prims, S.primf, chain, n_chain, S.pool, P.pool_super, P.cap_super, S.off + G.ncoarse, S.len + G.ncoarse);
+        FB_LAUNCH();
+        FB_CUDA(cudaMemsetAsync(S.misc, 0, 256, st));
+        k_classify_program<<<fb_div_up(G.nblocks, kProgWarps), 32 * kProgWarps, 0, st>>>(
+            G, prims, S.primf, chain, n_chain, S.pool, S.off + G.ncoarse, S.len + G.ncoarse, kind, cma, S.blk_off,
+            S.blk_len, S.blk_pool, P.blk_cap, S.misc + 2);
     }
     FB_LAUNCH();
     if (int rc = launch_compact(kind, G.nblocks, active, count, S.status, S.misc, st)) return rc;
@@ -2086,11 +2304,15 @@ int leaf_impl(const FbGeom& g, const FbPrim* prims, int n_prims, const FbInsn* c
     const int64_t* sb_off = S.off + G.ncoarse;
     const int32_t* sb_len = S.len + G.ncoarse;
     if (mode != 1) {
+#define FB_LEAF_PROGRAM(BB)                                                                                  \
+    k_leaf_program<BB><<<grid, 128, 0, st>>>(G, prims, S.primf, chain, n_chain, active, count, capacity, tiles, kind, \
+                                             S.blk_off, S.blk_len, S.blk_pool, P.blk_cap)
         switch (G.B) {
-        case 4: k_leaf_program<4><<<grid, 128, 0, st>>>(G, prims, chain, n_chain, active, count, capacity, tiles); break;
-        case 8: k_leaf_program<8><<<grid, 128, 0, st>>>(G, prims, chain, n_chain, active, count, capacity, tiles); break;
-        default: k_leaf_program<16><<<grid, 128, 0, st>>>(G, prims, chain, n_chain, active, count, capacity, tiles);
+        case 4: FB_LEAF_PROGRAM(4); break;
+        case 8: FB_LEAF_PROGRAM(8); break;
+        default: FB_LEAF_PROGRAM(16);
         }
+#undef FB_LEAF_PROGRAM
     } else {
 #define FB_LEAF(BB, EDGE)                                                                                   \
     k_leaf<BB, EDGE><<<grid, 32 * kLeafWarps, 0, st>>>(G, prims, S.primf, chain, S.pool, sb_off, sb_len, active, \
