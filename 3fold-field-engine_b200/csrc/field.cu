@@ -23,6 +23,7 @@
 // (classification rule), :167-190 (tile order), :277 (ascending compaction); dense input
 // src/field_engine/faltkarna_v1_mesh_to_sdf.py:602-657.
 #include "common.cuh"
+#include "cull.cuh"
 #include "dense.cuh"
 #include "prims.cuh"
 #include <algorithm>
@@ -282,288 +283,18 @@ __global__ void k_sqrt_sum(const float* __restrict__ x, float* __restrict__ out,
         out[i] = sqrt_sum(x[i]);
 }
 
+// sqrt_rn over n inputs (the self-test export fb_sqrt_rn_probe).
+__global__ void k_sqrt_rn(const float* __restrict__ x, float* __restrict__ out, int64_t n) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        out[i] = sqrt_rn(x[i]);
+}
+
 __global__ void k_full_list(uint32_t* __restrict__ list, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) list[i] = (uint32_t)i << 2;
 }
 
 // ------------------------------------------------------------------------------------ culling
-// One interval step of the chain walk.  Returns 0 skip, 1 keep, 2 reset to "set", 3 reset to
-// "set negated".  [alo, ahi] bounds the accumulator over the region.
-__device__ __forceinline__ int interval_step(int op, float k, float plo, float phi, float& alo, float& ahi) {
-    switch (op) {
-    case CH_SET:
-        alo = plo; ahi = phi;
-        return 2;
-    case CH_SETNEG:
-        alo = -phi; ahi = -plo;
-        return 3;
-    case CH_UNION:
-        if (plo > ahi + k) return 0;
-        if (phi < alo - k) { alo = plo; ahi = phi; return 2; }
-        alo = fminf(alo, plo) - 0.25f * k;
-        ahi = fminf(ahi, phi);
-        return 1;
-    case CH_INTERSECT:
-        if (phi < alo - k) return 0;
-        if (plo > ahi + k) { alo = plo; ahi = phi; return 2; }
-        alo = fmaxf(alo, plo);
-        ahi = fmaxf(ahi, phi) + 0.25f * k;
-        return 1;
-    case CH_SUBTRACT:
-        if (-plo < alo - k) return 0;
-        if (-phi > ahi + k) { alo = -phi; ahi = -plo; return 3; }
-        alo = fmaxf(alo, -phi);
-        ahi = fmaxf(ahi, -plo) + 0.25f * k;
-        return 1;
-    default:  // offset
-        alo -= k; ahi -= k;
-        return 1;
-    }
-}
-
-__device__ __forceinline__ int effective_op(uint32_t entry, int op) {
-    const uint32_t mode = entry & 3u;
-    return mode == 1u ? CH_SET : (mode == 2u ? CH_SETNEG : op);
-}
-
-// Interval of one chain element's primitive around (cx, cy, cz) with radius R.
-__device__ __forceinline__ void element_interval(const PrimF& P, float cx, float cy, float cz, float R, float eps,
-                                                 float& lo, float& hi) {
-    const float v = primf_world(P, cx, cy, cz);
-    const float r = fmaf(P.lip, R, eps + 1e-6f * fabsf(v));
-    lo = v - r;
-    hi = v + r;
-}
-
-// A hard (k == 0) union / intersection / subtraction: consecutive ones of the same kind form a
-// run whose result is an order-free min or max of the accumulator and the run's elements.
-__device__ __forceinline__ bool runnable(int op, float k) {
-    return k == 0.f && (op == CH_UNION || op == CH_INTERSECT || op == CH_SUBTRACT);
-}
-
-struct Elem {
-    uint32_t ent;
-    int op;
-    float k;
-    float lo, hi;  // bounds of the value the combine sees (-p for a subtraction)
-};
-
-// The same enclosure from the primitive's bounding ball (PrimF.ball == 1): no evaluation of the
-// primitive, a few loads -- looser by up to the ball's diameter.
-__device__ __forceinline__ void element_interval_ball(const PrimF& P, float cx, float cy, float cz, float R, float eps,
-                                                      float& lo, float& hi) {
-    const float dx = cx - P.p[8], dy = cy - P.p[9], dz = cz - P.p[10];
-    const float d = sqrtf(fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
-    const float k = P.ball_k, rw = P.p[11];
-    const float m = eps + 1e-6f * (k * (d + R + rw) + fabsf(P.off));
-    lo = fmaf(k, d - R - rw, -P.off) - m;
-    hi = fmaf(k, d + R + rw, -P.off) + m;
-}
-
-__device__ __forceinline__ Elem load_elem(const uint32_t* __restrict__ in, int e, const FbInsn* __restrict__ chain,
-                                          const PrimF* __restrict__ primf, float cx, float cy, float cz, float R,
-                                          float eps, bool with_bounds, bool ball = false) {
-    Elem E;
-    E.ent = in ? in[e] : (uint32_t)e << 2;  // a null list is the whole chain in order
-    const FbInsn I = chain[E.ent >> 2];
-    E.op = effective_op(E.ent, I.op);
-    E.k = (float)I.k;
-    E.lo = E.hi = 0.f;
-    if (with_bounds && E.op != CH_OFFSET) {
-        float lo, hi;
-        const PrimF& P = primf[I.arg];
-        if (ball && P.ball != 0.f) element_interval_ball(P, cx, cy, cz, R, eps, lo, hi);
-        else element_interval(P, cx, cy, cz, R, eps, lo, hi);
-        if (E.op == CH_SUBTRACT || E.op == CH_SETNEG) { E.lo = -hi; E.hi = -lo; }
-        else { E.lo = lo; E.hi = hi; }
-    }
-    return E;
-}
-
-// Run decision.  union: result = min(acc, run); an element whose lower bound exceeds
-// H = min(acc_hi, min run hi) is never the minimum and is dropped; when min run hi < acc_lo the
-// accumulator so far is dominated everywhere and dropped (the run restarts the list).
-// intersection / subtraction: the mirror image with max.  All comparisons are strict, so every
-// decision is exact for the float values the bounds enclose.
-struct RunState {
-    float bound;   // H (union) or L (max kinds)
-    bool reset;
-};
-
-__device__ __forceinline__ RunState run_decide(int op, float agg, float alo, float ahi) {
-    RunState r;
-    if (op == CH_UNION) {
-        r.reset = agg < alo;
-        r.bound = r.reset ? agg : fminf(ahi, agg);
-    } else {
-        r.reset = agg > ahi;
-        r.bound = r.reset ? agg : fmaxf(alo, agg);
-    }
-    return r;
-}
-
-__device__ __forceinline__ bool run_keep(int op, const Elem& E, float bound) {
-    return op == CH_UNION ? !(E.lo > bound) : !(E.hi < bound);
-}
-
-// Warp-cooperative chain walk over `in` for the region centred at (cx, cy, cz) with radius R.
-// Hard runs are decided with two warp-parallel passes (aggregate bound, then keep/drop with
-// ballot compaction); other elements (offsets, smooth booleans, sets) step one at a time.
-// Returns the kept count (may exceed cap: then the output is incomplete and must not be used).
-// kBall: bound primitives by their bounding balls where they have one (the coarse level, where
-// every region walks the whole chain).
-template <bool kBall = false>
-__device__ int warp_walk(const uint32_t* __restrict__ in, int n_in, const FbInsn* __restrict__ chain,
-                         const PrimF* __restrict__ primf, float cx, float cy, float cz, float R, float eps,
-                         uint32_t* __restrict__ out, int cap) {
-    const int lane = threadIdx.x & 31;
-    const unsigned below = (1u << lane) - 1u;
-    float alo = 0.f, ahi = 0.f;
-    int n = 0;
-    int i = 0;
-    while (i < n_in) {
-        const Elem head = load_elem(in, i, chain, primf, cx, cy, cz, R, eps, false);
-        if (!runnable(head.op, head.k)) {
-            const Elem E = load_elem(in, i, chain, primf, cx, cy, cz, R, eps, true);
-            float plo = E.lo, phi = E.hi;  // back to the primitive's own bounds
-            if (E.op == CH_SUBTRACT || E.op == CH_SETNEG) { plo = -E.hi; phi = -E.lo; }
-            const int act = interval_step(E.op, E.k, plo, phi, alo, ahi);
-            if (act) {
-                uint32_t rec = E.ent;
-                if (act == 2) { n = 0; rec = (E.ent & ~3u) | 1u; }
-                if (act == 3) { n = 0; rec = (E.ent & ~3u) | 2u; }
-                if (n < cap && lane == 0) out[n] = rec;
-                ++n;
-            }
-            ++i;
-            continue;
-        }
-        const int op = head.op;
-        // pass 1, 32 elements at a time: the run's end (the first element of another kind) and the
-        // aggregate bound of the elements before it.  With ball bounds the same pass also writes the
-        // candidates: elements not beaten by the bound so far (the minimum over everything up to and
-        // including their chunk) -- a superset of those the final bound keeps.
-        float agg = op == CH_UNION ? 3.0e38f : -3.0e38f;
-        int j = n_in;
-        const int n0 = n;
-        for (int b = i; b < n_in; b += 32) {
-            const int e = b + lane;
-            bool same = false;
-            Elem E;
-            if (e < n_in) {
-                E = load_elem(in, e, chain, primf, cx, cy, cz, R, eps, true, kBall);
-                same = e == i || (E.op == op && runnable(E.op, E.k));
-            }
-            const unsigned stop = __ballot_sync(0xffffffffu, e < n_in && !same);
-            const int end = stop ? b + __ffs(stop) - 1 : min(b + 32, n_in);
-            if (e < end) agg = op == CH_UNION ? fminf(agg, E.hi) : fmaxf(agg, E.lo);
-            if (kBall) {
-                float run = agg;
-                for (int o = 16; o > 0; o >>= 1) {
-                    const float t = __shfl_xor_sync(0xffffffffu, run, o);
-                    run = op == CH_UNION ? fminf(run, t) : fmaxf(run, t);
-                }
-                const bool keep = e < end && run_keep(op, E, run);
-                const unsigned kept = __ballot_sync(0xffffffffu, keep);
-                if (keep) {
-                    const int pos = n + __popc(kept & below);
-                    if (pos < cap) out[pos] = E.ent;
-                }
-                n += __popc(kept);
-            }
-            if (stop) {
-                j = end;
-                break;
-            }
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-            const float t = __shfl_xor_sync(0xffffffffu, agg, o);
-            agg = op == CH_UNION ? fminf(agg, t) : fmaxf(agg, t);
-        }
-        RunState rs = run_decide(op, agg, alo, ahi);
-        float klo = 3.0e38f, khi = -3.0e38f;
-        if (kBall) {
-            // pass 1 wrote the candidates (every other element of the run provably loses, so the run's
-            // result is the candidates' result); the exact bounds of the candidates alone give the
-            // run's decision, and the candidates are compacted in place with it
-            const int nc = n - n0;  // candidates at out[n0, n)
-            if (n > cap) {          // overflowed: the region falls back to its parent's list anyway
-                i = j;
-                continue;
-            }
-            float agg2 = op == CH_UNION ? 3.0e38f : -3.0e38f;
-            for (int b = 0; b < nc; b += 32) {
-                if (b + lane < nc) {
-                    const Elem E = load_elem(out + n0, b + lane, chain, primf, cx, cy, cz, R, eps, true);
-                    agg2 = op == CH_UNION ? fminf(agg2, E.hi) : fmaxf(agg2, E.lo);
-                }
-            }
-            for (int o = 16; o > 0; o >>= 1) {
-                const float t = __shfl_xor_sync(0xffffffffu, agg2, o);
-                agg2 = op == CH_UNION ? fminf(agg2, t) : fmaxf(agg2, t);
-            }
-            rs = run_decide(op, agg2, alo, ahi);
-            n = rs.reset ? 0 : n0;  // compaction target: positions never above the ones being read
-            bool first = rs.reset;
-            for (int b = 0; b < nc; b += 32) {
-                bool keep = false;
-                Elem E;
-                if (b + lane < nc) {
-                    E = load_elem(out + n0, b + lane, chain, primf, cx, cy, cz, R, eps, true);
-                    keep = run_keep(op, E, rs.bound);
-                    if (keep) { klo = fminf(klo, E.lo); khi = fmaxf(khi, E.hi); }
-                }
-                const unsigned kept = __ballot_sync(0xffffffffu, keep);  // every read precedes the writes
-                if (keep) {
-                    const int pos = n + __popc(kept & below);
-                    uint32_t rec = E.ent;
-                    if (first && pos == 0) rec = (E.ent & ~3u) | (op == CH_SUBTRACT ? 2u : 1u);
-                    out[pos] = rec;
-                }
-                if (kept) first = false;
-                n += __popc(kept);
-            }
-        } else {
-            if (rs.reset) n = 0;
-            bool first = rs.reset;
-            // pass 2: keep / drop, ballot compaction in chain order
-            for (int b = i; b < j; b += 32) {
-                const int e = b + lane;
-                bool keep = false;
-                Elem E;
-                if (e < j) {
-                    E = load_elem(in, e, chain, primf, cx, cy, cz, R, eps, true);
-                    keep = run_keep(op, E, rs.bound);
-                    if (keep) { klo = fminf(klo, E.lo); khi = fmaxf(khi, E.hi); }
-                }
-                const unsigned kept = __ballot_sync(0xffffffffu, keep);
-                if (keep) {
-                    const int pos = n + __popc(kept & below);
-                    uint32_t rec = E.ent;
-                    if (first && pos == 0) rec = (E.ent & ~3u) | (op == CH_SUBTRACT ? 2u : 1u);
-                    if (pos < cap) out[pos] = rec;
-                }
-                if (kept) first = false;
-                n += __popc(kept);
-            }
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-            klo = fminf(klo, __shfl_xor_sync(0xffffffffu, klo, o));
-            khi = fmaxf(khi, __shfl_xor_sync(0xffffffffu, khi, o));
-        }
-        if (op == CH_UNION) {
-            alo = rs.reset ? klo : fminf(alo, klo);
-            ahi = rs.bound;
-        } else {
-            alo = rs.bound;
-            ahi = rs.reset ? khi : fmaxf(ahi, khi);
-        }
-        i = j;
-    }
-    return n;
-}
-
 // The same walk by one thread (each block's own list in k_classify_blocks): the lanes of a warp
 // walk the same superblock list together, so its loads are broadcasts.
 __device__ int seq_walk(const uint32_t* __restrict__ in, int n_in, const FbInsn* __restrict__ chain,
@@ -3119,6 +2850,16 @@ int fb_sqrt_sum_probe(const float* d_x, float* d_out, int64_t n, void* stream) n
     if (n == 0) return FB_OK;
     const unsigned grid = (unsigned)std::min<int64_t>((n + 255) / 256, 148 * 16);
     k_sqrt_sum<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(d_x, d_out, n);
+    FB_LAUNCH();
+    return FB_OK;
+}
+
+// The canonical evaluations' square root (sqrt_rn) over n device floats, stream-ordered.
+int fb_sqrt_rn_probe(const float* d_x, float* d_out, int64_t n, void* stream) noexcept {
+    if (!d_x || !d_out || n < 0) return FB_INVALID;
+    if (n == 0) return FB_OK;
+    const unsigned grid = (unsigned)std::min<int64_t>((n + 255) / 256, 148 * 16);
+    k_sqrt_rn<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(d_x, d_out, n);
     FB_LAUNCH();
     return FB_OK;
 }

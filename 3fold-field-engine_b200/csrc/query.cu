@@ -2,10 +2,9 @@
 //
 // Recipes (src/field_engine/ikarus_v1/eval_warp.py:478-488 eval_batch, :718-733 gradient_batch):
 //   k_eval_points evaluates the compiled program at float32 points (thread per point).  With a
-//   built field's culling lists (the lists a classification left in its scratch) each point inside
-//   the grid walks only its block's list where the classification kept one, else its superblock's
-//   -- exact for every point of that region, by the same strict-domination argument as the build --
-//   instead of the whole chain.
+//   built field's culling lists (the lists a classification left in its scratch) k_query_warp (few
+//   points) and k_query_sorted (many) cull the superblock's list once more to the points at hand --
+//   exact, by the same strict-domination argument as the build -- instead of walking the whole chain.
 //   k_gradient_points: central differences with step h along each axis, the six offset points
 //   formed in float64 and rounded to float32 as the reference does.
 // Per-block pitch fields (src/field_engine/faltkarna_v1_multires.py:84-104, :384-459):
@@ -13,6 +12,7 @@
 //   k_multires_value answers avstand (trilinear at the brick's own pitch, +-margin outside active
 //   bricks) and k_multires_gradient the brick-clamped central difference.
 #include "common.cuh"
+#include "cull.cuh"
 #include "prims.cuh"
 #include <algorithm>
 #include <cmath>
@@ -64,17 +64,15 @@ struct Accel {  // a built field's culling lists (nullptr pool: walk the whole c
     int64_t blk_cap;
     int blk_all;
     double x0, y0, z0, pitch;
-    int nx, ny, nz, B, S, nsy, nsz, nbx, nby, nbz;
+    int nx, ny, nz, B, S, nsx, nsy, nsz, nbx, nby, nbz;
+    float eps;  // the bounds' float32 slack near the grid, at least the build's own
 };
 
-// The list a point at (x, y, z) walks and its key: block b (0 <= b < nblocks) where the
-// classification kept the block's list, nblocks + superblock for other points inside the grid,
-// nblocks + nsuper (nullptr list) for the whole chain.
-__device__ __forceinline__ int64_t accel_list(const Accel& A, int n_chain, float x, float y, float z,
-                                              const uint32_t*& list, int& len) {
-    const int64_t nblocks = (int64_t)A.nbx * A.nby * A.nbz;
-    const int64_t nsuper = (int64_t)((A.nbx + A.S - 1) / A.S) * A.nsy * A.nsz;
-    if (A.pool) {
+// The list a point at (x, y, z) walks on its own: its block's where the classification kept one, its
+// superblock's elsewhere inside the grid, the whole chain (nullptr) outside.
+__device__ __forceinline__ void accel_list(const Accel& A, int n_chain, float x, float y, float z,
+                                           const uint32_t*& list, int& len) {
+    {
         // the voxel cell containing the point, inside the grid's block range
         const double fx = ((double)x - A.x0) / A.pitch, fy = ((double)y - A.y0) / A.pitch,
                      fz = ((double)z - A.z0) / A.pitch;
@@ -90,93 +88,355 @@ __device__ __forceinline__ int64_t accel_list(const Accel& A, int n_chain, float
                     if (n >= 0 && off >= 0 && off + n <= A.blk_cap) {
                         list = A.blk_pool + off;
                         len = n;
-                        return b;
+                        return;
                     }
                 }
             }
             const int64_t s = ((int64_t)(bi / A.S) * A.nsy + bj / A.S) * A.nsz + bk / A.S;
             list = A.pool + A.sb_off[s];
             len = A.sb_len[s];
-            return nblocks + s;
+            return;
         }
     }
     list = nullptr;
     len = n_chain;
-    return nblocks + nsuper;
-}
-
-__device__ __forceinline__ float eval_accel(const PrimF* primf, const FbInsn* chain, int n_chain, int chain_mode,
-                                            const Accel& A, float x, float y, float z) {
-    if (chain_mode) {
-        const uint32_t* list;
-        int len;
-        accel_list(A, n_chain, x, y, z, list, len);
-        return eval_point(primf, chain, n_chain, 1, list, len, x, y, z);
-    }
-    return eval_point(primf, chain, n_chain, chain_mode, nullptr, n_chain, x, y, z);
 }
 
 __global__ void k_eval_points(const PrimF* __restrict__ primf, const FbInsn* __restrict__ chain, int n_chain,
-                              int chain_mode, Accel A, const float* __restrict__ pts, int64_t n,
-                              float* __restrict__ out) {
+                              int chain_mode, const float* __restrict__ pts, int64_t n, float* __restrict__ out) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        out[i] = eval_accel(primf, chain, n_chain, chain_mode, A, pts[3 * i], pts[3 * i + 1], pts[3 * i + 2]);
+        out[i] = eval_point(primf, chain, n_chain, chain_mode, nullptr, n_chain, pts[3 * i], pts[3 * i + 1], pts[3 * i + 2]);
 }
 
 // Central difference with step h: (f(p + h e_a) - f(p - h e_a)) / (2h) in float32, the offset
 // points formed in float64 and rounded to float32 (eval_warp.py:718-733).  `value` (nullable)
 // also receives f(p).
 __global__ void k_gradient_points(const PrimF* __restrict__ primf, const FbInsn* __restrict__ chain, int n_chain,
-                                  int chain_mode, Accel A, const float* __restrict__ pts, int64_t n, double h,
+                                  int chain_mode, const float* __restrict__ pts, int64_t n, double h,
                                   float* __restrict__ grad, float* __restrict__ value) {
     const float inv = (float)(2.0 * h);
+    auto eval = [&](float x, float y, float z) {
+        return eval_point(primf, chain, n_chain, chain_mode, nullptr, n_chain, x, y, z);
+    };
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const double p[3] = {pts[3 * i], pts[3 * i + 1], pts[3 * i + 2]};
         for (int a = 0; a < 3; ++a) {
             float q[2][3];
             for (int s = 0; s < 2; ++s)
                 for (int c = 0; c < 3; ++c) q[s][c] = (float)(c == a ? p[c] + (s ? -h : h) : p[c]);
-            const float vp = eval_accel(primf, chain, n_chain, chain_mode, A, q[0][0], q[0][1], q[0][2]);
-            const float vm = eval_accel(primf, chain, n_chain, chain_mode, A, q[1][0], q[1][1], q[1][2]);
-            grad[3 * i + a] = (vp - vm) / inv;
+            grad[3 * i + a] = (eval(q[0][0], q[0][1], q[0][2]) - eval(q[1][0], q[1][1], q[1][2])) / inv;
         }
-        if (value) value[i] = eval_accel(primf, chain, n_chain, chain_mode, A, (float)p[0], (float)p[1], (float)p[2]);
+        if (value) value[i] = eval((float)p[0], (float)p[1], (float)p[2]);
     }
 }
 
-// ------------------------------------------------------------------------------------ binned queries
-// Evaluation points sorted by the list they walk, so that the lanes of a warp share one list
-// (broadcast loads, one primitive kind at a time) instead of each lane walking its own.  Point e of
-// a query with `nvar` variants is point e / nvar at variant e % nvar: 0 the point itself, 1 + 2a + s
-// the offset along axis a (s = 0: +h, 1: -h), formed in float64 and rounded to float32 exactly as
-// k_gradient_points forms them, and every value is computed by the same eval_point -- so the
-// results are bit-identical to the unsorted kernels.
-__device__ __forceinline__ void variant_point(const float* __restrict__ pts, int64_t e, int nvar, double h, float& x,
-                                              float& y, float& z) {
-    const int64_t i = e / nvar;
-    const int v = (int)(e - i * nvar);
-    const double p[3] = {pts[3 * i], pts[3 * i + 1], pts[3 * i + 2]};
-    float q[3];
-    for (int c = 0; c < 3; ++c) q[c] = (float)p[c];
-    if (v > 0) {
-        const int a = (v - 1) >> 1, s = (v - 1) & 1;
-        q[a] = (float)(p[a] + (s ? -h : h));
+// ------------------------------------------------------------------------------------ queries near a field
+// A point has NV evaluations: variant 0 the point itself and, with a gradient (NV = 7), 1 + 2a + s the
+// offset along axis a (s = 0: +h, 1: -h), formed in float64 and rounded to float32 as
+// k_gradient_points forms them.  A superblock's list holds for its whole bounding ball (that is what
+// the build culled it for), so the variants of one or of many points of a superblock that lie in the
+// ball share the list -- and a warp first culls it once more, to the ball around just those points
+// (warp_walk_once, the build's own exact rule), before anything is evaluated.  Points outside every ball
+// (beyond the grid's edge) have the whole chain culled to the ball around them in the same way.  What
+// is left -- an offset that leaves its point's ball, non-finite coordinates -- walks its own list
+// (accel_list).  Values are independent of the list they come from, so all paths give the whole
+// chain's values bit for bit.
+constexpr int kQueryWarps = 4;
+constexpr int kQueryCap = 192;  // survivors kept per warp; a longer list is walked as it is
+
+struct Variants {
+    float p[3], plus[3], minus[3];
+    __device__ __forceinline__ float at(int v, int axis) const {
+        float q = p[axis];
+        if (v == 1 + 2 * axis) q = plus[axis];
+        if (v == 2 + 2 * axis) q = minus[axis];
+        return q;
     }
-    x = q[0];
-    y = q[1];
-    z = q[2];
+};
+
+__device__ __forceinline__ Variants load_variants(const float* __restrict__ pts, int64_t i, double h) {
+    Variants V;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const float x = pts[3 * i + a];
+        V.p[a] = (float)(double)x;
+        V.plus[a] = (float)((double)x + h);
+        V.minus[a] = (float)((double)x - h);
+    }
+    return V;
 }
 
-__global__ void k_query_keys(Accel A, int n_chain, const float* __restrict__ pts, int64_t ne, int nvar, double h,
-                             int32_t* __restrict__ keys, int32_t* __restrict__ count) {
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < ne; e += (int64_t)gridDim.x * blockDim.x) {
-        float x, y, z;
-        variant_point(pts, e, nvar, h, x, y, z);
-        const uint32_t* list;
-        int len;
-        const int32_t key = (int32_t)accel_list(A, n_chain, x, y, z, list, len);
-        keys[e] = key;
-        atomicAdd(&count[key], 1);
+// The superblock nearest a point, the bit mask of the point's variants inside that superblock's ball
+// (0 when the point itself is not), and the point's sorting cell: C^3 cells per superblock.
+struct Place {
+    int s, cell;
+    unsigned inside, beyond;  // beyond: outside that ball and outside the grid (the whole chain's)
+};
+
+template <int NV>
+__device__ __forceinline__ Place place_of(const Accel& A, const Variants& V, int C) {
+    const double edge = (double)A.S * A.B, inv = 1.0 / (A.pitch * edge);
+    const double o[3] = {A.x0, A.y0, A.z0};
+    const int ns[3] = {A.nsx, A.nsy, A.nsz};
+    int si[3], ci[3];
+    double ctr[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const double f = ((double)V.p[a] - o[a]) * inv;  // in superblocks
+        const double g = fmin(fmax(f, 0.0), (double)ns[a] - 0.5);  // NaN: 0
+        si[a] = (int)g;
+        ci[a] = min((int)((g - si[a]) * C), C - 1);
+        ctr[a] = o[a] + (si[a] + 0.5) * edge * A.pitch;
+    }
+    const double R = 0.5 * 1.7320508 * edge * A.pitch, R2 = R * R * (1.0 - 1e-5);
+    Place P;
+    P.s = (si[0] * A.nsy + si[1]) * A.nsz + si[2];
+    // boustrophedon inside the superblock: consecutive cells touch, so a warp's points stay close
+    const int y = (ci[0] & 1) ? C - 1 - ci[1] : ci[1];
+    P.cell = (P.s * C + ci[0]) * C * C + y * C + (((ci[0] * C + y) & 1) ? C - 1 - ci[2] : ci[2]);
+    double d2[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const double d = (double)V.p[a] - ctr[a];
+        d2[a] = d * d;
+    }
+    const double sum = d2[0] + d2[1] + d2[2];
+    P.inside = sum <= R2 ? 1u : 0u;  // false for NaN
+    P.beyond = 0u;
+    if (NV > 1 && P.inside) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const double dp = (double)V.plus[a] - ctr[a], dm = (double)V.minus[a] - ctr[a];
+            if (sum - d2[a] + dp * dp <= R2) P.inside |= 2u << (2 * a);
+            if (sum - d2[a] + dm * dm <= R2) P.inside |= 4u << (2 * a);
+        }
+    }
+    const unsigned all = (1u << NV) - 1u;
+    if (P.inside != all) {
+        const int nb[3] = {A.nbx, A.nby, A.nbz};
+        auto out = [&](int a, float x) {
+            const double f = ((double)x - o[a]) * inv * A.S;  // in blocks
+            return !(f >= 0.0 && f <= (double)nb[a]);
+        };
+        unsigned off[3];  // per axis: bit 0 the point, 1 +h, 2 -h beyond the grid along it
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+            off[a] = out(a, V.p[a]) | (NV > 1 ? out(a, V.plus[a]) << 1 | out(a, V.minus[a]) << 2 : 0);
+        const unsigned any = (off[0] | off[1] | off[2]) & 1u;
+        P.beyond = any;
+        if (NV > 1) {
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const unsigned rest = (off[(a + 1) % 3] | off[(a + 2) % 3]) & 1u;
+                P.beyond |= ((off[a] >> 1 & 1u) | rest) << (1 + 2 * a) | ((off[a] >> 2) | rest) << (2 + 2 * a);
+            }
+        }
+        P.beyond &= ~P.inside & all;
+    }
+    return P;
+}
+
+// The largest coordinate of a point's variants where all are finite and far from overflow, else -1.
+template <int NV>
+__device__ __forceinline__ float finite_reach(const Variants& V) {
+    float m = 0.f;
+    bool ok = true;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        m = fmaxf(m, fabsf(V.p[a]));
+        ok &= fabsf(V.p[a]) < 1.0e15f;
+        if (NV > 1) {
+            m = fmaxf(m, fmaxf(fabsf(V.plus[a]), fabsf(V.minus[a])));
+            ok &= fabsf(V.plus[a]) < 1.0e15f && fabsf(V.minus[a]) < 1.0e15f;
+        }
+    }
+    return ok ? m : -1.f;
+}
+
+// A warp's survivors in shared memory.
+struct Survivors {
+    uint32_t ent[kQueryCap];
+    float lo[kQueryCap], hi[kQueryCap];
+};
+
+// `list` (nullptr: the whole chain) culled to the ball (c, R) of points whose coordinates reach `reach`;
+// left as it is where the survivors do not fit.
+__device__ __forceinline__ void cull_to(const uint32_t*& list, int& len, const FbInsn* __restrict__ chain,
+                                        const PrimF* __restrict__ primf, const float* c, float R, float reach,
+                                        float eps, Survivors& out) {
+    const float e = fmaxf(eps, 16.f * 1.2e-7f * reach);  // 16 float32 ulps
+    const int m = warp_walk_once(list, len, chain, primf, c[0], c[1], c[2], R, e, out.ent, out.lo, out.hi, kQueryCap);
+    if (m <= kQueryCap) {
+        list = out.ent;
+        len = m;
+    }
+}
+
+// eval_point out of line: the rare paths' copy.
+static __device__ __noinline__ float eval_list(const PrimF* __restrict__ primf, const FbInsn* __restrict__ chain,
+                                               const uint32_t* list, int len, float x, float y, float z) {
+    return eval_point(primf, chain, len, 1, list, len, x, y, z);
+}
+
+static __device__ __noinline__ float canon_rare(const PrimF& P, float x, float y, float z) {
+    return canon_f(P.type, P.p, x, y, z);
+}
+
+// Two values of one kind, canon_f's operations on primf_world's coordinates.
+template <int T>
+__device__ __forceinline__ void canon_pair(const PrimF& P, const float* x, const float* y, const float* z, float* v) {
+#pragma unroll
+    for (int k = 0; k < 2; ++k) v[k] = canon_f(T, P.p, x[k], y[k], z[k]);
+}
+
+__device__ __forceinline__ void eval_pair(const PrimF& P, const float* qx, const float* qy, const float* qz, float* v) {
+    float x[2], y[2], z[2];
+    if (P.ident) {  // products with 1 and 0 are exact: the sums with the translation are all that rounds
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            x[k] = qx[k] + P.A[3];
+            y[k] = qy[k] + P.A[7];
+            z[k] = qz[k] + P.A[11];
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            x[k] = fmaf(P.A[0], qx[k], fmaf(P.A[1], qy[k], fmaf(P.A[2], qz[k], P.A[3])));
+            y[k] = fmaf(P.A[4], qx[k], fmaf(P.A[5], qy[k], fmaf(P.A[6], qz[k], P.A[7])));
+            z[k] = fmaf(P.A[8], qx[k], fmaf(P.A[9], qy[k], fmaf(P.A[10], qz[k], P.A[11])));
+        }
+    }
+    switch (P.type) {
+    case P_SPHERE: canon_pair<P_SPHERE>(P, x, y, z, v); break;
+    case P_BOX: canon_pair<P_BOX>(P, x, y, z, v); break;
+    case P_CAPSULE: canon_pair<P_CAPSULE>(P, x, y, z, v); break;
+    case P_TORUS: canon_pair<P_TORUS>(P, x, y, z, v); break;
+    default:
+#pragma unroll
+        for (int k = 0; k < 2; ++k) v[k] = canon_rare(P, x[k], y[k], z[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) v[k] = fmaf(P.s, v[k], -P.off);
+}
+
+// The chain's list at the variants of a lane's point, eval_point's values.  Each element is read once;
+// its variants go in pairs through one copy of the code, the accumulators rotating through registers:
+// with the seven variants unrolled inside every kind the loop missed the instruction cache.
+template <int NV>
+__device__ __forceinline__ void eval_variants(const PrimF* __restrict__ primf, const FbInsn* __restrict__ chain,
+                                              const uint32_t* list, int len, const Variants& V, float* acc) {
+    constexpr int kPairs = (NV + 1) / 2;  // pair 0 the point itself (twice), pair 1 + a the offsets along axis a
+    float r[2 * kPairs];
+#pragma unroll
+    for (int k = 0; k < 2 * kPairs; ++k) r[k] = 0.f;
+    for (int i = 0; i < len; ++i) {
+        const uint32_t e = list ? list[i] : (uint32_t)i << 2;
+        const FbInsn I = chain[e >> 2];
+        const int op = effective_op(e, I.op);
+        const float kk = (float)I.k;
+        if (op == CH_OFFSET) {
+#pragma unroll
+            for (int k = 0; k < 2 * kPairs; ++k) r[k] -= kk;
+            continue;
+        }
+        const PrimF& P = primf[I.arg];
+#pragma unroll 1
+        for (int j = 0; j < kPairs; ++j) {
+            float qx[2], qy[2], qz[2], v[2];
+            qx[0] = j == 1 ? V.plus[0] : V.p[0];
+            qy[0] = j == 2 ? V.plus[1] : V.p[1];
+            qz[0] = j == 3 ? V.plus[2] : V.p[2];
+            qx[1] = j == 1 ? V.minus[0] : V.p[0];
+            qy[1] = j == 2 ? V.minus[1] : V.p[1];
+            qz[1] = j == 3 ? V.minus[2] : V.p[2];
+            eval_pair(P, qx, qy, qz, v);
+            float a0 = r[0], a1 = r[1];
+            if (kk == 0.f && op == CH_UNION) {
+                a0 = sel_min(a0, v[0]);
+                a1 = sel_min(a1, v[1]);
+            } else {
+                a0 = chain_apply(op, a0, v[0], kk);
+                a1 = chain_apply(op, a1, v[1], kk);
+            }
+#pragma unroll
+            for (int k = 0; k + 2 < 2 * kPairs; ++k) r[k] = r[k + 2];
+            r[2 * kPairs - 2] = a0;
+            r[2 * kPairs - 1] = a1;
+        }
+    }
+    acc[0] = r[0];
+#pragma unroll
+    for (int k = 1; k < NV; ++k) acc[k] = r[k + 1];
+}
+
+__device__ __forceinline__ void write_point(int64_t i, const float* v, float inv, float* __restrict__ grad,
+                                            float* __restrict__ value) {
+    if (grad) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) grad[3 * i + a] = (v[1 + 2 * a] - v[2 + 2 * a]) / inv;
+    }
+    if (value) value[i] = v[0];
+}
+
+// A warp per point, for few points: no sorting passes.  The superblock's list is culled to the ball
+// around the point's variants (a handful of elements remain), and lane v evaluates variant v.  Bound by
+// the latency of the culling's loads and reductions: 1000 points of a 64^3 field in 9 us, against 55 us
+// in eight kernels when all 7000 evaluations were sorted by the list that each walked.
+template <int NV>
+__global__ void __launch_bounds__(32 * kQueryWarps) k_query_warp(const PrimF* __restrict__ primf,
+                                                                 const FbInsn* __restrict__ chain, int n_chain,
+                                                                 Accel A, const float* __restrict__ pts, int64_t n,
+                                                                 double h, float* __restrict__ grad,
+                                                                 float* __restrict__ value) {
+    __shared__ Survivors s_list[kQueryWarps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const float inv = (float)(2.0 * h);
+    const int64_t nwarps = (int64_t)gridDim.x * kQueryWarps;
+    for (int64_t i = blockIdx.x * (int64_t)kQueryWarps + warp; i < n; i += nwarps) {
+        const Variants V = load_variants(pts, i, h);
+        const Place P = place_of<NV>(A, V, 1);
+        const uint32_t* list = A.pool + A.sb_off[P.s];
+        int len = A.sb_len[P.s];
+        const float reach = finite_reach<NV>(V);
+        // else the whole chain, culled to the ball around all variants
+        const bool ball = (P.inside & 1u) && !P.beyond;
+        if (ball || reach >= 0.f) {
+            float R = 0.f;
+            if (NV > 1) {
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    if (!ball || (P.inside & (2u << (2 * a)))) R = fmaxf(R, fabsf(V.plus[a] - V.p[a]));
+                    if (!ball || (P.inside & (4u << (2 * a)))) R = fmaxf(R, fabsf(V.minus[a] - V.p[a]));
+                }
+            }
+            R *= 1.00001f;
+            if (!ball) {
+                list = nullptr;
+                len = n_chain;
+            }
+            cull_to(list, len, chain, primf, V.p, R, ball ? 0.f : reach, A.eps, s_list[warp]);
+        }
+        __syncwarp();
+        float r = 0.f;
+        if (lane < NV) {
+            const float x = V.at(lane, 0), y = V.at(lane, 1), z = V.at(lane, 2);
+            if (ball ? !((P.inside >> lane) & 1u) : reach < 0.f) accel_list(A, n_chain, x, y, z, list, len);
+            r = eval_list(primf, chain, list, len, x, y, z);
+        }
+        float v[NV];
+#pragma unroll
+        for (int k = 0; k < NV; ++k) v[k] = __shfl_sync(0xffffffffu, r, k);
+        if (lane == 0) write_point(i, v, inv, NV > 1 ? grad : nullptr, value);
+        __syncwarp();
+    }
+}
+
+// A point's sorting cell (outside the grid: the nearest one) and its rank among the cell's points.
+__global__ void k_query_keys(Accel A, const float* __restrict__ pts, int64_t n, int C, int2* __restrict__ keys,
+                             int32_t* __restrict__ count) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const int32_t key = place_of<1>(A, load_variants(pts, i, 0.0), C).cell;
+        keys[i] = make_int2(key, atomicAdd(&count[key], 1));
     }
 }
 
@@ -252,70 +512,175 @@ __global__ void k_scan_add(int32_t* __restrict__ data, int64_t n, const int32_t*
         data[i] += tile_sums[i / kScanTile];
 }
 
-// cursor[key] starts at the key's first sorted position and ends past its last.
-__global__ void k_query_scatter(const int32_t* __restrict__ keys, int64_t ne, int32_t* __restrict__ cursor,
+// start[key] is the key's first sorted position.
+__global__ void k_query_scatter(const int2* __restrict__ keys, int64_t n, const int32_t* __restrict__ start,
                                 int32_t* __restrict__ order) {
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < ne; e += (int64_t)gridDim.x * blockDim.x)
-        order[atomicAdd(&cursor[keys[e]], 1)] = (int32_t)e;
-}
-
-__global__ void k_query_eval_sorted(const PrimF* __restrict__ primf, const FbInsn* __restrict__ chain, int n_chain,
-                                    Accel A, const float* __restrict__ pts, int64_t ne, int nvar, double h,
-                                    const int32_t* __restrict__ order, float* __restrict__ vals) {
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < ne; t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t e = order[t];
-        float x, y, z;
-        variant_point(pts, e, nvar, h, x, y, z);
-        const uint32_t* list;
-        int len;
-        accel_list(A, n_chain, x, y, z, list, len);
-        vals[e] = eval_point(primf, chain, n_chain, 1, list, len, x, y, z);
-    }
-}
-
-// value = variant 0, gradient component a = (v(1 + 2a) - v(2 + 2a)) / (2h), k_gradient_points' arithmetic.
-__global__ void k_query_combine(const float* __restrict__ vals, int64_t n, double h, float* __restrict__ grad,
-                                float* __restrict__ value) {
-    const float inv = (float)(2.0 * h);
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const float* v = vals + 7 * i;
-        for (int a = 0; a < 3; ++a) grad[3 * i + a] = (v[1 + 2 * a] - v[2 + 2 * a]) / inv;
-        if (value) value[i] = v[0];
+        const int2 k = keys[i];
+        order[start[k.x] + k.y] = (int32_t)i;
     }
 }
 
-struct BinnedPlan {
-    int64_t ne, nbins, ntiles;
-    int64_t keys, order, vals, count, tiles, total;
+// A thread per point in sorted order.  The warp's points of one superblock form a group: its list is
+// culled to the ball around the group's variants, then every lane evaluates its NV variants on what is
+// left.  Variants outside the ball are handed out to the lanes afterwards, each on its own list.
+// Bound by instruction issue and the latencies of 20 warps per SM (52 % of issue slots, 30 of 32
+// lanes): 10^6 points with gradients on a 256^3 field of 576 elements in 445 us, against 2680 us for
+// 7 10^6 sorted evaluations on the whole superblock lists (and 1100 us for their keys and scatter, which
+// go by points now: 24 us).  Groups are kept to one superblock: one group of far points in a warp, whose
+// ball nothing is culled from, took 600 us by itself.
+template <int NV>
+__global__ void __launch_bounds__(32 * kQueryWarps, 5) k_query_sorted(const PrimF* __restrict__ primf,
+                                                                   const FbInsn* __restrict__ chain, int n_chain,
+                                                                   Accel A, const float* __restrict__ pts, int64_t n,
+                                                                   double h, const int32_t* __restrict__ order,
+                                                                   float* __restrict__ grad,
+                                                                   float* __restrict__ value) {
+    __shared__ Survivors s_list[kQueryWarps];
+    __shared__ uint8_t s_item[kQueryWarps][32 * NV];
+    __shared__ float s_val[kQueryWarps][32 * NV];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const float inv = (float)(2.0 * h);
+    const int64_t nwarps = (int64_t)gridDim.x * kQueryWarps;
+    for (int64_t w = blockIdx.x * (int64_t)kQueryWarps + warp; w * 32 < n; w += nwarps) {
+        const bool live = w * 32 + lane < n;
+        const int64_t i = live ? order[w * 32 + lane] : 0;
+        const Variants V = load_variants(pts, i, h);
+        const Place P = place_of<NV>(A, V, 1);
+        float r[NV];
+#pragma unroll
+        for (int k = 0; k < NV; ++k) r[k] = 0.f;
+        // groups: the variants in one superblock's ball, then those beyond the grid nearest to one
+        const float reach = finite_reach<NV>(V);
+        const bool ball = P.inside & 1u;
+        const unsigned beyond = live && reach >= 0.f ? P.beyond : 0u;
+        unsigned todo = __ballot_sync(0xffffffffu, live && ball), after = __ballot_sync(0xffffffffu, beyond != 0u);
+        while (todo | after) {
+            const bool whole = !todo;
+            const int s = __shfl_sync(0xffffffffu, P.s, __ffs(whole ? after : todo) - 1);
+            const bool in = (whole ? beyond != 0u : live && ball) && P.s == s;
+            const unsigned mask = !in ? 0u : (whole ? beyond : P.inside);
+            float lo[3], hi[3];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const unsigned fixed = mask & ~(6u << (2 * a));  // variants at the point's own coordinate a
+                lo[a] = fixed ? V.p[a] : 3.0e38f;
+                hi[a] = fixed ? V.p[a] : -3.0e38f;
+                if (NV > 1) {
+                    if (mask & (2u << (2 * a))) { lo[a] = fminf(lo[a], V.plus[a]); hi[a] = fmaxf(hi[a], V.plus[a]); }
+                    if (mask & (4u << (2 * a))) { lo[a] = fminf(lo[a], V.minus[a]); hi[a] = fmaxf(hi[a], V.minus[a]); }
+                }
+            }
+            float c[3], d = 0.f;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                for (int o = 16; o > 0; o >>= 1) {
+                    lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
+                    hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
+                }
+                c[a] = 0.5f * lo[a] + 0.5f * hi[a];
+                const float e = fmaxf(hi[a] - c[a], c[a] - lo[a]);
+                d = fmaf(e, e, d);
+            }
+            const float R = sqrtf(d) * 1.00001f;
+            const uint32_t* list = nullptr;  // the whole chain
+            int len = n_chain;
+            float far = 0.f;
+            if (whole) {
+                far = in ? reach : 0.f;
+                for (int o = 16; o > 0; o >>= 1) far = fmaxf(far, __shfl_xor_sync(0xffffffffu, far, o));
+            } else {
+                list = A.pool + A.sb_off[s];
+                len = A.sb_len[s];
+            }
+            cull_to(list, len, chain, primf, c, R, far, A.eps, s_list[warp]);
+            float acc[NV];
+            eval_variants<NV>(primf, chain, list, len, V, acc);
+#pragma unroll
+            for (int k = 0; k < NV; ++k)
+                if ((mask >> k) & 1u) r[k] = acc[k];
+            const unsigned done = __ballot_sync(0xffffffffu, in);
+            if (whole) after &= ~done;
+            else todo &= ~done;
+            __syncwarp();
+        }
+        // variants left over
+        const unsigned left = live ? ~(P.inside | beyond) & ((1u << NV) - 1u) : 0u;
+        int before = __popc(left);
+        const int mine = before;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, before, o);
+            if (lane >= o) before += y;
+        }
+        const int total = __shfl_sync(0xffffffffu, before, 31);
+        if (total) {
+            before -= mine;
+            for (unsigned b = left; b; b &= b - 1) s_item[warp][before++] = (uint8_t)(lane * 8 + __ffs(b) - 1);
+            __syncwarp();
+            for (int t = 0; t < total; t += 32) {
+                const int item = t + lane < total ? s_item[warp][t + lane] : 0;
+                const int own = item >> 3, v = item & 7;
+                float q[3];
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    q[a] = __shfl_sync(0xffffffffu, V.p[a], own);
+                    const float qp = __shfl_sync(0xffffffffu, V.plus[a], own), qm = __shfl_sync(0xffffffffu, V.minus[a], own);
+                    if (v == 1 + 2 * a) q[a] = qp;
+                    if (v == 2 + 2 * a) q[a] = qm;
+                }
+                if (t + lane < total) {
+                    const uint32_t* list;
+                    int len;
+                    accel_list(A, n_chain, q[0], q[1], q[2], list, len);
+                    s_val[warp][own * NV + v] = eval_list(primf, chain, list, len, q[0], q[1], q[2]);
+                }
+                __syncwarp();
+            }
+#pragma unroll
+            for (int k = 0; k < NV; ++k)
+                if ((left >> k) & 1u) r[k] = s_val[warp][lane * NV + k];
+            __syncwarp();
+        }
+        if (live) write_point(i, r, inv, NV > 1 ? grad : nullptr, value);
+    }
+}
+
+// Up to kWarpPoints points go a warp per point, without scratch; more are sorted first.  Values and
+// gradients, a warp per point against sorted points: 32 000 points 94 / 93 us (64^3 field of 54
+// elements), 143 / 204 us (256^3, 576) and 151 / 249 us (300^3, 787); 64 000 points 179 / 84, 260 / 193
+// and 265 / 240 us: the lines cross between 32 000 and 64 000.
+constexpr int64_t kWarpPoints = 40960;
+
+struct SortedPlan {
+    int64_t nbins, ntiles;
+    int C;  // sorting cells per superblock edge
+    int64_t keys, order, count, tiles, total;
 };
 
-BinnedPlan binned_plan(int64_t n, int nvar, int64_t nbins) {
-    BinnedPlan p{};
-    auto al = [](int64_t b) { return (b + 255) / 256 * 256; };
-    p.ne = n * nvar;
-    p.nbins = nbins;
-    p.ntiles = (nbins + kScanTile - 1) / kScanTile;
-    int64_t at = 0;
-    p.keys = at; at += al(p.ne * 4);
-    p.order = at; at += al(p.ne * 4);
-    p.vals = at; at += al(p.ne * 4);
-    p.count = at; at += al(nbins * 4);
-    p.tiles = at; at += al(p.ntiles * 4);
-    p.total = at;
-    return p;
-}
+constexpr int64_t kMaxBins = int64_t(kScanTile) * kScanTile;  // one tile-sum CTA covers them
+constexpr int64_t kMaxSortedPoints = int64_t(1) << 31;        // sorted positions are int32
 
-int64_t accel_bins(const int32_t* dims) {
+// false: that grid or that many points are not sorted.
+bool sorted_plan(const int32_t* dims, int64_t n, SortedPlan& p) {
     const int B = dims[3];
-    if (B < 1) return -1;
+    if (B < 1 || n >= kMaxSortedPoints) return false;
     const int64_t nbx = (dims[0] + B - 1) / B, nby = (dims[1] + B - 1) / B, nbz = (dims[2] + B - 1) / B;
     const int64_t S = std::max(1, fb_super_edge(dims[0], dims[1], dims[2]) / B);
     const int64_t ns = ((nbx + S - 1) / S) * ((nby + S - 1) / S) * ((nbz + S - 1) / S);
-    return nbx * nby * nbz + ns + 1;
+    for (p.C = 4; p.C > 1 && ns * p.C * p.C * p.C > kMaxBins; p.C /= 2) {
+    }
+    p.nbins = ns * p.C * p.C * p.C;
+    if (ns < 1 || p.nbins > kMaxBins) return false;
+    auto al = [](int64_t b) { return (b + 255) / 256 * 256; };
+    p.ntiles = (p.nbins + kScanTile - 1) / kScanTile;
+    int64_t at = 0;
+    p.keys = at; at += al(n * 8);
+    p.order = at; at += al(n * 4);
+    p.count = at; at += al(p.nbins * 4);
+    p.tiles = at; at += al(p.ntiles * 4);
+    p.total = at;
+    return true;
 }
-
-constexpr int64_t kMaxBins = int64_t(kScanTile) * kScanTile;  // one tile-sum CTA covers them
-constexpr int64_t kMaxBinnedPoints = int64_t(1) << 31;          // sorted positions are int32
 
 // ------------------------------------------------------------------------------------ multires
 struct Multi {
@@ -672,14 +1037,13 @@ int fb_grid_pairs_device(const float* d_params, int32_t n_leaves, const float* d
 // whole chain / program.
 int fb_query_prepare(const FbPrim* d_prims, int32_t n_prims, void* d_primf, void* stream) noexcept;
 
-// Scratch bytes of the sorted query path for n points (with_grad: value + gradient, 7 evaluations
-// per point) on an accelerated grid of dims (nx, ny, nz, B); -1 when that grid takes the unsorted path.
+// Scratch bytes of the sorted query path for n points on an accelerated grid of dims (nx, ny, nz, B); 0
+// or -1: the query takes a path without scratch (few points; a grid that is not sorted).
 int64_t fb_query_scratch_bytes(const int32_t* accel_dims, int64_t n, int32_t with_grad) noexcept {
-    if (!accel_dims || n < 0) return -1;
-    const int64_t nbins = accel_bins(accel_dims);
-    const int nvar = with_grad ? 7 : 1;
-    if (nbins <= 0 || nbins > kMaxBins || n * nvar >= kMaxBinnedPoints) return -1;
-    return binned_plan(n, nvar, nbins).total;
+    (void)with_grad;
+    SortedPlan P;
+    if (!accel_dims || n < 0 || !sorted_plan(accel_dims, n, P)) return -1;
+    return n <= kWarpPoints ? 0 : P.total;
 }
 
 int fb_query_points_device(const void* d_primf, const FbInsn* d_chain, int32_t n_chain, int32_t mode,
@@ -700,6 +1064,7 @@ int fb_query_points_device(const void* d_primf, const FbInsn* d_chain, int32_t n
         A.nx = accel_dims[0]; A.ny = accel_dims[1]; A.nz = accel_dims[2]; A.B = accel_dims[3];
         A.nbx = (A.nx + A.B - 1) / A.B; A.nby = (A.ny + A.B - 1) / A.B; A.nbz = (A.nz + A.B - 1) / A.B;
         A.S = std::max(1, fb_super_edge(A.nx, A.ny, A.nz) / A.B);
+        A.nsx = (A.nbx + A.S - 1) / A.S;
         A.nsy = (A.nby + A.S - 1) / A.S;
         A.nsz = (A.nbz + A.S - 1) / A.S;
         if (blk_off && blk_len && blk_pool && blk_cap > 0 && (blk_all || d_kind)) {
@@ -712,44 +1077,61 @@ int fb_query_points_device(const void* d_primf, const FbInsn* d_chain, int32_t n
         }
     }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int grid = (int)std::min<int64_t>((n + 127) / 128, (int64_t)fb_sm_count() * 16);
     const PrimF* primf = static_cast<const PrimF*>(d_primf);
-    const int nvar = d_grad ? 7 : 1;
-    const int64_t nbins = A.pool ? accel_bins(accel_dims) : -1;
-    if (d_scratch && A.pool && nbins > 0 && nbins <= kMaxBins && n * nvar < kMaxBinnedPoints) {
-        const BinnedPlan P = binned_plan(n, nvar, nbins);
-        if (scratch_len < P.total) return FB_INVALID;
-        char* b = static_cast<char*>(d_scratch);
-        int32_t* keys = reinterpret_cast<int32_t*>(b + P.keys);
-        int32_t* order = reinterpret_cast<int32_t*>(b + P.order);
-        float* vals = d_grad ? reinterpret_cast<float*>(b + P.vals) : d_value;
-        int32_t* count = reinterpret_cast<int32_t*>(b + P.count);
-        int32_t* tiles = reinterpret_cast<int32_t*>(b + P.tiles);
-        const int ge = (int)std::min<int64_t>((P.ne + 255) / 256, (int64_t)fb_sm_count() * 16);
-        FB_CUDA(cudaMemsetAsync(count, 0, nbins * 4, st));
-        k_query_keys<<<ge, 256, 0, st>>>(A, n_chain, d_points, P.ne, nvar, h, keys, count);
-        FB_LAUNCH();
-        k_scan_tiles<<<(unsigned)P.ntiles, kScanThreads, 0, st>>>(count, nbins, tiles);
-        FB_LAUNCH();
-        k_scan_sums<<<1, kScanThreads, 0, st>>>(tiles, (int)P.ntiles);
-        FB_LAUNCH();
-        k_scan_add<<<(int)std::min<int64_t>((nbins + 255) / 256, (int64_t)fb_sm_count() * 16), 256, 0, st>>>(
-            count, nbins, tiles);
-        FB_LAUNCH();
-        k_query_scatter<<<ge, 256, 0, st>>>(keys, P.ne, count, order);
-        FB_LAUNCH();
-        k_query_eval_sorted<<<ge, 256, 0, st>>>(primf, d_chain, n_chain, A, d_points, P.ne, nvar, h, order, vals);
-        FB_LAUNCH();
-        if (d_grad) {
-            k_query_combine<<<grid, 128, 0, st>>>(vals, n, h, d_grad, d_value);
+    if (A.pool) {
+        // 16 float32 ulps of the largest coordinate a superblock's ball reaches: the build's slack
+        float far = 0.f;
+        const double reach = (A.S * A.B + 1) * A.pitch;
+        const double lo[3] = {A.x0, A.y0, A.z0};
+        const int ext[3] = {A.nbx * A.B, A.nby * A.B, A.nbz * A.B};
+        for (int a = 0; a < 3; ++a)
+            far = std::max(far, (float)std::max(std::fabs(lo[a] - reach), std::fabs(lo[a] + ext[a] * A.pitch + reach)));
+        A.eps = 16.f * (std::nextafter(far, 3.4e38f) - far);
+        SortedPlan P;
+        if (d_scratch && n > kWarpPoints && sorted_plan(accel_dims, n, P)) {
+            if (scratch_len < P.total) return FB_INVALID;
+            char* b = static_cast<char*>(d_scratch);
+            int2* keys = reinterpret_cast<int2*>(b + P.keys);
+            int32_t* order = reinterpret_cast<int32_t*>(b + P.order);
+            int32_t* count = reinterpret_cast<int32_t*>(b + P.count);
+            int32_t* tiles = reinterpret_cast<int32_t*>(b + P.tiles);
+            const int ge = (int)std::min<int64_t>((n + 255) / 256, (int64_t)fb_sm_count() * 16);
+            FB_CUDA(cudaMemsetAsync(count, 0, P.nbins * 4, st));
+            k_query_keys<<<ge, 256, 0, st>>>(A, d_points, n, P.C, keys, count);
             FB_LAUNCH();
+            k_scan_tiles<<<(unsigned)P.ntiles, kScanThreads, 0, st>>>(count, P.nbins, tiles);
+            FB_LAUNCH();
+            k_scan_sums<<<1, kScanThreads, 0, st>>>(tiles, (int)P.ntiles);
+            FB_LAUNCH();
+            k_scan_add<<<(int)std::min<int64_t>((P.nbins + 255) / 256, (int64_t)fb_sm_count() * 16), 256, 0, st>>>(
+                count, P.nbins, tiles);
+            FB_LAUNCH();
+            k_query_scatter<<<ge, 256, 0, st>>>(keys, n, count, order);
+            FB_LAUNCH();
+            const int gs = (int)std::min<int64_t>((n + 127) / 128, (int64_t)fb_sm_count() * 64);
+            if (d_grad)
+                k_query_sorted<7><<<gs, 32 * kQueryWarps, 0, st>>>(primf, d_chain, n_chain, A, d_points, n, h, order,
+                                                                   d_grad, d_value);
+            else
+                k_query_sorted<1><<<gs, 32 * kQueryWarps, 0, st>>>(primf, d_chain, n_chain, A, d_points, n, 0.0, order,
+                                                                   nullptr, d_value);
+            FB_LAUNCH();
+            return FB_OK;
         }
+        const int gw = (int)std::min<int64_t>((n + kQueryWarps - 1) / kQueryWarps, (int64_t)fb_sm_count() * 64);
+        if (d_grad)
+            k_query_warp<7><<<gw, 32 * kQueryWarps, 0, st>>>(primf, d_chain, n_chain, A, d_points, n, h, d_grad, d_value);
+        else
+            k_query_warp<1><<<gw, 32 * kQueryWarps, 0, st>>>(primf, d_chain, n_chain, A, d_points, n, 0.0, nullptr,
+                                                             d_value);
+        FB_LAUNCH();
         return FB_OK;
     }
+    const int grid = (int)std::min<int64_t>((n + 127) / 128, (int64_t)fb_sm_count() * 16);
     if (d_grad) {
-        k_gradient_points<<<grid, 128, 0, st>>>(primf, d_chain, n_chain, mode, A, d_points, n, h, d_grad, d_value);
+        k_gradient_points<<<grid, 128, 0, st>>>(primf, d_chain, n_chain, mode, d_points, n, h, d_grad, d_value);
     } else {
-        k_eval_points<<<grid, 128, 0, st>>>(primf, d_chain, n_chain, mode, A, d_points, n, d_value);
+        k_eval_points<<<grid, 128, 0, st>>>(primf, d_chain, n_chain, mode, d_points, n, d_value);
     }
     return cudaGetLastError() == cudaSuccess ? FB_OK : FB_RUNTIME;
 }

@@ -190,6 +190,8 @@ int fb_compact_timeout_probe(const int32_t* d_kind, int64_t n, int32_t* d_active
  * evaluations use (a Newton step from the approximate reciprocal square root): d_out[i] = that root
  * of d_x[i] for n device floats, stream-ordered.  Inputs are sums of squares (>= 0, or NaN). */
 int fb_sqrt_sum_probe(const float* d_x, float* d_out, int64_t n, void* stream);
+/* The canonical forms' square root (sqrtf's bits for every non-negative float), the same way. */
+int fb_sqrt_rn_probe(const float* d_x, float* d_out, int64_t n, void* stream);
 /* No counterpart in the reference.  Self-test of the quotient the 8^3 leaf tiles use for the sphere's
  * difference form (a Newton step from the approximate reciprocal): d_out[i] = d_num[i] / d_den[i] for
  * n device floats, d_den[i] > 0, stream-ordered. */
@@ -317,9 +319,9 @@ int fb_query_points_device(const void* d_primf, const fb_insn* d_chain, int32_t 
                            const int32_t* blk_off, const int32_t* blk_len, const uint32_t* blk_pool, int64_t blk_cap,
                            int32_t blk_all, const float* d_points, int64_t n, double h, float* d_value, float* d_grad,
                            void* d_scratch, int64_t scratch_len, void* stream);
-/* Scratch of the sorted query path (evaluation points sorted by the culled list they walk, so a
- * warp's lanes share one list); -1 when the grid takes the unsorted path.  No reference
- * counterpart: an execution strategy of fb_query_points_device, same results bit for bit. */
+/* Scratch of the sorted query path (points sorted by cell, so a warp's points share one culled list);
+ * 0 or -1 when that query takes a path without scratch (few points; a grid that is not sorted).  No
+ * reference counterpart: an execution strategy of fb_query_points_device, same results bit for bit. */
 int64_t fb_query_scratch_bytes(const int32_t* accel_dims, int64_t n, int32_t with_grad);
 
 /* Replace the per-block-pitch field's lattices and its avstand / gradient queries,
