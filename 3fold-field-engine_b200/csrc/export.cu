@@ -151,15 +151,6 @@ __device__ __forceinline__ int cube_triangles(const CubeLoops& L) {
     return __popc(L.cross) - 2 * loops;
 }
 
-// Value at global voxel (x, y, z) inside the grid: tile value, or -BIG / +BIG by the block's kind.
-__device__ __forceinline__ float voxel_value(const McField& F, int64_t x, int64_t y, int64_t z) {
-    const int B = F.B;
-    const int64_t blk = ((x / B) * F.nby + y / B) * F.nbz + z / B;
-    const int32_t s = F.slot[blk];
-    if (s >= 0) return F.tiles[(int64_t)s * B * B * B + ((x % B) * B + (y % B)) * B + (z % B)];
-    return F.kind[blk] < 0 ? -F.big : F.big;
-}
-
 // World position of the vertex on edge (p, axis), p the edge's lower end.
 __device__ __forceinline__ void edge_vertex(const McField& F, int64_t px, int64_t py, int64_t pz, int a, double g0,
                                             double g1, float* out) {
@@ -171,28 +162,133 @@ __device__ __forceinline__ void edge_vertex(const McField& F, int64_t px, int64_
     out[2] = (float)__dadd_rn(F.oz, __dmul_rn(F.pitch, p[2]));
 }
 
-// Vertex id of edge (p, axis): owner block, slot, popcount below the slot.  -1 if the edge has no
-// vertex (never for the edges of a cube's loops).
-__device__ int64_t vertex_id(const McField& F, int64_t px, int64_t py, int64_t pz, int a, const uint32_t* bits,
-                             const int32_t* wpre, const int32_t* voff, int64_t W) {
-    const int B = F.B;
-    int64_t blk = ((px / B) * F.nby + py / B) * F.nbz + pz / B;
-    int32_t s = F.slot[blk];
-    int64_t sl;
+// Triangles of the cubes that need no face decision, by the eight corners' inside bits: the loops of
+// cube_loops fanned as the emit pass fans them, three edges a triangle.  kAmbiguous marks the corner
+// patterns with a face of four crossings, whose loops depend on the values.
+constexpr int kAmbiguous = 255;
+constexpr int kMaxTableTris = 4;  // 12 crossing edges in four loops of three; any other split has fewer loops to fan
+
+struct CubeTable {
+    uint8_t ntri[256];
+    uint8_t edge[256][16];
+};
+
+constexpr int c_edge_corner0(int e) {
+    const int a = e >> 2, w = e & 3;
+    return a == 0 ? ((w & 1) << 1) | ((w >> 1) << 2) : (a == 1 ? (w & 1) | ((w >> 1) << 2) : (w & 1) | ((w >> 1) << 1));
+}
+
+constexpr int c_edge_of(int ca, int cb) {
+    const int x = ca ^ cb, d = x == 1 ? 0 : (x == 2 ? 1 : 2), c = ca & cb;
+    const int w = d == 0 ? ((c >> 1) & 1) | (((c >> 2) & 1) << 1)
+                         : (d == 1 ? (c & 1) | (((c >> 2) & 1) << 1) : (c & 1) | (((c >> 1) & 1) << 1));
+    return d * 4 + w;
+}
+
+constexpr unsigned c_edge_faces(int e) {
+    unsigned m = 0;
+    for (int b = 0; b < 3; ++b)
+        if (b != (e >> 2)) m |= 1u << (b * 2 + ((c_edge_corner0(e) >> b) & 1));
+    return m;
+}
+
+constexpr CubeTable make_cube_table() {
+    CubeTable T{};
+    for (int in = 0; in < 256; ++in) {
+        int next[12] = {-1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1};
+        unsigned cross = 0;
+        bool ambiguous = false;
+        for (int e = 0; e < 12; ++e) {
+            const int c0 = c_edge_corner0(e), c1 = c0 | (1 << (e >> 2));
+            cross |= (unsigned)(((in >> c0) & 1) != ((in >> c1) & 1)) << e;
+        }
+        for (int f = 0; f < 6; ++f) {
+            const int a = f >> 1, s = f & 1, u = (a + 1) % 3, v = (a + 2) % 3, b = s << a;
+            const int q[4] = {b, b | (1 << (s ? u : v)), b | (1 << u) | (1 << v), b | (1 << (s ? v : u))};
+            int k = 0, st = -1, en = -1;
+            for (int i = 0; i < 4; ++i) {
+                const int i0 = (in >> q[i]) & 1, i1 = (in >> q[(i + 1) & 3]) & 1;
+                k += i0 != i1;
+                if (i0 && !i1) st = c_edge_of(q[i], q[(i + 1) & 3]);
+                if (!i0 && i1) en = c_edge_of(q[i], q[(i + 1) & 3]);
+            }
+            if (k == 2) next[st] = en;
+            ambiguous |= k == 4;
+        }
+        if (ambiguous) {
+            T.ntri[in] = kAmbiguous;
+            continue;
+        }
+        int n = 0;
+        unsigned todo = cross;
+        while (todo) {
+            int e0 = 0;
+            while (!((todo >> e0) & 1u)) ++e0;
+            int el[12] = {}, len = 0, e = e0;
+            do {
+                todo &= ~(1u << e);
+                el[len++] = e;
+                e = next[e];
+            } while (e != e0 && len < 12);
+            unsigned seen = 0, twice = 0;
+            for (int i = 0; i < len; ++i) {
+                const unsigned f = c_edge_faces(el[i]) & c_edge_faces(el[i + 1 < len ? i + 1 : 0]);
+                twice |= seen & f;
+                seen |= f;
+            }
+            int c = 0;
+            while (c < len && (c_edge_faces(el[c]) & twice)) ++c;
+            if (c == len) c = 0;
+            for (int i = 1; i + 1 < len; ++i, ++n) {
+                T.edge[in][3 * n] = (uint8_t)el[c];
+                T.edge[in][3 * n + 1] = (uint8_t)el[(c + i + 1) % len];
+                T.edge[in][3 * n + 2] = (uint8_t)el[(c + i) % len];
+            }
+        }
+        T.ntri[in] = (uint8_t)n;
+    }
+    return T;
+}
+
+constexpr CubeTable kCubeTable = make_cube_table();
+constexpr bool table_fits() {
+    for (int in = 0; in < 256; ++in)
+        if (kCubeTable.ntri[in] != kAmbiguous && kCubeTable.ntri[in] > kMaxTableTris) return false;
+    return true;
+}
+static_assert(table_fits(), "five triangles need a face decision");
+__device__ const CubeTable d_cube_table = kCubeTable;
+
+// Where a local vertex coordinate lies along one axis: the block below (0), this one (1), the next (2).
+__device__ __forceinline__ int block_side(int q, int B) { return q < 0 ? 0 : (q >= B ? 2 : 1); }
+
+// A block's place and surroundings, in shared memory.
+struct McBlock {
+    int slot[27];    // leaf slots of the 3^3 neighbourhood (13: the block); -1 inactive, -2 outside the grid
+    float fill[27];  // an inactive neighbour's value
+};
+
+// Vertex id of edge (p, axis), p in the block's own coordinates (-1 .. B): owner block, slot, popcount
+// below the slot.  -1 if the edge has no vertex (never for the edges of a cube's loops).
+__device__ __forceinline__ int64_t vertex_id(const McBlock& N, int B, const int* p, int a,
+                                             const uint32_t* __restrict__ bits, const int32_t* __restrict__ wpre,
+                                             const int32_t* __restrict__ voff, int W) {
+    int o[3] = {block_side(p[0], B), block_side(p[1], B), block_side(p[2], B)};
+    int s = N.slot[o[0] * 9 + o[1] * 3 + o[2]];
+    int sl;
     if (s >= 0) {
-        sl = (((px % B) * B + (py % B)) * B + (pz % B)) * 3 + a;
+        sl = (((p[0] - (o[0] - 1) * B) * B + p[1] - (o[1] - 1) * B) * B + p[2] - (o[2] - 1) * B) * 3 + a;
     } else {
-        int64_t q[3] = {px, py, pz};
-        q[a] += 1;
-        blk = ((q[0] / B) * F.nby + q[1] / B) * F.nbz + q[2] / B;
-        s = F.slot[blk];
+        o[a] = block_side(p[a] + 1, B);
+        s = N.slot[o[0] * 9 + o[1] * 3 + o[2]];
         if (s < 0) return -1;
         const int u = a == 0 ? 1 : 0, v = a == 2 ? 1 : 2;
-        sl = 3LL * B * B * B + (int64_t)a * B * B + (q[u] % B) * B + (q[v] % B);
+        sl = 3 * B * B * B + a * B * B + (p[u] - (o[u] - 1) * B) * B + p[v] - (o[v] - 1) * B;
     }
-    const uint32_t word = bits[s * W + (sl >> 5)];
+    const int64_t at = (int64_t)s * W + (sl >> 5);
+    const uint32_t word = bits[at];
     if (!((word >> (sl & 31)) & 1u)) return -1;
-    return (int64_t)voff[s] + wpre[s * W + (sl >> 5)] + __popc(word & ((1u << (sl & 31)) - 1u));
+    return (int64_t)voff[s] + wpre[at] + __popc(word & ((1u << (sl & 31)) - 1u));
 }
 
 // Block-wide exclusive scan of one int per thread (kMcThreads); returns the prefix, *total the sum.
@@ -205,225 +301,315 @@ __device__ __forceinline__ int block_scan(int v, int* s_warp, int* total) {
     }
     if (lane == 31) s_warp[warp] = inc;
     __syncthreads();
-    if (warp == 0) {
-        int w = lane < kMcThreads / 32 ? s_warp[lane] : 0;
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= o) w += y;
-        }
-        if (lane < kMcThreads / 32) s_warp[lane] = w;
+    int before = inc - v, sum = 0;
+#pragma unroll
+    for (int w = 0; w < kMcThreads / 32; ++w) {
+        if (w < warp) before += s_warp[w];
+        sum += s_warp[w];
     }
-    __syncthreads();
-    const int before = (warp ? s_warp[warp - 1] : 0) + inc - v;
-    *total = s_warp[kMcThreads / 32 - 1];
+    *total = sum;
     __syncthreads();
     return before;
 }
 
+// Triangle (f0, f1, f2) with positions q0, q1, q2: its signed volume term v0 . (v1 x v2).
+__device__ __forceinline__ double write_triangle(int64_t at, const int64_t* vid, const float (*q)[3],
+                                                 int32_t* __restrict__ faces, int32_t* __restrict__ err) {
+    if (vid[0] < 0 || vid[1] < 0 || vid[2] < 0) atomicAdd(err, 1);
+    faces[3 * at] = (int32_t)vid[0];
+    faces[3 * at + 1] = (int32_t)vid[1];
+    faces[3 * at + 2] = (int32_t)vid[2];
+    const double ax = q[0][0], ay = q[0][1], az = q[0][2], bx = q[1][0], by = q[1][1], bz = q[1][2];
+    const double cx = q[2][0], cy = q[2][1], cz = q[2][2];
+    return ax * (by * cz - bz * cy) + ay * (bz * cx - bx * cz) + az * (bx * cy - by * cx);
+}
+
 // One CTA per active block (grid-stride).  kEmit = false: edge bits, word prefixes, vertex and
-// triangle counts.  kEmit = true: vertices, triangles and the block's volume term.
-template <bool kEmit>
+// triangle counts.  kEmit = true: vertices, triangles and the block's volume term.  kB: the block edge
+// (0: any, read from the field).
+// Bound by the latency of its passes over a block, so what a block does not need is left out: most
+// active blocks lie in the margin's shell and hold no crossing (the count pass ends after the staged
+// signs, the emit pass at the counts); index arithmetic is 32-bit with the block edge a constant;
+// corner signs are bytes; loops come from a table except where a face needs its decision; and the emit
+// pass hands out triangles, not cubes, to the threads.  27 balls on 256 x 256 x 250: count 301 -> 61 us,
+// emit 414 -> 60 us.
+constexpr int kMcItems = 1024;  // triangles (or undecided cubes) handed out at a time
+static_assert(kMcItems >= kMcThreads * kMaxTableTris, "one round of cubes must fit");
+
+template <int kB, bool kEmit>
 __global__ void __launch_bounds__(kMcThreads) k_mc(McField F, const int32_t* __restrict__ active, int64_t n_active,
                                                    uint32_t* __restrict__ bits, int32_t* __restrict__ wpre,
                                                    int32_t* __restrict__ vcount, int32_t* __restrict__ tcount,
                                                    float* __restrict__ verts, int64_t* __restrict__ vkey,
                                                    int32_t* __restrict__ faces, double* __restrict__ vol_part,
                                                    int32_t* __restrict__ err, unsigned long long* __restrict__ totals) {
-    extern __shared__ float s_val[];  // (B + 2)^3 values of the block and its low/high shell
-    __shared__ int s_nslot[27];
+    extern __shared__ float s_val[];  // (B + 2)^3 values of the block and its low/high shell, then their signs
+    __shared__ McBlock s_nb;
     __shared__ int s_warp[kMcThreads / 32];
+    __shared__ int s_sum;
     __shared__ double s_vol[kMcThreads / 32];
-    const int B = F.B, R = B + 2;
-    const int64_t W = mc_words(B), S = mc_slots(B);
+    __shared__ uint2 s_item[kEmit ? kMcItems : 1];  // emit: cube | triangle << 16, offset in the block's range
+    const int B = kB ? kB : F.B, R = B + 2, R3 = R * R * R;
+    const int S = 3 * B * B * B + 3 * B * B, W = (S + 31) / 32;
+    uint8_t* s_in = reinterpret_cast<uint8_t*>(s_val + R3);  // value < level
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t nbx = (F.nx + B - 1) / B;
     for (int64_t sa = blockIdx.x; sa < n_active; sa += gridDim.x) {
+        if (kEmit && vcount[sa + 1] == vcount[sa] && tcount[sa + 1] == tcount[sa]) {
+            if (threadIdx.x == 0) vol_part[sa] = 0.0;
+            continue;
+        }
         const int64_t id = active[sa];
         const int64_t bx = id / ((int64_t)F.nby * F.nbz), by = (id / F.nbz) % F.nby, bz = id % F.nbz;
-        const int64_t x0 = bx * B, y0 = by * B, z0 = bz * B;
+        const int64_t o[3] = {bx * B, by * B, bz * B};
+        // vertices the block's region has inside the grid, along each axis: local 0 (or -1) up to top
+        const int top[3] = {(int)min((int64_t)B, F.nx - 1 - o[0]), (int)min((int64_t)B, F.ny - 1 - o[1]),
+                            (int)min((int64_t)B, F.nz - 1 - o[2])};
+        const int bot[3] = {o[0] > 0 ? -1 : 0, o[1] > 0 ? -1 : 0, o[2] > 0 ? -1 : 0};
         if (threadIdx.x < 27) {
             const int64_t nx_ = bx + threadIdx.x / 9 - 1, ny_ = by + (threadIdx.x / 3) % 3 - 1, nz_ = bz + threadIdx.x % 3 - 1;
             int v = -2;  // outside the grid
-            if (nx_ >= 0 && nx_ < nbx && ny_ >= 0 && ny_ < F.nby && nz_ >= 0 && nz_ < F.nbz)
-                v = F.slot[(nx_ * F.nby + ny_) * F.nbz + nz_];
-            s_nslot[threadIdx.x] = v;
+            float fill = 0.f;
+            if (nx_ >= 0 && nx_ < nbx && ny_ >= 0 && ny_ < F.nby && nz_ >= 0 && nz_ < F.nbz) {
+                const int64_t n = (nx_ * F.nby + ny_) * F.nbz + nz_;
+                v = F.slot[n];
+                fill = F.kind[n] < 0 ? -F.big : F.big;
+            }
+            s_nb.slot[threadIdx.x] = v;
+            s_nb.fill[threadIdx.x] = fill;
         }
-        for (int r = threadIdx.x; r < R * R * R; r += kMcThreads) {
-            const int64_t x = x0 - 1 + r / (R * R), y = y0 - 1 + (r / R) % R, z = z0 - 1 + r % R;
-            float v = 0.f;
-            if (x >= 0 && x < F.nx && y >= 0 && y < F.ny && z >= 0 && z < F.nz) v = voxel_value(F, x, y, z);
-            s_val[r] = v;
-        }
+        if (threadIdx.x == 0) s_sum = 0;
         __syncthreads();
-        auto val = [&](int64_t x, int64_t y, int64_t z) -> double {  // value - level, from the region
-            return __dsub_rn((double)s_val[((x - x0 + 1) * R + (y - y0 + 1)) * R + (z - z0 + 1)], F.level);
-        };
-        // ---- edges ----
-        int run = 0;  // vertices before this chunk (emit) / count (count pass)
-        for (int64_t c0 = 0; c0 < S; c0 += kMcThreads) {
-            const int64_t sl = c0 + threadIdx.x;
-            bool hit = false;
-            int64_t p[3] = {0, 0, 0};
-            int a = 0;
-            if (sl < S) {
-                if (sl < 3LL * B * B * B) {
-                    a = (int)(sl % 3);
-                    const int64_t lin = sl / 3;
-                    p[0] = x0 + lin / (B * B);
-                    p[1] = y0 + (lin / B) % B;
-                    p[2] = z0 + lin % B;
+        int seen = 0;  // bit 0: a value inside, bit 1: one outside
+        for (int r = threadIdx.x; r < R3; r += kMcThreads) {
+            const int p[3] = {r / (R * R) - 1, (r / R) % R - 1, r % R - 1};
+            float v = 0.f;
+            bool in = false;
+            if (p[0] >= bot[0] && p[0] <= top[0] && p[1] >= bot[1] && p[1] <= top[1] && p[2] >= bot[2] && p[2] <= top[2]) {
+                const int s0 = block_side(p[0], B), s1 = block_side(p[1], B), s2 = block_side(p[2], B);
+                const int nb = s0 * 9 + s1 * 3 + s2, s = s_nb.slot[nb];
+                v = s < 0 ? s_nb.fill[nb]
+                          : F.tiles[(int64_t)s * (B * B * B) + ((p[0] - (s0 - 1) * B) * B + p[1] - (s1 - 1) * B) * B +
+                                    p[2] - (s2 - 1) * B];
+                in = __dsub_rn((double)v, F.level) < 0.0;
+                seen |= in ? 1 : 2;
+            }
+            s_val[r] = v;
+            s_in[r] = in;
+        }
+        const bool crossed = __syncthreads_or(seen & 1) && __syncthreads_or(seen & 2);
+        if (!kEmit && !crossed) {
+            if (threadIdx.x == 0) {
+                vcount[sa] = 0;
+                tcount[sa] = 0;
+            }
+            __syncthreads();
+            continue;
+        }
+        auto at = [&](const int* p) { return ((p[0] + 1) * R + p[1] + 1) * R + p[2] + 1; };
+        auto val = [&](int r) { return __dsub_rn((double)s_val[r], F.level); };
+        const int step[3] = {R * R, R, 1};
+        // ---- edges: a warp per bit word ----
+        int verts_here = 0;
+        for (int w = warp; w < W; w += kMcThreads / 32) {
+            const int sl = w * 32 + lane;
+            uint32_t word = 0;
+            if (kEmit) {
+                word = bits[sa * W + w];
+                if (!word) continue;
+            }
+            bool hit = kEmit && ((word >> lane) & 1u);
+            int p[3] = {0, 0, 0}, a = 0;
+            if (kEmit ? hit : sl < S) {
+                if (sl < 3 * B * B * B) {
+                    a = sl % 3;
+                    const int lin = sl / 3;
+                    p[0] = lin / (B * B);
+                    p[1] = (lin / B) % B;
+                    p[2] = lin % B;
                 } else {
-                    const int64_t r = sl - 3LL * B * B * B;
-                    a = (int)(r / (B * B));
+                    const int r = sl - 3 * B * B * B;
+                    a = r / (B * B);
                     const int u = a == 0 ? 1 : 0, v = a == 2 ? 1 : 2;
-                    p[0] = x0;
-                    p[1] = y0;
-                    p[2] = z0;
-                    p[u] += (r % (B * B)) / B;
-                    p[v] += r % B;
-                    p[a] -= 1;
+                    p[u] = (r % (B * B)) / B;
+                    p[v] = r % B;
+                    p[a] = -1;
                 }
-                const int64_t n[3] = {F.nx, F.ny, F.nz};
-                bool ok = p[0] >= 0 && p[1] >= 0 && p[2] >= 0 && p[0] < n[0] && p[1] < n[1] && p[2] < n[2] &&
-                          p[a] + 1 < n[a];
-                if (ok && sl >= 3LL * B * B * B) {  // entering edge: ours only when its lower block is inactive
-                    const int nb = a == 0 ? 4 : (a == 1 ? 10 : 12);  // the (-1) neighbour along a
-                    ok = s_nslot[nb] < 0;
-                }
-                if (ok) {
-                    int64_t q[3] = {p[0], p[1], p[2]};
-                    q[a] += 1;
-                    const double g0 = val(p[0], p[1], p[2]), g1 = val(q[0], q[1], q[2]);
-                    hit = (g0 < 0.0) != (g1 < 0.0);
-                    if (kEmit && hit) {
-                        // vertex id: this block's offset + words before + bits below, from the count pass
-                        const uint32_t word = bits[sa * W + (sl >> 5)];
-                        const int64_t vid = (int64_t)vcount[sa] + wpre[sa * W + (sl >> 5)] +
-                                            __popc(word & ((1u << (sl & 31)) - 1u));
-                        edge_vertex(F, p[0], p[1], p[2], a, g0, g1, verts + 3 * vid);
-                        if (vkey) vkey[vid] = ((p[0] * F.ny + p[1]) * F.nz + p[2]) * 3 + a;
-                    }
+                const int r = at(p);
+                if (kEmit) {
+                    const int64_t vid = (int64_t)vcount[sa] + wpre[sa * W + w] + __popc(word & ((1u << lane) - 1u));
+                    const int64_t g[3] = {o[0] + p[0], o[1] + p[1], o[2] + p[2]};
+                    edge_vertex(F, g[0], g[1], g[2], a, val(r), val(r + step[a]), verts + 3 * vid);
+                    if (vkey) vkey[vid] = ((g[0] * F.ny + g[1]) * F.nz + g[2]) * 3 + a;
+                } else {
+                    bool ok = p[0] <= top[0] && p[1] <= top[1] && p[2] <= top[2] && p[a] >= bot[a] && p[a] + 1 <= top[a];
+                    // an entering edge is ours only when its lower block is inactive
+                    if (sl >= 3 * B * B * B) ok = ok && s_nb.slot[a == 0 ? 4 : (a == 1 ? 10 : 12)] < 0;
+                    hit = ok && s_in[r] != s_in[r + step[a]];
                 }
             }
-            const unsigned ball = __ballot_sync(0xffffffffu, hit);
             if (!kEmit) {
-                // word prefixes inside the block: a running count over the chunk's words
-                const int wc = (threadIdx.x & 31) == 0 ? __popc(ball) : 0;
-                int chunk_total;
-                const int before = block_scan(wc, s_warp, &chunk_total);
-                if ((threadIdx.x & 31) == 0 && sl < S) {
-                    bits[sa * W + (sl >> 5)] = ball;
-                    wpre[sa * W + (sl >> 5)] = run + before;
+                const unsigned ball = __ballot_sync(0xffffffffu, hit);
+                if (lane == 0) {
+                    bits[sa * W + w] = ball;
+                    wpre[sa * W + w] = __popc(ball);  // its prefix below
                 }
-                run += chunk_total;
             }
         }
-        if (!kEmit && threadIdx.x == 0) {
-            vcount[sa] = run;
-            atomicAdd(&totals[0], (unsigned long long)run);
+        if (!kEmit) {
+            __syncthreads();
+            if (warp == 0) {  // exclusive prefixes of the words' counts
+                for (int w0 = 0; w0 < W; w0 += 32) {
+                    const int c = w0 + lane < W ? wpre[sa * W + w0 + lane] : 0;
+                    int inc = c;
+                    for (int d = 1; d < 32; d <<= 1) {
+                        const int y = __shfl_up_sync(0xffffffffu, inc, d);
+                        if (lane >= d) inc += y;
+                    }
+                    if (w0 + lane < W) wpre[sa * W + w0 + lane] = verts_here + inc - c;
+                    verts_here += __shfl_sync(0xffffffffu, inc, 31);
+                }
+                if (lane == 0) {
+                    vcount[sa] = verts_here;
+                    if (verts_here) atomicAdd(&totals[0], (unsigned long long)verts_here);
+                }
+            }
         }
-        // ---- cubes: lowest corners x0 - 1 .. x0 + B - 1 per axis, lexicographic ----
-        const int C = B + 1;
-        const int64_t ncube = (int64_t)C * C * C;
-        int tri_run = 0;
+        // ---- cubes: lowest corners -1 .. B - 1 per axis, lexicographic ----
+        const int C = B + 1, ncube = C * C * C;
+        int run = 0, items = 0, tri_sum = 0;
         double vol = 0.0;
-        for (int64_t c0 = 0; c0 < ncube; c0 += kMcThreads) {
-            const int64_t ci = c0 + threadIdx.x;
-            int ntri = 0;
-            CubeLoops L;
-            L.cross = 0;
-            int64_t m[3] = {0, 0, 0};
-            if (ci < ncube) {
-                m[0] = x0 - 1 + ci / (C * C);
-                m[1] = y0 - 1 + (ci / C) % C;
-                m[2] = z0 - 1 + ci % C;
-                bool ok = m[0] >= 0 && m[1] >= 0 && m[2] >= 0 && m[0] + 1 < F.nx && m[1] + 1 < F.ny && m[2] + 1 < F.nz;
-                if (ok && (m[0] < x0 || m[1] < y0 || m[2] < z0)) {
-                    // a cube reaching into the low shell: ours if its first corner in an active block is here
-                    int first = -1;
-                    for (int c = 0; c < 8 && first < 0; ++c) {
-                        const int o0 = m[0] + (c & 1) < x0 ? 0 : (m[0] + (c & 1) >= x0 + B ? 2 : 1);
-                        const int o1 = m[1] + ((c >> 1) & 1) < y0 ? 0 : (m[1] + ((c >> 1) & 1) >= y0 + B ? 2 : 1);
-                        const int o2 = m[2] + ((c >> 2) & 1) < z0 ? 0 : (m[2] + ((c >> 2) & 1) >= z0 + B ? 2 : 1);
-                        const int nb = o0 * 9 + o1 * 3 + o2;
-                        if (s_nslot[nb] >= 0) first = nb;
-                    }
-                    ok = first == 13;
+        auto corners = [&](int r, double* g) {
+#pragma unroll
+            for (int c = 0; c < 8; ++c) g[c] = val(r + ((c & 1) ? R * R : 0) + ((c & 2) ? R : 0) + ((c & 4) ? 1 : 0));
+        };
+        auto edge_point = [&](const int* m, int e, int64_t& vid, float* q) {
+            const int c0 = edge_corner0(e), a = e >> 2;
+            const int p[3] = {m[0] + (c0 & 1), m[1] + ((c0 >> 1) & 1), m[2] + ((c0 >> 2) & 1)};
+            vid = vertex_id(s_nb, B, p, a, bits, wpre, vcount, W);
+            const int r = at(p);
+            edge_vertex(F, o[0] + p[0], o[1] + p[1], o[2] + p[2], a, val(r), val(r + step[a]), q);
+        };
+        auto flush = [&]() {  // the threads take the handed-out items
+            __syncthreads();
+            const int64_t base = tcount[sa];
+            for (int i = threadIdx.x; i < items; i += kMcThreads) {
+                const uint2 it = s_item[i];
+                const int ci = it.x & 0xffff, t = it.x >> 16;
+                const int m[3] = {ci / (C * C) - 1, (ci / C) % C - 1, ci % C - 1};
+                const int r = at(m);
+                if (t < kMaxTableTris) {
+                    int in = 0;
+#pragma unroll
+                    for (int c = 0; c < 8; ++c)
+                        in |= s_in[r + ((c & 1) ? R * R : 0) + ((c & 2) ? R : 0) + ((c & 4) ? 1 : 0)] << c;
+                    int64_t vid[3];
+                    float q[3][3];
+                    for (int k = 0; k < 3; ++k) edge_point(m, d_cube_table.edge[in][3 * t + k], vid[k], q[k]);
+                    vol += write_triangle(base + it.y, vid, q, faces, err);
+                    continue;
                 }
-                if (ok) {
-                    double g[8];
-                    for (int c = 0; c < 8; ++c) g[c] = val(m[0] + (c & 1), m[1] + ((c >> 1) & 1), m[2] + ((c >> 2) & 1));
-                    L = cube_loops(g);
-                    ntri = cube_triangles(L);
-                }
-            }
-            if (!kEmit) {
-                tri_run += ntri;
-                continue;
-            }
-            int chunk_total;
-            const int before = block_scan(ntri, s_warp, &chunk_total);
-            if (ntri) {
-                int64_t at = (int64_t)tcount[sa] + tri_run + before;
+                double g[8];
+                corners(r, g);
+                const CubeLoops L = cube_loops(g);
+                int64_t to = base + it.y;
                 unsigned todo = L.cross;
                 while (todo) {
                     const int e0 = __ffs(todo) - 1;
-                    int64_t vid[12];
-                    float pos[12][3];
                     int el[12];
                     int len = 0, e = e0;
                     do {  // a permutation cycle of at most 12 edges (cube_triangles counted it)
                         todo &= ~(1u << e);
-                        el[len] = e;
-                        const int cc = edge_corner0(e);
-                        const int64_t px = m[0] + (cc & 1), py = m[1] + ((cc >> 1) & 1), pz = m[2] + ((cc >> 2) & 1);
-                        const int ax = e >> 2;
-                        vid[len] = vertex_id(F, px, py, pz, ax, bits, wpre, vcount, W);
-                        int64_t q[3] = {px, py, pz};
-                        q[ax] += 1;
-                        edge_vertex(F, px, py, pz, ax, val(px, py, pz), val(q[0], q[1], q[2]), pos[len]);
-                        ++len;
+                        el[len++] = e;
                         e = loop_next(L, e);
                     } while (e >= 0 && e != e0 && len < 12);
                     // fan centre: the first vertex on no face that the loop crosses twice (a fan
                     // from such a face would lay a flat triangle into it), else the lowest edge
-                    unsigned seen = 0, twice = 0;
-                    for (int i = 0; i < len; ++i) {
-                        const unsigned f = edge_faces(el[i]) & edge_faces(el[i + 1 < len ? i + 1 : 0]);
-                        twice |= seen & f;
-                        seen |= f;
+                    unsigned faces_seen = 0, twice = 0;
+                    for (int i2 = 0; i2 < len; ++i2) {
+                        const unsigned f = edge_faces(el[i2]) & edge_faces(el[i2 + 1 < len ? i2 + 1 : 0]);
+                        twice |= faces_seen & f;
+                        faces_seen |= f;
                     }
                     int c = 0;
                     while (c < len && (edge_faces(el[c]) & twice)) ++c;
                     if (c == len) c = 0;
-                    for (int i = 1; i + 1 < len; ++i) {
-                        const int j0 = c, j1 = (c + i + 1) % len, j2 = (c + i) % len;
-                        const int64_t t3 = 3 * (at++);
-                        if (vid[j0] < 0 || vid[j1] < 0 || vid[j2] < 0) atomicAdd(err, 1);
-                        faces[t3] = (int32_t)vid[j0];
-                        faces[t3 + 1] = (int32_t)vid[j1];
-                        faces[t3 + 2] = (int32_t)vid[j2];
-                        // signed volume term v0 . (v1 x v2) of the triangle as written
-                        const double ax_ = pos[j0][0], ay = pos[j0][1], az = pos[j0][2];
-                        const double bx_ = pos[j1][0], by_ = pos[j1][1], bz_ = pos[j1][2];
-                        const double cx = pos[j2][0], cy = pos[j2][1], cz = pos[j2][2];
-                        vol += ax_ * (by_ * cz - bz_ * cy) + ay * (bz_ * cx - bx_ * cz) + az * (bx_ * cy - by_ * cx);
+                    for (int i2 = 1; i2 + 1 < len; ++i2) {
+                        int64_t vid[3];
+                        float q[3][3];
+                        edge_point(m, el[c], vid[0], q[0]);
+                        edge_point(m, el[(c + i2 + 1) % len], vid[1], q[1]);
+                        edge_point(m, el[(c + i2) % len], vid[2], q[2]);
+                        vol += write_triangle(to++, vid, q, faces, err);
                     }
                 }
             }
-            tri_run += chunk_total;
+            __syncthreads();
+            items = 0;
+        };
+        for (int c0 = 0; c0 < ncube; c0 += kMcThreads) {
+            const int ci = c0 + threadIdx.x;
+            int ntri = 0, n_items = 0;
+            if (ci < ncube) {
+                const int m[3] = {ci / (C * C) - 1, (ci / C) % C - 1, ci % C - 1};
+                bool ok = true;
+#pragma unroll
+                for (int a = 0; a < 3; ++a) ok &= m[a] >= bot[a] && m[a] + 1 <= top[a];
+                int in = 0;
+                const int r = at(m);
+                if (ok) {
+#pragma unroll
+                    for (int c = 0; c < 8; ++c)
+                        in |= s_in[r + ((c & 1) ? R * R : 0) + ((c & 2) ? R : 0) + ((c & 4) ? 1 : 0)] << c;
+                    ok = in != 0 && in != 255;
+                }
+                if (ok && (m[0] < 0 || m[1] < 0 || m[2] < 0)) {
+                    // a cube reaching into the low shell: ours if its first corner in an active block is here
+                    int first = -1;
+                    for (int c = 0; c < 8 && first < 0; ++c) {
+                        const int nb = block_side(m[0] + (c & 1), B) * 9 + block_side(m[1] + ((c >> 1) & 1), B) * 3 +
+                                       block_side(m[2] + ((c >> 2) & 1), B);
+                        if (s_nb.slot[nb] >= 0) first = nb;
+                    }
+                    ok = first == 13;
+                }
+                if (ok) {
+                    ntri = n_items = d_cube_table.ntri[in];
+                    if (ntri == kAmbiguous) {
+                        double g[8];
+                        corners(r, g);
+                        ntri = cube_triangles(cube_loops(g));
+                        n_items = ntri ? kMaxTableTris + 1 : 0;  // marks one item for the whole cube
+                    }
+                }
+            }
+            if (!kEmit) {
+                tri_sum += ntri;
+                continue;
+            }
+            const int put = n_items > kMaxTableTris ? 1 : n_items;
+            int total;
+            const int before = block_scan(put << 16 | ntri, s_warp, &total);  // at most 1024 items, 3072 triangles
+            if (items + (total >> 16) > kMcItems) flush();
+            for (int t = 0; t < put; ++t)
+                s_item[items + (before >> 16) + t] =
+                    make_uint2((uint32_t)ci | (uint32_t)(n_items > kMaxTableTris ? kMaxTableTris : t) << 16,
+                               (uint32_t)(run + (before & 0xffff) + t));
+            items += total >> 16;
+            run += total & 0xffff;
         }
         if (!kEmit) {
-            // block triangle count: a reduction over the threads' sums
-            int dummy;
-            const int before = block_scan(tri_run, s_warp, &dummy);
-            (void)before;
+            for (int d = 16; d > 0; d >>= 1) tri_sum += __shfl_xor_sync(0xffffffffu, tri_sum, d);
+            if (lane == 0 && tri_sum) atomicAdd(&s_sum, tri_sum);
+            __syncthreads();
             if (threadIdx.x == 0) {
-                tcount[sa] = dummy;
-                atomicAdd(&totals[1], (unsigned long long)dummy);
+                tcount[sa] = s_sum;
+                if (s_sum) atomicAdd(&totals[1], (unsigned long long)s_sum);
             }
         } else {
-            for (int o = 16; o > 0; o >>= 1) vol += __shfl_xor_sync(0xffffffffu, vol, o);
-            if ((threadIdx.x & 31) == 0) s_vol[threadIdx.x >> 5] = vol;
+            flush();
+            for (int d = 16; d > 0; d >>= 1) vol += __shfl_xor_sync(0xffffffffu, vol, d);
+            if (lane == 0) s_vol[warp] = vol;
             __syncthreads();
             if (threadIdx.x == 0) {
                 double t = 0.0;
@@ -464,20 +650,35 @@ int mc_field(McField& F, const int32_t* d_kind, const float* d_tiles, int64_t nx
     return FB_OK;
 }
 
-size_t mc_smem(int B) { return (size_t)(B + 2) * (B + 2) * (B + 2) * sizeof(float); }
+size_t mc_smem(int B) { return (size_t)(B + 2) * (B + 2) * (B + 2) * (sizeof(float) + 1); }
+
+template <int kB, bool kEmit>
+int mc_launch_block(const McField& F, const int32_t* d_active, int64_t n_active, uint32_t* bits, int32_t* wpre,
+              int32_t* vcount, int32_t* tcount, float* verts, int64_t* vkey, int32_t* faces, double* vol_part,
+              int32_t* err, unsigned long long* totals, cudaStream_t st) {
+    if (n_active == 0) return FB_OK;
+    const size_t smem = mc_smem(F.B);
+    if (smem > 48 * 1024) FB_CUDA(cudaFuncSetAttribute(k_mc<kB, kEmit>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int grid = (int)std::min<int64_t>(n_active, (int64_t)fb_sm_count() * 8);
+    k_mc<kB, kEmit><<<grid, kMcThreads, smem, st>>>(F, d_active, n_active, bits, wpre, vcount, tcount, verts, vkey,
+                                                   faces, vol_part, err, totals);
+    FB_LAUNCH();
+    return FB_OK;
+}
 
 template <bool kEmit>
 int mc_launch(const McField& F, const int32_t* d_active, int64_t n_active, uint32_t* bits, int32_t* wpre,
               int32_t* vcount, int32_t* tcount, float* verts, int64_t* vkey, int32_t* faces, double* vol_part,
               int32_t* err, unsigned long long* totals, cudaStream_t st) {
-    if (n_active == 0) return FB_OK;
-    const size_t smem = mc_smem(F.B);
-    if (smem > 48 * 1024) FB_CUDA(cudaFuncSetAttribute(k_mc<kEmit>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int grid = (int)std::min<int64_t>(n_active, (int64_t)fb_sm_count() * 8);
-    k_mc<kEmit><<<grid, kMcThreads, smem, st>>>(F, d_active, n_active, bits, wpre, vcount, tcount, verts, vkey,
-                                               faces, vol_part, err, totals);
-    FB_LAUNCH();
-    return FB_OK;
+#define FB_MC(BB) mc_launch_block<BB, kEmit>(F, d_active, n_active, bits, wpre, vcount, tcount, verts, vkey, faces, \
+                                             vol_part, err, totals, st)
+    switch (F.B) {
+    case 4: return FB_MC(4);
+    case 8: return FB_MC(8);
+    case 16: return FB_MC(16);
+    default: return FB_MC(0);
+    }
+#undef FB_MC
 }
 
 // ---- connected components of the exported mesh (faltvolym_v1.py:95-101 keeps the largest) ----
