@@ -45,10 +45,31 @@ __device__ __forceinline__ int effective_op(uint32_t entry, int op) {
     return mode == 1u ? CH_SET : (mode == 2u ? CH_SETNEG : op);
 }
 
+// primf_world with the rarely used kinds out of line: the culling walks have several copies of it, and
+// with every kind inlined in each they missed the instruction cache.
+static __device__ __noinline__ float canon_out_of_line(const PrimF& P, float x, float y, float z) {
+    return canon_f(P.type, P.p, x, y, z);
+}
+
+__device__ __forceinline__ float primf_world_common(const PrimF& P, float x, float y, float z) {
+    const float lx = fmaf(P.A[0], x, fmaf(P.A[1], y, fmaf(P.A[2], z, P.A[3])));
+    const float ly = fmaf(P.A[4], x, fmaf(P.A[5], y, fmaf(P.A[6], z, P.A[7])));
+    const float lz = fmaf(P.A[8], x, fmaf(P.A[9], y, fmaf(P.A[10], z, P.A[11])));
+    float c;
+    switch (P.type) {
+    case P_SPHERE: c = canon_f(P_SPHERE, P.p, lx, ly, lz); break;
+    case P_BOX: c = canon_f(P_BOX, P.p, lx, ly, lz); break;
+    case P_CAPSULE: c = canon_f(P_CAPSULE, P.p, lx, ly, lz); break;
+    case P_TORUS: c = canon_f(P_TORUS, P.p, lx, ly, lz); break;
+    default: c = canon_out_of_line(P, lx, ly, lz);
+    }
+    return fmaf(P.s, c, -P.off);
+}
+
 // Interval of one chain element's primitive around (cx, cy, cz) with radius R.
 __device__ __forceinline__ void element_interval(const PrimF& P, float cx, float cy, float cz, float R, float eps,
                                                  float& lo, float& hi) {
-    const float v = primf_world(P, cx, cy, cz);
+    const float v = primf_world_common(P, cx, cy, cz);
     const float r = fmaf(P.lip, R, eps + 1e-6f * fabsf(v));
     lo = v - r;
     hi = v + r;
@@ -67,21 +88,28 @@ struct Elem {
     float lo, hi;  // bounds of the value the combine sees (-p for a subtraction)
 };
 
-// The same enclosure from the primitive's bounding ball (PrimF.ball == 1): no evaluation of the
-// primitive, a few loads -- looser by up to the ball's diameter.
-__device__ __forceinline__ void element_interval_ball(const PrimF& P, float cx, float cy, float cz, float R, float eps,
+// A primitive's bounding ball by itself (PrimF.ball, ball_k, off, p[8..11]): what the coarse level reads
+// of every element.  32 consecutive bytes: gathered from the 128-byte records, 32 lanes' loads took 32
+// cache lines each and the records of 4096 elements did not stay in L1.
+struct __align__(16) Ball {
+    float x, y, z, r;
+    float k, off, has, pad;  // value scale and offset; has != 0: the ball holds
+};
+
+// The enclosure from the bounding ball: no evaluation of the primitive, a few loads -- looser by up to
+// the ball's diameter.
+__device__ __forceinline__ void element_interval_ball(const Ball& P, float cx, float cy, float cz, float R, float eps,
                                                       float& lo, float& hi) {
-    const float dx = cx - P.p[8], dy = cy - P.p[9], dz = cz - P.p[10];
+    const float dx = cx - P.x, dy = cy - P.y, dz = cz - P.z;
     const float d = sqrt_rn(fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
-    const float k = P.ball_k, rw = P.p[11];
-    const float m = eps + 1e-6f * (k * (d + R + rw) + fabsf(P.off));
-    lo = fmaf(k, d - R - rw, -P.off) - m;
-    hi = fmaf(k, d + R + rw, -P.off) + m;
+    const float m = eps + 1e-6f * (P.k * (d + R + P.r) + fabsf(P.off));
+    lo = fmaf(P.k, d - R - P.r, -P.off) - m;
+    hi = fmaf(P.k, d + R + P.r, -P.off) + m;
 }
 
 __device__ __forceinline__ Elem load_elem(const uint32_t* __restrict__ in, int e, const FbInsn* __restrict__ chain,
                                           const PrimF* __restrict__ primf, float cx, float cy, float cz, float R,
-                                          float eps, bool with_bounds, bool ball = false) {
+                                          float eps, bool with_bounds, const Ball* __restrict__ balls = nullptr) {
     Elem E;
     E.ent = in ? in[e] : (uint32_t)e << 2;  // a null list is the whole chain in order
     const FbInsn I = chain[E.ent >> 2];
@@ -90,9 +118,11 @@ __device__ __forceinline__ Elem load_elem(const uint32_t* __restrict__ in, int e
     E.lo = E.hi = 0.f;
     if (with_bounds && E.op != CH_OFFSET) {
         float lo, hi;
-        const PrimF& P = primf[I.arg];
-        if (ball && P.ball != 0.f) element_interval_ball(P, cx, cy, cz, R, eps, lo, hi);
-        else element_interval(P, cx, cy, cz, R, eps, lo, hi);
+        Ball b;
+        b.has = 0.f;
+        if (balls) b = balls[I.arg];
+        if (b.has != 0.f) element_interval_ball(b, cx, cy, cz, R, eps, lo, hi);
+        else element_interval(primf[I.arg], cx, cy, cz, R, eps, lo, hi);
         if (E.op == CH_SUBTRACT || E.op == CH_SETNEG) { E.lo = -hi; E.hi = -lo; }
         else { E.lo = lo; E.hi = hi; }
     }
@@ -125,13 +155,32 @@ __device__ __forceinline__ bool run_keep(int op, const Elem& E, float bound) {
     return op == CH_UNION ? !(E.lo > bound) : !(E.hi < bound);
 }
 
+// One element that is no part of a run: interval_step on its primitive's own bounds.
+__device__ __forceinline__ int single_step(const Elem& E, float& alo, float& ahi) {
+    const bool neg = E.op == CH_SUBTRACT || E.op == CH_SETNEG;
+    return interval_step(E.op, E.k, neg ? -E.hi : E.lo, neg ? -E.lo : E.hi, alo, ahi);
+}
+
+// The accumulator's bounds after a run whose kept elements have bounds [klo, khi] (a warp's lanes each
+// hold their part).
+__device__ __forceinline__ void end_run(int op, const RunState& rs, float klo, float khi, float& alo, float& ahi) {
+    for (int o = 16; o > 0; o >>= 1) {
+        klo = fminf(klo, __shfl_xor_sync(0xffffffffu, klo, o));
+        khi = fmaxf(khi, __shfl_xor_sync(0xffffffffu, khi, o));
+    }
+    if (op == CH_UNION) {
+        alo = rs.reset ? klo : fminf(alo, klo);
+        ahi = rs.bound;
+    } else {
+        alo = rs.bound;
+        ahi = rs.reset ? khi : fmaxf(ahi, khi);
+    }
+}
+
 // Warp-cooperative chain walk over `in` for the region centred at (cx, cy, cz) with radius R.
 // Hard runs are decided with two warp-parallel passes (aggregate bound, then keep/drop with
 // ballot compaction); other elements (offsets, smooth booleans, sets) step one at a time.
 // Returns the kept count (may exceed cap: then the output is incomplete and must not be used).
-// kBall: bound primitives by their bounding balls where they have one (the coarse level, where
-// every region walks the whole chain).
-template <bool kBall = false>
 __device__ int warp_walk(const uint32_t* __restrict__ in, int n_in, const FbInsn* __restrict__ chain,
                          const PrimF* __restrict__ primf, float cx, float cy, float cz, float R, float eps,
                          uint32_t* __restrict__ out, int cap) {
@@ -144,9 +193,7 @@ __device__ int warp_walk(const uint32_t* __restrict__ in, int n_in, const FbInsn
         const Elem head = load_elem(in, i, chain, primf, cx, cy, cz, R, eps, false);
         if (!runnable(head.op, head.k)) {
             const Elem E = load_elem(in, i, chain, primf, cx, cy, cz, R, eps, true);
-            float plo = E.lo, phi = E.hi;  // back to the primitive's own bounds
-            if (E.op == CH_SUBTRACT || E.op == CH_SETNEG) { plo = -E.hi; phi = -E.lo; }
-            const int act = interval_step(E.op, E.k, plo, phi, alo, ahi);
+            const int act = single_step(E, alo, ahi);
             if (act) {
                 uint32_t rec = E.ent;
                 if (act == 2) { n = 0; rec = (E.ent & ~3u) | 1u; }
@@ -159,37 +206,20 @@ __device__ int warp_walk(const uint32_t* __restrict__ in, int n_in, const FbInsn
         }
         const int op = head.op;
         // pass 1, 32 elements at a time: the run's end (the first element of another kind) and the
-        // aggregate bound of the elements before it.  With ball bounds the same pass also writes the
-        // candidates: elements not beaten by the bound so far (the minimum over everything up to and
-        // including their chunk) -- a superset of those the final bound keeps.
+        // aggregate bound of the elements before it
         float agg = op == CH_UNION ? 3.0e38f : -3.0e38f;
         int j = n_in;
-        const int n0 = n;
         for (int b = i; b < n_in; b += 32) {
             const int e = b + lane;
             bool same = false;
             Elem E;
             if (e < n_in) {
-                E = load_elem(in, e, chain, primf, cx, cy, cz, R, eps, true, kBall);
+                E = load_elem(in, e, chain, primf, cx, cy, cz, R, eps, true);
                 same = e == i || (E.op == op && runnable(E.op, E.k));
             }
             const unsigned stop = __ballot_sync(0xffffffffu, e < n_in && !same);
             const int end = stop ? b + __ffs(stop) - 1 : min(b + 32, n_in);
             if (e < end) agg = op == CH_UNION ? fminf(agg, E.hi) : fmaxf(agg, E.lo);
-            if (kBall) {
-                float run = agg;
-                for (int o = 16; o > 0; o >>= 1) {
-                    const float t = __shfl_xor_sync(0xffffffffu, run, o);
-                    run = op == CH_UNION ? fminf(run, t) : fmaxf(run, t);
-                }
-                const bool keep = e < end && run_keep(op, E, run);
-                const unsigned kept = __ballot_sync(0xffffffffu, keep);
-                if (keep) {
-                    const int pos = n + __popc(kept & below);
-                    if (pos < cap) out[pos] = E.ent;
-                }
-                n += __popc(kept);
-            }
             if (stop) {
                 j = end;
                 break;
@@ -199,84 +229,169 @@ __device__ int warp_walk(const uint32_t* __restrict__ in, int n_in, const FbInsn
             const float t = __shfl_xor_sync(0xffffffffu, agg, o);
             agg = op == CH_UNION ? fminf(agg, t) : fmaxf(agg, t);
         }
-        RunState rs = run_decide(op, agg, alo, ahi);
+        const RunState rs = run_decide(op, agg, alo, ahi);
         float klo = 3.0e38f, khi = -3.0e38f;
-        if (kBall) {
-            // pass 1 wrote the candidates (every other element of the run provably loses, so the run's
-            // result is the candidates' result); the exact bounds of the candidates alone give the
-            // run's decision, and the candidates are compacted in place with it
-            const int nc = n - n0;  // candidates at out[n0, n)
-            if (n > cap) {          // overflowed: the region falls back to its parent's list anyway
-                i = j;
-                continue;
+        if (rs.reset) n = 0;
+        bool first = rs.reset;
+        // pass 2: keep / drop, ballot compaction in chain order
+        for (int b = i; b < j; b += 32) {
+            const int e = b + lane;
+            bool keep = false;
+            Elem E;
+            if (e < j) {
+                E = load_elem(in, e, chain, primf, cx, cy, cz, R, eps, true);
+                keep = run_keep(op, E, rs.bound);
+                if (keep) { klo = fminf(klo, E.lo); khi = fmaxf(khi, E.hi); }
             }
-            float agg2 = op == CH_UNION ? 3.0e38f : -3.0e38f;
-            for (int b = 0; b < nc; b += 32) {
-                if (b + lane < nc) {
-                    const Elem E = load_elem(out + n0, b + lane, chain, primf, cx, cy, cz, R, eps, true);
-                    agg2 = op == CH_UNION ? fminf(agg2, E.hi) : fmaxf(agg2, E.lo);
+            const unsigned kept = __ballot_sync(0xffffffffu, keep);
+            if (keep) {
+                const int pos = n + __popc(kept & below);
+                uint32_t rec = E.ent;
+                if (first && pos == 0) rec = (E.ent & ~3u) | (op == CH_SUBTRACT ? 2u : 1u);
+                if (pos < cap) out[pos] = rec;
+            }
+            if (kept) first = false;
+            n += __popc(kept);
+        }
+        end_run(op, rs, klo, khi, alo, ahi);
+        i = j;
+    }
+    return n;
+}
+
+// The same walk of the whole chain (the coarse level, where every region walks it), bounding
+// primitives by their bounding balls where they have one.  Pass 1 of a run also writes its candidates:
+// elements not beaten by the bound so far, a superset of those the final bound keeps (every other
+// element provably loses, so the run's result is the candidates' result); the exact bounds of the
+// candidates alone give the run's decision, and they are compacted in place with it.  Few warps walk
+// here (a region each), so a warp keeps the loads of kBallChunks chunks in flight.  4096 regions of 4096
+// elements: 541 -> XX us with the balls in a table of their own.
+constexpr int kBallChunks = 4;
+
+__device__ int warp_walk_ball(int n_in, const FbInsn* __restrict__ chain, const PrimF* __restrict__ primf,
+                              const Ball* __restrict__ balls, float cx, float cy, float cz, float R, float eps,
+                              uint32_t* __restrict__ out, int cap, float* klo_of, float* khi_of, int n_of) {
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    float alo = 0.f, ahi = 0.f;
+    int n = 0;
+    int i = 0;
+    while (i < n_in) {
+        const Elem head = load_elem(nullptr, i, chain, primf, cx, cy, cz, R, eps, false);
+        if (!runnable(head.op, head.k)) {
+            const Elem E = load_elem(nullptr, i, chain, primf, cx, cy, cz, R, eps, true);
+            const int act = single_step(E, alo, ahi);
+            if (act) {
+                uint32_t rec = E.ent;
+                if (act == 2) { n = 0; rec = (E.ent & ~3u) | 1u; }
+                if (act == 3) { n = 0; rec = (E.ent & ~3u) | 2u; }
+                if (n < cap && lane == 0) out[n] = rec;
+                ++n;
+            }
+            ++i;
+            continue;
+        }
+        const int op = head.op;
+        float agg = op == CH_UNION ? 3.0e38f : -3.0e38f;
+        int j = n_in;
+        const int n0 = n;
+        for (int b = i; b < n_in; b += 32 * kBallChunks) {
+            Elem E[kBallChunks];
+#pragma unroll
+            for (int c = 0; c < kBallChunks; ++c) {
+                const int e = b + 32 * c + lane;
+                E[c].op = -1;
+                E[c].k = E[c].lo = E[c].hi = 0.f;
+                E[c].ent = 0u;
+                if (e < n_in) E[c] = load_elem(nullptr, e, chain, primf, cx, cy, cz, R, eps, true, balls);
+            }
+            int end = min(b + 32 * kBallChunks, n_in);
+            bool stopped = false;
+#pragma unroll
+            for (int c = 0; c < kBallChunks; ++c) {
+                const int e = b + 32 * c + lane;
+                const bool same = e == i || (E[c].op == op && runnable(E[c].op, E[c].k));
+                const unsigned stop = __ballot_sync(0xffffffffu, e < n_in && !same);
+                if (stop && !stopped) {
+                    stopped = true;
+                    end = b + 32 * c + __ffs(stop) - 1;
                 }
             }
+            float run = agg;
+#pragma unroll
+            for (int c = 0; c < kBallChunks; ++c)
+                if (b + 32 * c + lane < end) run = op == CH_UNION ? fminf(run, E[c].hi) : fmaxf(run, E[c].lo);
             for (int o = 16; o > 0; o >>= 1) {
-                const float t = __shfl_xor_sync(0xffffffffu, agg2, o);
-                agg2 = op == CH_UNION ? fminf(agg2, t) : fmaxf(agg2, t);
+                const float t = __shfl_xor_sync(0xffffffffu, run, o);
+                run = op == CH_UNION ? fminf(run, t) : fmaxf(run, t);
             }
-            rs = run_decide(op, agg2, alo, ahi);
-            n = rs.reset ? 0 : n0;  // compaction target: positions never above the ones being read
-            bool first = rs.reset;
-            for (int b = 0; b < nc; b += 32) {
-                bool keep = false;
-                Elem E;
-                if (b + lane < nc) {
-                    E = load_elem(out + n0, b + lane, chain, primf, cx, cy, cz, R, eps, true);
-                    keep = run_keep(op, E, rs.bound);
-                    if (keep) { klo = fminf(klo, E.lo); khi = fmaxf(khi, E.hi); }
-                }
-                const unsigned kept = __ballot_sync(0xffffffffu, keep);  // every read precedes the writes
-                if (keep) {
-                    const int pos = n + __popc(kept & below);
-                    uint32_t rec = E.ent;
-                    if (first && pos == 0) rec = (E.ent & ~3u) | (op == CH_SUBTRACT ? 2u : 1u);
-                    out[pos] = rec;
-                }
-                if (kept) first = false;
-                n += __popc(kept);
-            }
-        } else {
-            if (rs.reset) n = 0;
-            bool first = rs.reset;
-            // pass 2: keep / drop, ballot compaction in chain order
-            for (int b = i; b < j; b += 32) {
-                const int e = b + lane;
-                bool keep = false;
-                Elem E;
-                if (e < j) {
-                    E = load_elem(in, e, chain, primf, cx, cy, cz, R, eps, true);
-                    keep = run_keep(op, E, rs.bound);
-                    if (keep) { klo = fminf(klo, E.lo); khi = fmaxf(khi, E.hi); }
-                }
+            agg = run;
+#pragma unroll
+            for (int c = 0; c < kBallChunks; ++c) {
+                const bool keep = b + 32 * c + lane < end && run_keep(op, E[c], run);
                 const unsigned kept = __ballot_sync(0xffffffffu, keep);
                 if (keep) {
                     const int pos = n + __popc(kept & below);
-                    uint32_t rec = E.ent;
-                    if (first && pos == 0) rec = (E.ent & ~3u) | (op == CH_SUBTRACT ? 2u : 1u);
-                    if (pos < cap) out[pos] = rec;
+                    if (pos < cap) out[pos] = E[c].ent;
                 }
-                if (kept) first = false;
                 n += __popc(kept);
+            }
+            if (stopped) {
+                j = end;
+                break;
+            }
+        }
+        const int nc = n - n0;  // candidates at out[n0, n)
+        if (n > cap) {          // overflowed: the region falls back to its parent's list anyway
+            i = j;
+            continue;
+        }
+        __syncwarp();  // the candidates are read by other lanes
+        float agg2 = op == CH_UNION ? 3.0e38f : -3.0e38f;
+        for (int b = 0; b < nc; b += 32) {
+            if (b + lane < nc) {
+                const Elem E = load_elem(out + n0, b + lane, chain, primf, cx, cy, cz, R, eps, true);
+                if (b + lane < n_of) {  // kept for the decisions below (a lane reads what it wrote)
+                    klo_of[b + lane] = E.lo;
+                    khi_of[b + lane] = E.hi;
+                }
+                agg2 = op == CH_UNION ? fminf(agg2, E.hi) : fmaxf(agg2, E.lo);
             }
         }
         for (int o = 16; o > 0; o >>= 1) {
-            klo = fminf(klo, __shfl_xor_sync(0xffffffffu, klo, o));
-            khi = fmaxf(khi, __shfl_xor_sync(0xffffffffu, khi, o));
+            const float t = __shfl_xor_sync(0xffffffffu, agg2, o);
+            agg2 = op == CH_UNION ? fminf(agg2, t) : fmaxf(agg2, t);
         }
-        if (op == CH_UNION) {
-            alo = rs.reset ? klo : fminf(alo, klo);
-            ahi = rs.bound;
-        } else {
-            alo = rs.bound;
-            ahi = rs.reset ? khi : fmaxf(ahi, khi);
+        const RunState rs = run_decide(op, agg2, alo, ahi);
+        float klo = 3.0e38f, khi = -3.0e38f;
+        n = rs.reset ? 0 : n0;  // compaction target: positions never above the ones being read
+        bool first = rs.reset;
+        for (int b = 0; b < nc; b += 32) {
+            bool keep = false;
+            Elem E;
+            if (b + lane < nc) {
+                if (b + lane < n_of) {
+                    E.ent = out[n0 + b + lane];
+                    E.lo = klo_of[b + lane];
+                    E.hi = khi_of[b + lane];
+                } else {
+                    E = load_elem(out + n0, b + lane, chain, primf, cx, cy, cz, R, eps, true);
+                }
+                keep = run_keep(op, E, rs.bound);
+                if (keep) { klo = fminf(klo, E.lo); khi = fmaxf(khi, E.hi); }
+            }
+            const unsigned kept = __ballot_sync(0xffffffffu, keep);  // every read precedes the writes
+            if (keep) {
+                const int pos = n + __popc(kept & below);
+                uint32_t rec = E.ent;
+                if (first && pos == 0) rec = (E.ent & ~3u) | (op == CH_SUBTRACT ? 2u : 1u);
+                out[pos] = rec;
+            }
+            if (kept) first = false;
+            n += __popc(kept);
+            __syncwarp();
         }
+        end_run(op, rs, klo, khi, alo, ahi);
         i = j;
     }
     return n;
@@ -322,17 +437,7 @@ static __device__ __noinline__ int warp_walk_once(const uint32_t* in, int n_in, 
             n += __popc(kept);
             __syncwarp();
         }
-        for (int o = 16; o > 0; o >>= 1) {
-            klo = fminf(klo, __shfl_xor_sync(0xffffffffu, klo, o));
-            khi = fmaxf(khi, __shfl_xor_sync(0xffffffffu, khi, o));
-        }
-        if (run == CH_UNION) {
-            alo = rs.reset ? klo : fminf(alo, klo);
-            ahi = rs.bound;
-        } else {
-            alo = rs.bound;
-            ahi = rs.reset ? khi : fmaxf(ahi, khi);
-        }
+        end_run(run, rs, klo, khi, alo, ahi);
         run = -1;
     };
     for (int b = 0; b < n_in; b += 32) {

@@ -121,7 +121,7 @@ bool geom_ok(const FbGeom& g) {
 
 // ------------------------------------------------------------------------------------ scratch
 struct Plan {
-    int64_t primf, pool, off, len, status, misc, total;
+    int64_t primf, balls, pool, off, len, status, misc, total;
     int64_t blk_off, blk_len, blk_pool, blk_cap;  // per-block culled lists of active blocks
     int64_t pool_full, pool_coarse, pool_super;  // element offsets inside pool
     int64_t ntiles;
@@ -141,6 +141,7 @@ Plan make_plan(const Geo& G, int n_prims, int n_chain) {
     Plan p{};
     int64_t at = 0;
     p.primf = at; at += align256((int64_t)std::max(n_prims, 1) * sizeof(PrimF));
+    p.balls = at; at += align256((int64_t)std::max(n_prims, 1) * sizeof(Ball));
     p.cap_coarse = level_cap(G.ncoarse, kCapCoarse, n_chain);
     p.cap_super = level_cap(G.nsuper, kCapSuper, n_chain);
     p.pool_full = 0;
@@ -165,7 +166,7 @@ Plan make_plan(const Geo& G, int n_prims, int n_chain) {
 int64_t compact_scratch(int64_t nblocks) { return align256((nblocks + kTile - 1) / kTile * 8) + 256; }
 
 // ------------------------------------------------------------------------------------ prepare
-__device__ void prepare_prim(const FbPrim* __restrict__ prims, int i, PrimF* __restrict__ out) {
+__device__ void prepare_prim(const FbPrim* __restrict__ prims, int i, PrimF* __restrict__ out, Ball* __restrict__ balls) {
     const FbPrim P = prims[i];
     PrimF F;
     F.type = P.type;
@@ -270,11 +271,13 @@ __device__ void prepare_prim(const FbPrim* __restrict__ prims, int i, PrimF* __r
         F.p[11] = (float)(rw * (1.0 + 1e-6) + 1e-6 * mag);  // covers rounding the centre to float32
     }
     out[i] = F;
+    if (balls) balls[i] = Ball{F.p[8], F.p[9], F.p[10], F.p[11], F.ball_k, F.off, F.ball, 0.f};
 }
 
-__global__ void k_prepare_prims(const FbPrim* __restrict__ prims, int n, PrimF* __restrict__ out) {
+__global__ void k_prepare_prims(const FbPrim* __restrict__ prims, int n, PrimF* __restrict__ out,
+                                Ball* __restrict__ balls) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) prepare_prim(prims, i, out);
+    if (i < n) prepare_prim(prims, i, out, balls);
 }
 
 // sqrt_sum over n inputs (the self-test export fb_sqrt_sum_probe).
@@ -357,14 +360,22 @@ __device__ int seq_walk(const uint32_t* __restrict__ in, int n_in, const FbInsn*
     return n;
 }
 
+// A warp's candidates and survivors of one walk, in shared memory.
+constexpr int kWalked = 192;
+struct Walked {
+    uint32_t ent[kWalked];
+    float lo[kWalked], hi[kWalked];
+};
+
 // Level cull.  Regions of `edge` voxels on a (rnx, rny, rnz) grid; parent region = coords / div
 // on a (pnx, pny, pnz) grid (parent_off == nullptr: the single full list [0, n_full)).
 template <bool kBall>
 __device__ void cull_region(const Geo& G, const FbInsn* __restrict__ chain, const PrimF* __restrict__ primf,
+                            const Ball* __restrict__ balls,
                             uint32_t* __restrict__ pool, const int64_t* __restrict__ parent_off,
                             const int32_t* __restrict__ parent_len, int n_full, int div, int pny, int pnz,
                             int64_t* __restrict__ off, int32_t* __restrict__ len, int64_t pool_base, int cap, int edge,
-                            int rny, int rnz, int64_t r) {
+                            int rny, int rnz, int64_t r, Walked& walked) {
     const int rz = (int)(r % rnz), ry = (int)((r / rnz) % rny), rx = (int)(r / ((int64_t)rnz * rny));
     int64_t poff = 0;
     int plen = n_full;
@@ -379,8 +390,18 @@ __device__ void cull_region(const Geo& G, const FbInsn* __restrict__ chain, cons
     const float cz = G.fz0 + (rz * edge + half) * G.fpitch;
     const float R = 1.7320509f * half * G.fpitch;
     uint32_t* dst = pool + pool_base + r * cap;
-    const int n = warp_walk<kBall>(parent_off ? pool + poff : nullptr, plen, chain, primf, cx, cy, cz, R, G.eps, dst,
-                                   cap);
+    int n;
+    if (kBall) {
+        n = warp_walk_ball(plen, chain, primf, balls, cx, cy, cz, R, G.eps, dst, cap, walked.lo, walked.hi, kWalked);
+    } else {
+        const int lane = threadIdx.x & 31;
+        n = warp_walk_once(pool + poff, plen, chain, primf, cx, cy, cz, R, G.eps, walked.ent, walked.lo, walked.hi, kWalked);
+        if (n > kWalked) {
+            n = warp_walk(pool + poff, plen, chain, primf, cx, cy, cz, R, G.eps, dst, cap);
+        } else {
+            for (int i = lane; i < min(n, cap); i += 32) dst[i] = walked.ent[i];
+        }
+    }
     if ((threadIdx.x & 31) == 0) {
         if (n <= cap) {
             off[r] = pool_base + r * cap;
@@ -394,14 +415,16 @@ __device__ void cull_region(const Geo& G, const FbInsn* __restrict__ chain, cons
 
 template <bool kBall>
 __global__ void k_cull(Geo G, const FbInsn* __restrict__ chain, const PrimF* __restrict__ primf,
+                       const Ball* __restrict__ balls,
                        uint32_t* __restrict__ pool, const int64_t* __restrict__ parent_off,
                        const int32_t* __restrict__ parent_len, int n_full, int div, int pny, int pnz,
                        int64_t* __restrict__ off, int32_t* __restrict__ len, int64_t pool_base, int cap, int edge,
                        int rnx, int rny, int rnz) {
+    __shared__ Walked s_walked[4];
     const int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     if (r >= (int64_t)rnx * rny * rnz) return;
-    cull_region<kBall>(G, chain, primf, pool, parent_off, parent_len, n_full, div, pny, pnz, off, len, pool_base, cap,
-                       edge, rny, rnz, r);
+    cull_region<kBall>(G, chain, primf, balls, pool, parent_off, parent_len, n_full, div, pny, pnz, off, len, pool_base, cap,
+                       edge, rny, rnz, r, s_walked[threadIdx.x >> 5]);
 }
 
 
@@ -465,55 +488,197 @@ __device__ __forceinline__ double vertex_d(double origin, int64_t i, double pitc
     return rn_add(origin, rn_mul((double)i, pitch));
 }
 
-// Thread-per-block classification of a chain recipe: thread t of the superblock-major order --
-// threads of one superblock are consecutive, so a warp never spans two superblocks and walks in
-// lockstep with broadcast loads -- evaluates its block's 8 corners in float32 in block-local
-// coordinates.  The block culls the superblock list itself (seq_walk, kCapBlock entries) and an
-// active block keeps that list for the leaf pass and point queries: the warp's lists are
-// placed with one atomicAdd on `cursor` (blk_len -1 where a list overflowed or the pool is full;
-// the leaf pass then culls the block itself).  Every lane of a warp reaches the placement, so
-// threads outside the grid only skip the evaluation.
 template <int VG, bool kEdge = true>
 __device__ __forceinline__ uint32_t eval_group(const LocalPrim& P, float dx, float dy, const float* dz, float* v);
 template <int VG>
 __device__ __forceinline__ void combine_group(int op, float k, float* acc, const float* v);
 
-__device__ void classify_block(const Geo& G, const FbPrim* __restrict__ prims, const PrimF* __restrict__ primf,
-                               const FbInsn* __restrict__ chain, const uint32_t* __restrict__ pool,
-                               const int64_t* __restrict__ sb_off, const int32_t* __restrict__ sb_len,
-                               int32_t* __restrict__ kind, float* __restrict__ cma, int32_t* __restrict__ blk_off,
-                               int32_t* __restrict__ blk_len, uint32_t* __restrict__ blk_pool, int64_t blk_cap,
-                               int* __restrict__ cursor, int64_t t) {
-    const int S = G.S;
-    const int T = threads_per_super(S);
-    const int64_t s_id = t / T;
-    const int local = (int)(t % T);
-    const int sz = (int)(s_id % G.nsz), sy = (int)((s_id / G.nsz) % G.nsy), sx = (int)(s_id / ((int64_t)G.nsz * G.nsy));
-    const int bi = sx * S + local / (S * S), bj = sy * S + (local / S) % S, bk = sz * S + local % S;
-    const bool valid = s_id < G.nsuper && local < S * S * S && bi < G.nbx && bj < G.nby && bk < G.nbz;
-    const int64_t b = ((int64_t)bi * G.nby + bj) * G.nbz + bk;
+// One element's values at a block's 8 corners combined into v, in block-local coordinates; nonzero
+// where a corner sampled a grid table at its boundary.
+__device__ __forceinline__ uint32_t corner_element(const FbPrim& D, const PrimF& F, double ox, double oy, double oz,
+                                                   int op, float k, float side, float* v) {
+    LocalPrim P;
+    // canonical forms (no extent): the corner decisions have the float64 guard band
+    localise(D, F, ox, oy, oz, op, k, P);
+    // the corners as 4 (x, y) columns of 2 along z: one inlined evaluation body (the kind
+    // switch outside, the points inside) walked over the columns, the corner values rotated
+    // through registers -- 8 unrolled kind switches would not fit the instruction cache
+    const float dz2[2] = {0.f, side};
+    uint32_t edge = 0;
+    for (int col = 0; col < 4; ++col) {
+        float pv[2], acc2[2] = {v[0], v[4]};
+        edge |= eval_group<2>(P, (col & 1) ? side : 0.f, (col & 2) ? side : 0.f, dz2, pv);
+        combine_group<2>(op, k, acc2, pv);
+        const float t0 = acc2[0], t4 = acc2[1];
+        v[0] = v[1]; v[1] = v[2]; v[2] = v[3]; v[3] = t0;
+        v[4] = v[5]; v[5] = v[6]; v[6] = v[7]; v[7] = t4;
+    }
+    return edge;
+}
+
+// Where a warp's blocks' lists go in the pool: lane's first slot, from an inclusive scan of their
+// lengths and one atomicAdd (`need` 0: none).  Every lane of the warp calls it.
+__device__ __forceinline__ int64_t place_lists(int need, int* __restrict__ cursor) {
+    const int lane = threadIdx.x & 31;
+    int incl = need;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    const int total = __shfl_sync(0xffffffffu, incl, 31);
+    int base = 0;
+    if (lane == 31 && total > 0) base = atomicAdd(cursor, total);
+    return (int64_t)__shfl_sync(0xffffffffu, base, 31) + incl - need;
+}
+
+// One block of the grid: its indices, and its corner at float64.
+struct BlockAt {
+    int bi, bj, bk;
+    bool valid;
+    int64_t b;
+};
+
+// A warp's blocks share a subset of their superblock's list: what the list is culled to for the warp's
+// brick of 2 x 4 x 4 blocks (warp_walk_once, kSubset entries at most).  Each lane walks the subset for
+// its block -- the walk of seq_walk, but a kept element is a bit, and its bounds are formed a second
+// time only where some lane still has it as a candidate -- and the corners take the union of the lanes'
+// elements one at a time, so every load is a broadcast and the kind is the warp's.
+constexpr int kSubset = 96;
+constexpr int kShortList = 24;  // lists up to this are not worth a warp's walk
+
+struct Subset {  // shared, per warp
+    uint32_t ent[kSubset];
+    float lo[kSubset], hi[kSubset];
+};
+
+struct Bits96 {
+    uint32_t w[3];
+    __device__ __forceinline__ void clear() { w[0] = w[1] = w[2] = 0u; }
+    __device__ __forceinline__ void set(int e, bool on) {  // e the same in every lane
+        const uint32_t bit = on ? 1u << (e & 31) : 0u;
+        if (e < 32) w[0] |= bit;
+        else if (e < 64) w[1] |= bit;
+        else w[2] |= bit;
+    }
+    __device__ __forceinline__ bool get(int e) const {
+        return (e < 32 ? w[0] : (e < 64 ? w[1] : w[2])) >> (e & 31) & 1u;
+    }
+    __device__ __forceinline__ int count() const { return __popc(w[0]) + __popc(w[1]) + __popc(w[2]); }
+    __device__ __forceinline__ int lowest() const {
+        return w[0] ? __ffs(w[0]) - 1 : (w[1] ? 31 + __ffs(w[1]) : (w[2] ? 63 + __ffs(w[2]) : -1));
+    }
+};
+
+// The entry of bit e of a block's elements: its lowest one carries the block's own set mode.
+__device__ __forceinline__ uint32_t subset_entry(const uint32_t* ent, int e, int lowest, uint32_t head) {
+    return e == lowest && head ? (ent[e] & ~3u) | head : ent[e];
+}
+
+// float64 value of a block's elements at a world point (guard-band recheck).
+__device__ __noinline__ double subset_eval_d(const uint32_t* ent, Bits96 K, uint32_t head,
+                                             const FbInsn* __restrict__ chain, const FbPrim* __restrict__ prims,
+                                             double x, double y, double z) {
+    double acc = 0.0;
+    const int lowest = K.lowest();
+    for (int w = 0; w < 3; ++w)
+        for (uint32_t m = K.w[w]; m; m &= m - 1) {
+            const uint32_t e = subset_entry(ent, 32 * w + __ffs(m) - 1, lowest, head);
+            const FbInsn I = chain[e >> 2];
+            const int op = effective_op(e, I.op);
+            const double v = op == CH_OFFSET ? 0.0 : prim_world_d(prims[I.arg], x, y, z);
+            acc = chain_apply_d(op, acc, v, I.k);
+        }
+    return acc;
+}
+
+// seq_walk over the warp's subset; K receives the lane's elements and `head` the set mode of its lowest.
+__device__ __forceinline__ void subset_walk(const uint32_t* ent, int m, const FbInsn* __restrict__ chain,
+                                            const PrimF* __restrict__ primf, float cx, float cy, float cz, float R,
+                                            float eps, Bits96& K, uint32_t& head) {
+    float alo = 0.f, ahi = 0.f, agg = 0.f;
+    K.clear();
+    head = 0u;
+    Bits96 cand;
+    cand.clear();
+    int run = -1, i0 = 0;  // the open run's operation (-1: none) and first element
+    for (int i = 0; i <= m; ++i) {  // two copies of load_elem in all: the code has to stay small
+        Elem E;
+        E.op = -1;
+        E.k = 0.f;
+        if (i < m) E = load_elem(ent, i, chain, primf, cx, cy, cz, R, eps, true);
+        const bool hard = i < m && runnable(E.op, E.k);
+        if (run >= 0 && !(hard && E.op == run)) {  // the run ends: its elements by their final bound
+            const RunState rs = run_decide(run, agg, alo, ahi);
+            if (rs.reset) {
+                K.clear();
+                head = run == CH_SUBTRACT ? 2u : 1u;
+            }
+            float klo = 3.0e38f, khi = -3.0e38f;
+            for (int e = i0; e < i; ++e) {
+                const bool c = cand.get(e);
+                if (!__any_sync(0xffffffffu, c)) continue;
+                const Elem F = load_elem(ent, e, chain, primf, cx, cy, cz, R, eps, true);
+                const bool keep = c && run_keep(run, F, rs.bound);
+                K.set(e, keep);
+                if (keep) {
+                    klo = fminf(klo, F.lo);
+                    khi = fmaxf(khi, F.hi);
+                }
+            }
+            if (run == CH_UNION) {
+                alo = rs.reset ? klo : fminf(alo, klo);
+                ahi = rs.bound;
+            } else {
+                alo = rs.bound;
+                ahi = rs.reset ? khi : fmaxf(ahi, khi);
+            }
+            run = -1;
+        }
+        if (i == m) break;
+        if (!hard) {
+            const int act = single_step(E, alo, ahi);
+            if (act >= 2) {
+                K.clear();
+                head = (uint32_t)(act - 1);
+            }
+            K.set(i, act != 0);
+            continue;
+        }
+        if (run < 0) {
+            run = E.op;
+            i0 = i;
+            agg = run == CH_UNION ? 3.0e38f : -3.0e38f;
+        }
+        agg = run == CH_UNION ? fminf(agg, E.hi) : fmaxf(agg, E.lo);
+        cand.set(i, run_keep(run, E, agg));  // candidate: not beaten by the bound so far
+    }
+}
+
+// Where threads' blocks do not share a subset (superblocks of 1 or 8 blocks, several to a warp, or a
+// subset that did not fit): each block culls its superblock's list itself (seq_walk).
+__device__ __noinline__ void classify_alone(const Geo& G, const BlockAt& A, const FbPrim* __restrict__ prims,
+                                            const PrimF* __restrict__ primf, const FbInsn* __restrict__ chain,
+                                            const uint32_t* __restrict__ plist, int plen, int32_t* __restrict__ kind,
+                                            float* __restrict__ cma, int32_t* __restrict__ blk_off,
+                                            int32_t* __restrict__ blk_len, uint32_t* __restrict__ blk_pool,
+                                            int64_t blk_cap, int* __restrict__ cursor) {
     const int B = G.B;
     uint32_t blist[kCapBlock];
     int nblist = -1;
     int kd = 1;
-    if (valid) {
-        const uint32_t* list;
-        int len;
-        const uint32_t* plist = pool + sb_off[s_id];
-        const int plen = sb_len[s_id];
+    if (A.valid) {
         const float half = 0.5f * B;
-        const int n = seq_walk(plist, plen, chain, primf, G.fx0 + (bi * B + half) * G.fpitch,
-                               G.fy0 + (bj * B + half) * G.fpitch, G.fz0 + (bk * B + half) * G.fpitch,
+        const int n = seq_walk(plist, plen, chain, primf, G.fx0 + (A.bi * B + half) * G.fpitch,
+                               G.fy0 + (A.bj * B + half) * G.fpitch, G.fz0 + (A.bk * B + half) * G.fpitch,
                                1.7320509f * half * G.fpitch, G.eps, blist, kCapBlock);
         nblist = n;
-        list = n <= kCapBlock ? blist : plist;
-        len = n <= kCapBlock ? n : plen;
-        const double ox = G.x0 + (double)(bi * B) * G.pitch;
-        const double oy = G.y0 + (double)(bj * B) * G.pitch;
-        const double oz = G.z0 + (double)(bk * B) * G.pitch;
-        const float side = (float)B * G.fpitch;
+        const uint32_t* list = n <= kCapBlock ? blist : plist;
+        const int len = n <= kCapBlock ? n : plen;
+        const double ox = G.x0 + (double)(A.bi * B) * G.pitch;
+        const double oy = G.y0 + (double)(A.bj * B) * G.pitch;
+        const double oz = G.z0 + (double)(A.bk * B) * G.pitch;
         float v[8];
-        bool edge = false;  // a corner sampled a grid table at its boundary: decide in float64
+        uint32_t edge = 0;  // a corner sampled a grid table at its boundary: decide in float64
 #pragma unroll
         for (int c = 0; c < 8; ++c) v[c] = 0.f;
         for (int i = 0; i < len; ++i) {
@@ -526,56 +691,154 @@ __device__ void classify_block(const Geo& G, const FbPrim* __restrict__ prims, c
                 for (int c = 0; c < 8; ++c) v[c] -= k;
                 continue;
             }
-            LocalPrim P;
-            // canonical forms (no extent): the corner decisions have the float64 guard band
-            localise(prims[I.arg], primf[I.arg], ox, oy, oz, op, k, P);
-            // the corners as 4 (x, y) columns of 2 along z: one inlined evaluation body (the kind
-            // switch outside, the points inside) walked over the columns, the corner values rotated
-            // through registers -- 8 unrolled kind switches would not fit the instruction cache
-            const float dz2[2] = {0.f, side};
-            for (int col = 0; col < 4; ++col) {
-                float pv[2], acc2[2] = {v[0], v[4]};
-                edge |= eval_group<2>(P, (col & 1) ? side : 0.f, (col & 2) ? side : 0.f, dz2, pv) != 0;
-                combine_group<2>(op, k, acc2, pv);
-                const float t0 = acc2[0], t4 = acc2[1];
-                v[0] = v[1]; v[1] = v[2]; v[2] = v[3]; v[3] = t0;
-                v[4] = v[5]; v[5] = v[6]; v[6] = v[7]; v[7] = t4;
-            }
+            edge |= corner_element(prims[I.arg], primf[I.arg], ox, oy, oz, op, k, (float)B * G.fpitch, v);
         }
         if (edge) v[0] = __int_as_float(0x7fc00000);  // NaN: decide_block takes the float64 path
         float m;
         kd = decide_block(G, v, m, [&](int c) {
-            return list_eval_d(list, len, chain, prims, vertex_d(G.x0, (int64_t)bi * B + (c & 1) * B, G.pitch),
-                               vertex_d(G.y0, (int64_t)bj * B + ((c >> 1) & 1) * B, G.pitch),
-                               vertex_d(G.z0, (int64_t)bk * B + ((c >> 2) & 1) * B, G.pitch));
+            return list_eval_d(list, len, chain, prims, vertex_d(G.x0, (int64_t)A.bi * B + (c & 1) * B, G.pitch),
+                               vertex_d(G.y0, (int64_t)A.bj * B + ((c >> 1) & 1) * B, G.pitch),
+                               vertex_d(G.z0, (int64_t)A.bk * B + ((c >> 2) & 1) * B, G.pitch));
         });
-        kind[b] = kd;
-        cma[b] = m;
+        kind[A.b] = kd;
+        cma[A.b] = m;
     }
-    {
-        // the warp's active blocks' lists: an inclusive scan of their lengths, one atomicAdd
-        const int lane = threadIdx.x & 31;
-        const bool keep = valid && kd == 0 && nblist >= 0 && nblist <= kCapBlock;
-        const int need = keep ? nblist : 0;
-        int incl = need;
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += y;
+    const bool keep = A.valid && kd == 0 && nblist >= 0 && nblist <= kCapBlock;
+    const int need = keep ? nblist : 0;
+    const int64_t slot = place_lists(need, cursor);
+    if (A.valid && kd == 0) {
+        int len_b = -1;
+        if (keep && slot + need <= blk_cap) {
+            for (int i = 0; i < need; ++i) blk_pool[slot + i] = blist[i];
+            blk_off[A.b] = (int32_t)slot;
+            len_b = need;
         }
-        const int total = __shfl_sync(0xffffffffu, incl, 31);
-        int base = 0;
-        if (lane == 31 && total > 0) base = atomicAdd(cursor, total);
-        base = __shfl_sync(0xffffffffu, base, 31);
-        if (valid && kd == 0) {
-            const int64_t slot = (int64_t)base + incl - need;
-            int len_b = -1;
-            if (keep && slot + need <= blk_cap) {
-                for (int i = 0; i < need; ++i) blk_pool[slot + i] = blist[i];
-                blk_off[b] = (int32_t)slot;
-                len_b = need;
+        blk_len[A.b] = len_b;  // -1: the leaf pass culls the block itself
+    }
+}
+
+// Thread-per-block classification of a chain recipe: thread t of the superblock-major order --
+// threads of one superblock are consecutive, and a warp's 32 blocks of it form a brick -- evaluates its
+// block's 8 corners in float32 in block-local coordinates on the block's own culled list, which an
+// active block keeps for the leaf pass and point queries: the warp's lists are placed with one
+// atomicAdd on `cursor` (blk_len -1 where a list is longer than kCapBlock or the pool is full; the
+// leaf pass then culls the block itself).  Every lane of a warp reaches the placement, so threads
+// outside the grid only skip the evaluation.
+// Bound by instruction issue: walking the superblock's whole list twice per block and evaluating each
+// block's own list with the warp's kinds diverging took 9.9 k instructions a warp on 4^3 blocks of a
+// 512^3 part (1500 elements), 5.7 k now (1006 -> 625 us).  Where superblock lists are short it gains
+// little (1024^3 part of 4096 elements, 16 in a list: 729 -> 705 us; a batch of 20: 2.43 -> 2.04 ms, most
+// of it from 5 CTAs per SM below).
+__device__ __forceinline__ void classify_block(const Geo& G, const FbPrim* __restrict__ prims,
+                                               const PrimF* __restrict__ primf, const FbInsn* __restrict__ chain,
+                                               const uint32_t* __restrict__ pool, const int64_t* __restrict__ sb_off,
+                                               const int32_t* __restrict__ sb_len, int32_t* __restrict__ kind,
+                                               float* __restrict__ cma, int32_t* __restrict__ blk_off,
+                                               int32_t* __restrict__ blk_len, uint32_t* __restrict__ blk_pool,
+                                               int64_t blk_cap, int* __restrict__ cursor, int64_t t, Subset& sub) {
+    const int S = G.S, B = G.B;  // S is 1, 2, 4 or 8: T = S^3 threads a superblock, and shifts for divisions
+    const int T = threads_per_super(S);
+    const int64_t s_id = t >> (__ffs(T) - 1);
+    const int local = (int)(t & (T - 1));
+    // superblocks are at most (16384 / 16)^3 = 2^30
+    const uint32_t row = (uint32_t)s_id / (uint32_t)G.nsz;
+    const int sz = (int)((uint32_t)s_id - row * (uint32_t)G.nsz);
+    const int sx = (int)(row / (uint32_t)G.nsy), sy = (int)(row - (uint32_t)sx * (uint32_t)G.nsy);
+    const bool bricks = S >= 4;
+    BlockAt A;
+    int wi = 0, wj = 0, wk = 0;  // the warp's brick's first block in the superblock
+    if (bricks) {
+        const int q = S == 8 ? 1 : 0, w = local >> 5, l = local & 31;  // 2^q bricks along y and z
+        wi = (w >> (2 * q)) * 2;
+        wj = ((w >> q) & q) * 4;
+        wk = (w & q) * 4;
+        A.bi = sx * S + wi + (l >> 4);
+        A.bj = sy * S + wj + ((l >> 2) & 3);
+        A.bk = sz * S + wk + (l & 3);
+    } else {
+        A.bi = sx * S + local / (S * S);
+        A.bj = sy * S + (local / S) % S;
+        A.bk = sz * S + local % S;
+    }
+    A.valid = s_id < G.nsuper && local < S * S * S && A.bi < G.nbx && A.bj < G.nby && A.bk < G.nbz;
+    A.b = ((int64_t)A.bi * G.nby + A.bj) * G.nbz + A.bk;
+    const bool any = s_id < G.nsuper;  // the same for the whole warp where it has a brick
+    const uint32_t* plist = any ? pool + sb_off[s_id] : pool;
+    const int plen = any ? sb_len[s_id] : 0;
+    int m = kSubset + 1;
+    const uint32_t* ent = plist;  // a short list is the subset as it is
+    if (bricks && any && plen <= kShortList) {
+        m = plen;
+    } else if (bricks && any) {
+        ent = sub.ent;
+        const float fb = (float)B;
+        m = warp_walk_once(plist, plen, chain, primf, G.fx0 + ((sx * S + wi) * fb + fb) * G.fpitch,
+                           G.fy0 + ((sy * S + wj) * fb + 2.f * fb) * G.fpitch,
+                           G.fz0 + ((sz * S + wk) * fb + 2.f * fb) * G.fpitch, 3.0001f * fb * G.fpitch, G.eps, sub.ent,
+                           sub.lo, sub.hi, kSubset);
+    }
+    if (m > kSubset) {
+        classify_alone(G, A, prims, primf, chain, plist, plen, kind, cma, blk_off, blk_len, blk_pool, blk_cap, cursor);
+        return;
+    }
+    const float half = 0.5f * B;
+    Bits96 K;
+    uint32_t head;
+    // lanes outside the grid walk along (their superblock's list bounds them as well as any)
+    subset_walk(ent, m, chain, primf, G.fx0 + (A.bi * B + half) * G.fpitch, G.fy0 + (A.bj * B + half) * G.fpitch,
+                G.fz0 + (A.bk * B + half) * G.fpitch, 1.7320509f * half * G.fpitch, G.eps, K, head);
+    const int lowest = K.lowest();
+    const double ox = G.x0 + (double)(A.bi * B) * G.pitch;
+    const double oy = G.y0 + (double)(A.bj * B) * G.pitch;
+    const double oz = G.z0 + (double)(A.bk * B) * G.pitch;
+    float v[8];
+    uint32_t edge = 0;  // a corner sampled a grid table at its boundary: decide in float64
+#pragma unroll
+    for (int c = 0; c < 8; ++c) v[c] = 0.f;
+    for (int w = 0; w < 3; ++w) {
+        const uint32_t mine = A.valid ? (w == 0 ? K.w[0] : (w == 1 ? K.w[1] : K.w[2])) : 0u;
+        for (uint32_t u = __reduce_or_sync(0xffffffffu, mine); u; u &= u - 1) {
+            const int bit = __ffs(u) - 1, e = 32 * w + bit;
+            if (!((mine >> bit) & 1u)) continue;
+            const uint32_t rec = subset_entry(ent, e, lowest, head);
+            const FbInsn I = chain[rec >> 2];
+            const int op = effective_op(rec, I.op);
+            const float k = (float)I.k;
+            if (op == CH_OFFSET) {
+#pragma unroll
+                for (int c = 0; c < 8; ++c) v[c] -= k;
+            } else {
+                edge |= corner_element(prims[I.arg], primf[I.arg], ox, oy, oz, op, k, (float)B * G.fpitch, v);
             }
-            blk_len[b] = len_b;  // -1: the leaf pass culls the block itself
         }
+    }
+    int kd = 1;
+    if (A.valid) {
+        if (edge) v[0] = __int_as_float(0x7fc00000);  // NaN: decide_block takes the float64 path
+        float mn;
+        kd = decide_block(G, v, mn, [&](int c) {
+            return subset_eval_d(ent, K, head, chain, prims, vertex_d(G.x0, (int64_t)A.bi * B + (c & 1) * B, G.pitch),
+                                 vertex_d(G.y0, (int64_t)A.bj * B + ((c >> 1) & 1) * B, G.pitch),
+                                 vertex_d(G.z0, (int64_t)A.bk * B + ((c >> 2) & 1) * B, G.pitch));
+        });
+        kind[A.b] = kd;
+        cma[A.b] = mn;
+    }
+    const int n = K.count();
+    const bool keep = A.valid && kd == 0 && n <= kCapBlock;
+    const int need = keep ? n : 0;
+    const int64_t slot = place_lists(need, cursor);
+    if (A.valid && kd == 0) {
+        int len_b = -1;
+        if (keep && slot + need <= blk_cap) {
+            int i = 0;
+            for (int w = 0; w < 3; ++w)
+                for (uint32_t u = w == 0 ? K.w[0] : (w == 1 ? K.w[1] : K.w[2]); u; u &= u - 1)
+                    blk_pool[slot + i++] = subset_entry(ent, 32 * w + __ffs(u) - 1, lowest, head);
+            blk_off[A.b] = (int32_t)slot;
+            len_b = need;
+        }
+        blk_len[A.b] = len_b;  // -1: the leaf pass culls the block itself
     }
 }
 
@@ -590,9 +853,10 @@ __global__ void __launch_bounds__(128, 6) k_classify_blocks(Geo G, const FbPrim*
                                                              int32_t* __restrict__ blk_off, int32_t* __restrict__ blk_len,
                                                              uint32_t* __restrict__ blk_pool, int64_t blk_cap,
                                                              int* __restrict__ cursor) {
+    __shared__ Subset s_sub[4];
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     classify_block(G, prims, primf, chain, pool, sb_off, sb_len, kind, cma, blk_off, blk_len, blk_pool, blk_cap, cursor,
-                   t);
+                   t, s_sub[threadIdx.x >> 5]);
 }
 
 // ------------------------------------------------------------------------------------ general programs
@@ -1944,6 +2208,7 @@ struct Scratch {
     int32_t* blk_len;
     uint32_t* blk_pool;
     PrimF* primf;
+    Ball* balls;
     uint32_t* pool;
     int64_t* off;
     int32_t* len;
@@ -1955,6 +2220,7 @@ Scratch carve(void* base, const Plan& p, const Geo& G) {
     char* b = static_cast<char*>(base);
     Scratch s;
     s.primf = reinterpret_cast<PrimF*>(b + p.primf);
+    s.balls = reinterpret_cast<Ball*>(b + p.balls);
     s.pool = reinterpret_cast<uint32_t*>(b + p.pool);
     s.off = reinterpret_cast<int64_t*>(b + p.off);
     s.len = reinterpret_cast<int32_t*>(b + p.len);
@@ -1987,18 +2253,18 @@ int classify_impl(const FbGeom& g, const FbPrim* prims, int n_prims, const FbIns
     const Plan P = make_plan(G, n_prims, n_chain);
     if (scratch_len < P.total) return FB_INVALID;
     Scratch S = carve(scratch, P, G);
-    k_prepare_prims<<<fb_div_up(n_prims, 128), 128, 0, st>>>(prims, n_prims, S.primf);
+    k_prepare_prims<<<fb_div_up(n_prims, 128), 128, 0, st>>>(prims, n_prims, S.primf, S.balls);
     FB_LAUNCH();
     if (mode == 1) {
         k_full_list<<<fb_div_up(n_chain, 256), 256, 0, st>>>(S.pool + P.pool_full, n_chain);
         FB_LAUNCH();
         // coarse regions from the full chain
-        k_cull<true><<<fb_div_up(G.ncoarse * 32, 128), 128, 0, st>>>(G, chain, S.primf, S.pool, nullptr, nullptr, n_chain, 1,
+        k_cull<true><<<fb_div_up(G.ncoarse * 32, 128), 128, 0, st>>>(G, chain, S.primf, S.balls, S.pool, nullptr, nullptr, n_chain, 1,
                                                                1, 1, S.off, S.len, P.pool_coarse, P.cap_coarse,
                                                                G.S * G.B * kCoarseDiv, G.ncx, G.ncy, G.ncz);
         FB_LAUNCH();
         // superblocks from their coarse region
-        k_cull<false><<<fb_div_up(G.nsuper * 32, 128), 128, 0, st>>>(G, chain, S.primf, S.pool, S.off, S.len, 0, kCoarseDiv,
+        k_cull<false><<<fb_div_up(G.nsuper * 32, 128), 128, 0, st>>>(G, chain, S.primf, S.balls, S.pool, S.off, S.len, 0, kCoarseDiv,
                                                               G.ncy, G.ncz, S.off + G.ncoarse, S.len + G.ncoarse,
                                                               P.pool_super, P.cap_super, G.S * G.B, G.nsx, G.nsy, G.nsz);
         FB_LAUNCH();
@@ -2076,6 +2342,7 @@ struct RecDesc {
     Geo G;
     const FbPrim* prims;
     PrimF* primf;
+    Ball* balls;
     const FbInsn* chain;
     int32_t n_prims, n_chain;
     uint32_t* pool;
@@ -2118,7 +2385,7 @@ __global__ void k_b_prepare(const RecDesc* __restrict__ D, Group W, int64_t tota
     if (g >= total) return;
     const int j = group_find(W, g);
     const RecDesc& R = D[W.rec[j]];
-    prepare_prim(R.prims, (int)(g - W.pre[j]), R.primf);
+    prepare_prim(R.prims, (int)(g - W.pre[j]), R.primf, R.balls);
 }
 
 __global__ void k_b_full_list(const RecDesc* __restrict__ D, Group W, int64_t total) {
@@ -2133,6 +2400,8 @@ __global__ void k_b_full_list(const RecDesc* __restrict__ D, Group W, int64_t to
 // coarse region.
 template <int kLevel>
 __global__ void __launch_bounds__(128) k_b_cull(const RecDesc* __restrict__ D, Group W, int64_t total) {
+    __shared__ Walked s_walked[4];
+    Walked& walked = s_walked[threadIdx.x >> 5];
     const int64_t g = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     if (g >= total) return;
     const int j = group_find(W, g);
@@ -2140,24 +2409,28 @@ __global__ void __launch_bounds__(128) k_b_cull(const RecDesc* __restrict__ D, G
     const Geo& G = R.G;
     const int64_t r = g - W.pre[j];
     if (kLevel == 0)
-        cull_region<true>(G, R.chain, R.primf, R.pool, nullptr, nullptr, R.n_chain, 1, 1, 1, R.off, R.len,
-                          R.pool_coarse, R.cap_coarse, G.S * G.B * kCoarseDiv, G.ncy, G.ncz, r);
+        cull_region<true>(G, R.chain, R.primf, R.balls, R.pool, nullptr, nullptr, R.n_chain, 1, 1, 1, R.off, R.len,
+                          R.pool_coarse, R.cap_coarse, G.S * G.B * kCoarseDiv, G.ncy, G.ncz, r, walked);
     else
-        cull_region<false>(G, R.chain, R.primf, R.pool, R.off, R.len, 0, kCoarseDiv, G.ncy, G.ncz, R.off + G.ncoarse,
-                           R.len + G.ncoarse, R.pool_super, R.cap_super, G.S * G.B, G.nsy, G.nsz, r);
+        cull_region<false>(G, R.chain, R.primf, R.balls, R.pool, R.off, R.len, 0, kCoarseDiv, G.ncy, G.ncz, R.off + G.ncoarse,
+                           R.len + G.ncoarse, R.pool_super, R.cap_super, G.S * G.B, G.nsy, G.nsz, r, walked);
 }
 
 
 // Each recipe's thread range is a multiple of 32 (nsuper x threads_per_super), so a warp never
 // spans two recipes.
-__global__ void __launch_bounds__(128, 6) k_b_classify_blocks(const RecDesc* __restrict__ D, Group W, int64_t total,
+// 5 CTAs per SM (96 registers; the descriptors' loads spill less): 2.38 -> 2.04 ms for a batch of 20, where
+// the single-recipe kernel keeps 6 (705 against 718 us on the 1024^3 part).
+__global__ void __launch_bounds__(128, 5) k_b_classify_blocks(const RecDesc* __restrict__ D, Group W, int64_t total,
                                                                int* __restrict__ cursors) {
+    __shared__ Subset s_sub[4];
     const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (g >= total) return;
     const int j = group_find(W, g);
     const RecDesc& R = D[W.rec[j]];
     classify_block(R.G, R.prims, R.primf, R.chain, R.pool, R.off + R.G.ncoarse, R.len + R.G.ncoarse, R.kind,
-                          R.cma, R.blk_off, R.blk_len, R.blk_pool, R.blk_cap, &cursors[W.rec[j]], g - W.pre[j]);
+                          R.cma, R.blk_off, R.blk_len, R.blk_pool, R.blk_cap, &cursors[W.rec[j]], g - W.pre[j],
+                   s_sub[threadIdx.x >> 5]);
 }
 
 
@@ -2336,6 +2609,7 @@ void* fb_batch_create(const FbBatchItem* items, int32_t n, void* stream) noexcep
             d.G = G;
             d.prims = it.d_prims;
             d.primf = S.primf;
+            d.balls = S.balls;
             d.chain = it.d_chain;
             d.n_prims = it.n_prims;
             d.n_chain = it.n_chain;
@@ -2741,7 +3015,7 @@ int fb_field_reconstruct_device(const int32_t* d_kind, const int32_t* d_active, 
 int fb_query_prepare(const FbPrim* d_prims, int32_t n_prims, void* d_primf, void* stream) noexcept {
     if (!d_prims || !d_primf || n_prims < 1) return FB_INVALID;
     k_prepare_prims<<<fb_div_up(n_prims, 128), 128, 0, static_cast<cudaStream_t>(stream)>>>(
-        d_prims, n_prims, static_cast<PrimF*>(d_primf));
+        d_prims, n_prims, static_cast<PrimF*>(d_primf), nullptr);
     FB_LAUNCH();
     return FB_OK;
 }
