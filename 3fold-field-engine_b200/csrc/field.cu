@@ -726,7 +726,7 @@ __device__ __noinline__ void classify_alone(const Geo& G, const BlockAt& A, cons
 // outside the grid only skip the evaluation.
 // Bound by instruction issue: walking the superblock's whole list twice per block and evaluating each
 // block's own list with the warp's kinds diverging took 9.9 k instructions a warp on 4^3 blocks of a
-// 512^3 part (1500 elements), 5.7 k now (1006 -> 625 us).  Where superblock lists are short it gains
+// 512^3 part (1500 elements), 5.7 k now (1006 -> 622 us).  Where superblock lists are short it gains
 // little (1024^3 part of 4096 elements, 16 in a list: 729 -> 705 us; a batch of 20: 2.43 -> 2.04 ms, most
 // of it from 5 CTAs per SM below).
 __device__ __forceinline__ void classify_block(const Geo& G, const FbPrim* __restrict__ prims,
