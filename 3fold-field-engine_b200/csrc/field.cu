@@ -227,6 +227,10 @@ __device__ void prepare_prim(const FbPrim* __restrict__ prims, int i, PrimF* __r
         F.p[11] = __uint_as_float((unsigned)(t >> 32));
         break;
     }
+    case P_HALFSPACE:  // n . x: as steep as its normal is long (recipes may carry any normal)
+        canon = sqrt(p[0] * p[0] + p[1] * p[1] + p[2] * p[2]);
+        for (int j = 0; j < 3; ++j) F.p[j] = (float)p[j];
+        break;
     default:
         for (int j = 0; j < 12; ++j) F.p[j] = (float)p[j];
     }

@@ -325,6 +325,8 @@ def _canon_lipschitz(p):
     if p["type"] == P_CONE:
         r1, r2, h = p["p"][0], p["p"][1], p["p"][2]
         return 2.0 + abs(r2 - r1) / h
+    if p["type"] == P_HALFSPACE:
+        return float(np.linalg.norm(p["p"][:3]))
     return 1.0
 
 
