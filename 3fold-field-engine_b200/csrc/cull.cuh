@@ -66,11 +66,20 @@ __device__ __forceinline__ float primf_world_common(const PrimF& P, float x, flo
     return fmaf(P.s, c, -P.off);
 }
 
-// Interval of one chain element's primitive around (cx, cy, cz) with radius R.
+// A region's radius for element_interval, widened so that the bound also covers the float32 rounding that
+// comes with the coordinates (32 u |A| |x|_1 of PrimF.err's rule; |A|_1 is at most sqrt(3) of the norm in
+// `lip`).  What comes with a primitive's own frame is PrimF.err: a sphere of radius 300 through a unit
+// grid rounds by 4e-5 there, twenty times the grid's own 16 ulps.
+__device__ __forceinline__ float bounds_radius(float cx, float cy, float cz, float R) {
+    return fmaf(3.4e-6f, fabsf(cx) + fabsf(cy) + fabsf(cz) + 2.f * R, R);
+}
+
+// Interval of one chain element's primitive around (cx, cy, cz) with radius R (bounds_radius): holds every
+// value of it there, exact or computed in float32.
 __device__ __forceinline__ void element_interval(const PrimF& P, float cx, float cy, float cz, float R, float eps,
                                                  float& lo, float& hi) {
     const float v = primf_world_common(P, cx, cy, cz);
-    const float r = fmaf(P.lip, R, eps + 1e-6f * fabsf(v));
+    const float r = fmaf(P.lip, R, eps + P.err + 1e-6f * fabsf(v));
     lo = v - r;
     hi = v + r;
 }
@@ -93,7 +102,7 @@ struct Elem {
 // cache lines each and the records of 4096 elements did not stay in L1.
 struct __align__(16) Ball {
     float x, y, z, r;
-    float k, off, has, pad;  // value scale and offset; has != 0: the ball holds
+    float k, off, has, err;  // value scale and offset; has != 0: the ball holds; PrimF.err
 };
 
 // The enclosure from the bounding ball: no evaluation of the primitive, a few loads -- looser by up to
@@ -102,7 +111,7 @@ __device__ __forceinline__ void element_interval_ball(const Ball& P, float cx, f
                                                       float& lo, float& hi) {
     const float dx = cx - P.x, dy = cy - P.y, dz = cz - P.z;
     const float d = sqrt_rn(fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
-    const float m = eps + 1e-6f * (P.k * (d + R + P.r) + fabsf(P.off));
+    const float m = eps + P.err + 1e-6f * (P.k * (d + R + P.r) + fabsf(P.off));
     lo = fmaf(P.k, d - R - P.r, -P.off) - m;
     hi = fmaf(P.k, d + R + P.r, -P.off) + m;
 }
@@ -186,6 +195,7 @@ __device__ int warp_walk(const uint32_t* __restrict__ in, int n_in, const FbInsn
                          uint32_t* __restrict__ out, int cap) {
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
+    R = bounds_radius(cx, cy, cz, R);
     float alo = 0.f, ahi = 0.f;
     int n = 0;
     int i = 0;
@@ -273,6 +283,7 @@ __device__ int warp_walk_ball(int n_in, const FbInsn* __restrict__ chain, const 
                               uint32_t* __restrict__ out, int cap, float* klo_of, float* khi_of, int n_of) {
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
+    R = bounds_radius(cx, cy, cz, R);
     float alo = 0.f, ahi = 0.f;
     int n = 0;
     int i = 0;
@@ -407,6 +418,7 @@ static __device__ __noinline__ int warp_walk_once(const uint32_t* in, int n_in, 
                                                   float R, float eps, uint32_t* ent, float* blo, float* bhi, int cap) {
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
+    R = bounds_radius(cx, cy, cz, R);
     float alo = 0.f, ahi = 0.f, agg = 0.f;
     int n = 0, n0 = 0, run = -1;  // entries; where the open run's start; its operation (-1: none)
     auto finish = [&]() {

@@ -172,7 +172,7 @@ __device__ void prepare_prim(const FbPrim* __restrict__ prims, int i, PrimF* __r
     F.type = P.type;
     F.s = (float)P.s;
     F.off = (float)P.off;
-    F.ball = F.ball_k = F.pad = 0.f;
+    F.ball = F.ball_k = 0.f;
     bool ident = true;
     for (int r = 0; r < 3; ++r)
         for (int c = 0; c < 3; ++c) ident &= P.A[r * 4 + c] == (r == c ? 1.0 : 0.0);
@@ -235,6 +235,13 @@ __device__ void prepare_prim(const FbPrim* __restrict__ prims, int i, PrimF* __r
         for (int j = 0; j < 12; ++j) F.p[j] = (float)p[j];
     }
     F.lip = (float)(fabs(P.s) * sqrt(row) * canon * (1.0 + 1e-6));
+    // Rounding of float32 values (u = 2^-24) at two points, parameters rounded as well: each coordinate
+    // A x + t within 4 u of its terms' magnitudes, the canonical forms within 12 u of |q| and the sizes
+    // they subtract, so 32 u of |A| |x| (bounds_radius), |t| and the sizes for both points, 8 u of off.
+    double mag = 0.0;
+    for (int r = 0; r < 3; ++r) mag += fabs(P.A[4 * r + 3]);
+    for (int j = 0; j < 10; ++j) mag += fabs(p[j]);
+    F.err = (float)((32.0 * fabs(P.s) * canon * mag + 8.0 * fabs(P.off)) * (5.9604644775390625e-8 * (1.0 + 1e-6)));
     // Bounding ball, for kinds whose canonical value is the exact Euclidean distance, of the
     // canonical solid (centre cc, radius rc).  When the frame map is a similarity (A_lin^T A_lin =
     // a^2 I) and s > 0, value(x) = s a d_world(x) - off with d_world the exact distance to the world
@@ -268,14 +275,14 @@ __device__ void prepare_prim(const FbPrim* __restrict__ prims, int i, PrimF* __r
             cw[c] = v / a2;
         }
         const double rw = rc / a;
-        const double mag = fmax(fabs(cw[0]), fmax(fabs(cw[1]), fabs(cw[2])));
+        const double far = fmax(fabs(cw[0]), fmax(fabs(cw[1]), fabs(cw[2])));
         F.ball = 1.f;
         F.ball_k = (float)(P.s * a);
         for (int c = 0; c < 3; ++c) F.p[8 + c] = (float)cw[c];
-        F.p[11] = (float)(rw * (1.0 + 1e-6) + 1e-6 * mag);  // covers rounding the centre to float32
+        F.p[11] = (float)(rw * (1.0 + 1e-6) + 1e-6 * far);  // covers rounding the centre to float32
     }
     out[i] = F;
-    if (balls) balls[i] = Ball{F.p[8], F.p[9], F.p[10], F.p[11], F.ball_k, F.off, F.ball, 0.f};
+    if (balls) balls[i] = Ball{F.p[8], F.p[9], F.p[10], F.p[11], F.ball_k, F.off, F.ball, F.err};
 }
 
 __global__ void k_prepare_prims(const FbPrim* __restrict__ prims, int n, PrimF* __restrict__ out,
@@ -307,6 +314,7 @@ __global__ void k_full_list(uint32_t* __restrict__ list, int n) {
 __device__ int seq_walk(const uint32_t* __restrict__ in, int n_in, const FbInsn* __restrict__ chain,
                         const PrimF* __restrict__ primf, float cx, float cy, float cz, float R, float eps,
                         uint32_t* __restrict__ out, int cap) {
+    R = bounds_radius(cx, cy, cz, R);
     float alo = 0.f, ahi = 0.f;
     int n = 0;
     int i = 0;
@@ -599,6 +607,7 @@ __device__ __noinline__ double subset_eval_d(const uint32_t* ent, Bits96 K, uint
 __device__ __forceinline__ void subset_walk(const uint32_t* ent, int m, const FbInsn* __restrict__ chain,
                                             const PrimF* __restrict__ primf, float cx, float cy, float cz, float R,
                                             float eps, Bits96& K, uint32_t& head) {
+    R = bounds_radius(cx, cy, cz, R);
     float alo = 0.f, ahi = 0.f, agg = 0.f;
     K.clear();
     head = 0u;

@@ -65,7 +65,7 @@ struct Accel {  // a built field's culling lists (nullptr pool: walk the whole c
     int blk_all;
     double x0, y0, z0, pitch;
     int nx, ny, nz, B, S, nsx, nsy, nsz, nbx, nby, nbz;
-    float eps;  // the bounds' float32 slack near the grid, at least the build's own
+    float eps;  // slack of the bounds beside the primitives' own rounding, from the grid's coordinates
 };
 
 // The list a point at (x, y, z) walks on its own: its block's where the classification kept one, its
@@ -1079,7 +1079,7 @@ int fb_query_points_device(const void* d_primf, const FbInsn* d_chain, int32_t n
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const PrimF* primf = static_cast<const PrimF*>(d_primf);
     if (A.pool) {
-        // 16 float32 ulps of the largest coordinate a superblock's ball reaches: the build's slack
+        // 16 float32 ulps of the largest coordinate a superblock's ball reaches: the default guard's slack
         float far = 0.f;
         const double reach = (A.S * A.B + 1) * A.pitch;
         const double lo[3] = {A.x0, A.y0, A.z0};
