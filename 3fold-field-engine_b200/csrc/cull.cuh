@@ -275,7 +275,8 @@ __device__ int warp_walk(const uint32_t* __restrict__ in, int n_in, const FbInsn
 // element provably loses, so the run's result is the candidates' result); the exact bounds of the
 // candidates alone give the run's decision, and they are compacted in place with it.  Few warps walk
 // here (a region each), so a warp keeps the loads of kBallChunks chunks in flight.  4096 regions of 4096
-// elements: 541 -> XX us with the balls in a table of their own.
+// elements: 541 -> 318 us with the balls in a table of their own.  Returns the kept count, or cap + 1 where
+// the list does not fit.
 constexpr int kBallChunks = 4;
 
 __device__ int warp_walk_ball(int n_in, const FbInsn* __restrict__ chain, const PrimF* __restrict__ primf,
@@ -353,10 +354,8 @@ __device__ int warp_walk_ball(int n_in, const FbInsn* __restrict__ chain, const 
             }
         }
         const int nc = n - n0;  // candidates at out[n0, n)
-        if (n > cap) {          // overflowed: the region falls back to its parent's list anyway
-            i = j;
-            continue;
-        }
+        // overflowed: the bounds after this run are not known, so nothing later may be decided by them
+        if (n > cap) return cap + 1;
         __syncwarp();  // the candidates are read by other lanes
         float agg2 = op == CH_UNION ? 3.0e38f : -3.0e38f;
         for (int b = 0; b < nc; b += 32) {
