@@ -123,7 +123,7 @@ __device__ __forceinline__ Elem load_elem(const uint32_t* __restrict__ in, int e
     E.ent = in ? in[e] : (uint32_t)e << 2;  // a null list is the whole chain in order
     const FbInsn I = chain[E.ent >> 2];
     E.op = effective_op(E.ent, I.op);
-    E.k = (float)I.k;
+    E.k = E.op == CH_OFFSET ? (float)I.k : fmaxf((float)I.k, 0.f);  // a negative blend width is a hard boolean
     E.lo = E.hi = 0.f;
     if (with_bounds && E.op != CH_OFFSET) {
         float lo, hi;
