@@ -334,6 +334,7 @@ __device__ __forceinline__ double write_triangle(int64_t at, const int64_t* vid,
 // pass hands out triangles, not cubes, to the threads.  27 balls on 256 x 256 x 250: count 301 -> 61 us,
 // emit 414 -> 60 us.
 constexpr int kMcItems = 1024;  // triangles (or undecided cubes) handed out at a time
+constexpr size_t kMcStatic = kMcItems * sizeof(uint2) + 1024;  // k_mc's static shared memory is below it
 static_assert(kMcItems >= kMcThreads * kMaxTableTris, "one round of cubes must fit");
 
 template <int kB, bool kEmit>
@@ -658,7 +659,8 @@ int mc_launch_block(const McField& F, const int32_t* d_active, int64_t n_active,
               int32_t* err, unsigned long long* totals, cudaStream_t st) {
     if (n_active == 0) return FB_OK;
     const size_t smem = mc_smem(F.B);
-    if (smem > 48 * 1024) FB_CUDA(cudaFuncSetAttribute(k_mc<kB, kEmit>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // the limit without the opt-in is on the static and the dynamic part together
+    if (smem + kMcStatic > 48 * 1024) FB_CUDA(cudaFuncSetAttribute(k_mc<kB, kEmit>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int grid = (int)std::min<int64_t>(n_active, (int64_t)fb_sm_count() * 8);
     k_mc<kB, kEmit><<<grid, kMcThreads, smem, st>>>(F, d_active, n_active, bits, wpre, vcount, tcount, verts, vkey,
                                                    faces, vol_part, err, totals);
