@@ -285,6 +285,7 @@ __device__ __forceinline__ int64_t vertex_id(const McBlock& N, int B, const int*
         const int u = a == 0 ? 1 : 0, v = a == 2 ? 1 : 2;
         sl = 3 * B * B * B + a * B * B + (p[u] - (o[u] - 1) * B) * B + p[v] - (o[v] - 1) * B;
     }
+    if (voff[s] == voff[s + 1]) return -1;  // a block without a crossing has no bit words
     const int64_t at = (int64_t)s * W + (sl >> 5);
     const uint32_t word = bits[at];
     if (!((word >> (sl & 31)) & 1u)) return -1;
@@ -312,9 +313,11 @@ __device__ __forceinline__ int block_scan(int v, int* s_warp, int* total) {
     return before;
 }
 
-// Triangle (f0, f1, f2) with positions q0, q1, q2: its signed volume term v0 . (v1 x v2).
-__device__ __forceinline__ double write_triangle(int64_t at, const int64_t* vid, const float (*q)[3],
+// Triangle (f0, f1, f2) with positions q0, q1, q2, before the end of its block's range: its signed volume
+// term v0 . (v1 x v2).  A field that changed since the count pass may have more triangles than were counted.
+__device__ __forceinline__ double write_triangle(int64_t at, int64_t end, const int64_t* vid, const float (*q)[3],
                                                  int32_t* __restrict__ faces, int32_t* __restrict__ err) {
+    if (at >= end) return 0.0;
     if (vid[0] < 0 || vid[1] < 0 || vid[2] < 0) atomicAdd(err, 1);
     faces[3 * at] = (int32_t)vid[0];
     faces[3 * at + 1] = (int32_t)vid[1];
@@ -493,7 +496,7 @@ __global__ void __launch_bounds__(kMcThreads) k_mc(McField F, const int32_t* __r
         };
         auto flush = [&]() {  // the threads take the handed-out items
             __syncthreads();
-            const int64_t base = tcount[sa];
+            const int64_t base = tcount[sa], end = tcount[sa + 1];
             for (int i = threadIdx.x; i < items; i += kMcThreads) {
                 const uint2 it = s_item[i];
                 const int ci = it.x & 0xffff, t = it.x >> 16;
@@ -507,7 +510,7 @@ __global__ void __launch_bounds__(kMcThreads) k_mc(McField F, const int32_t* __r
                     int64_t vid[3];
                     float q[3][3];
                     for (int k = 0; k < 3; ++k) edge_point(m, d_cube_table.edge[in][3 * t + k], vid[k], q[k]);
-                    vol += write_triangle(base + it.y, vid, q, faces, err);
+                    vol += write_triangle(base + it.y, end, vid, q, faces, err);
                     continue;
                 }
                 double g[8];
@@ -541,7 +544,7 @@ __global__ void __launch_bounds__(kMcThreads) k_mc(McField F, const int32_t* __r
                         edge_point(m, el[c], vid[0], q[0]);
                         edge_point(m, el[(c + i2 + 1) % len], vid[1], q[1]);
                         edge_point(m, el[(c + i2) % len], vid[2], q[2]);
-                        vol += write_triangle(to++, vid, q, faces, err);
+                        vol += write_triangle(to++, end, vid, q, faces, err);
                     }
                 }
             }
@@ -609,6 +612,7 @@ __global__ void __launch_bounds__(kMcThreads) k_mc(McField F, const int32_t* __r
             }
         } else {
             flush();
+            if (threadIdx.x == 0 && run != tcount[sa + 1] - tcount[sa]) atomicAdd(err, 1);
             for (int d = 16; d > 0; d >>= 1) vol += __shfl_xor_sync(0xffffffffu, vol, d);
             if (lane == 0) s_vol[warp] = vol;
             __syncthreads();
@@ -842,7 +846,8 @@ int fb_mc_count_device(const int32_t* d_kind, const int32_t* d_active, int64_t n
 // (int32 vertex ids, d_tcount[n_active] of them, outward normals) and the enclosed volume
 // sum(v0 . (v1 x v2)) / 6 in float64 (d_volume[0]; d_vol_part: n_active float64 scratch), summed in a
 // fixed order.  The arguments of pass 1 unchanged.  d_err[0] counts triangle corners without a
-// vertex (0 unless the field changed in between).
+// vertex and blocks with another number of triangles than pass 1 counted (0 unless the field changed in
+// between; such corners are -1, and nothing is written beyond the counted totals).
 int fb_mc_emit_device(const int32_t* d_kind, const int32_t* d_active, int64_t n_active, const float* d_tiles,
                       int64_t nx, int64_t ny, int64_t nz, int32_t block, double ox, double oy, double oz, double pitch,
                       double level, float big, const int32_t* d_slot, const uint32_t* d_bits, const int32_t* d_wpre,

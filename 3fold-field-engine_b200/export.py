@@ -102,7 +102,7 @@ def _mesh(kind, active, n, tiles, nx, ny, nz, block, origin, pitch, level, keys,
                "marching cubes (emit)")
     vol, e = float(volume.cpu()[0]), int(err.cpu()[0])
     if e:
-        raise RuntimeError(f"marching cubes: {e} triangle corners without a vertex")
+        raise RuntimeError(f"marching cubes: {e} triangle corners or blocks at odds with the count pass")
     if to_host:
         return Mesh(verts.cpu().numpy(), faces.cpu().numpy(), vol, vkey.cpu().numpy() if keys else None)
     return Mesh(verts, faces, vol, vkey)

@@ -361,7 +361,8 @@ int fb_mc_count_device(const int32_t* d_kind, const int32_t* d_active, int64_t n
 /* d_verts: 3 float32 per vertex (world coordinates); d_vkey (optional): per vertex
  * (linear index of the edge's lower end) * 3 + axis; d_faces: 3 int32 per triangle, outward normals;
  * d_volume[0]: sum(v0 . (v1 x v2)) / 6 (d_vol_part: n_active float64 scratch); d_err[0]: triangle
- * corners without a vertex (0 unless the field changed between the passes). */
+ * corners without a vertex (-1 in d_faces) and blocks with another number of triangles than were counted
+ * (0 unless the field changed between the passes; nothing is written beyond the counted totals). */
 int fb_mc_emit_device(const int32_t* d_kind, const int32_t* d_active, int64_t n_active, const float* d_tiles,
                       int64_t nx, int64_t ny, int64_t nz, int32_t block, double ox, double oy, double oz, double pitch,
                       double level, float big, const int32_t* d_slot, const uint32_t* d_bits, const int32_t* d_wpre,
