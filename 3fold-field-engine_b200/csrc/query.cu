@@ -645,14 +645,22 @@ __global__ void __launch_bounds__(32 * kQueryWarps, 5) k_query_sorted(const Prim
     }
 }
 
-// Up to kWarpPoints points go a warp per point, without scratch; more are sorted first.  Values and
+// Up to warp_points points go a warp per point, without scratch; more are sorted first.  Values and
 // gradients, a warp per point against sorted points: 32 000 points 94 / 93 us (64^3 field of 54
 // elements), 143 / 204 us (256^3, 576) and 151 / 249 us (300^3, 787); 64 000 points 179 / 84, 260 / 193
 // and 265 / 240 us: the lines cross between 32 000 and 64 000.
+// Values alone leave a warp 31 idle lanes, so their lines cross sooner, and the later the more superblocks
+// the points are spread over (a sorted warp then culls for several of them): 64^3 field (64 superblocks)
+// 46 / 52 us at 16 384 points and 66 / 50 at 24 576; 256^3 (512) 81 / 93 at 20 480 and 120 / 89 at 32 768;
+// 300^3 (1000) 93 / 99 and 120 / 97 at 24 576 and 32 768; 512^3 (4096) 136 / 140 at 40 960.
 constexpr int64_t kWarpPoints = 40960;
 
+int64_t warp_points(int64_t nsuper, bool grad) {
+    return grad ? kWarpPoints : std::min<int64_t>(kWarpPoints, 19000 + 6 * nsuper);
+}
+
 struct SortedPlan {
-    int64_t nbins, ntiles;
+    int64_t nsuper, nbins, ntiles;
     int C;  // sorting cells per superblock edge
     int64_t keys, order, count, tiles, total;
 };
@@ -669,6 +677,7 @@ bool sorted_plan(const int32_t* dims, int64_t n, SortedPlan& p) {
     const int64_t ns = ((nbx + S - 1) / S) * ((nby + S - 1) / S) * ((nbz + S - 1) / S);
     for (p.C = 4; p.C > 1 && ns * p.C * p.C * p.C > kMaxBins; p.C /= 2) {
     }
+    p.nsuper = ns;
     p.nbins = ns * p.C * p.C * p.C;
     if (ns < 1 || p.nbins > kMaxBins) return false;
     auto al = [](int64_t b) { return (b + 255) / 256 * 256; };
@@ -1040,10 +1049,9 @@ int fb_query_prepare(const FbPrim* d_prims, int32_t n_prims, void* d_primf, void
 // Scratch bytes of the sorted query path for n points on an accelerated grid of dims (nx, ny, nz, B); 0
 // or -1: the query takes a path without scratch (few points; a grid that is not sorted).
 int64_t fb_query_scratch_bytes(const int32_t* accel_dims, int64_t n, int32_t with_grad) noexcept {
-    (void)with_grad;
     SortedPlan P;
     if (!accel_dims || n < 0 || !sorted_plan(accel_dims, n, P)) return -1;
-    return n <= kWarpPoints ? 0 : P.total;
+    return n <= warp_points(P.nsuper, with_grad != 0) ? 0 : P.total;
 }
 
 int fb_query_points_device(const void* d_primf, const FbInsn* d_chain, int32_t n_chain, int32_t mode,
@@ -1088,7 +1096,7 @@ int fb_query_points_device(const void* d_primf, const FbInsn* d_chain, int32_t n
             far = std::max(far, (float)std::max(std::fabs(lo[a] - reach), std::fabs(lo[a] + ext[a] * A.pitch + reach)));
         A.eps = 16.f * (std::nextafter(far, 3.4e38f) - far);
         SortedPlan P;
-        if (d_scratch && n > kWarpPoints && sorted_plan(accel_dims, n, P)) {
+        if (d_scratch && sorted_plan(accel_dims, n, P) && n > warp_points(P.nsuper, d_grad != nullptr)) {
             if (scratch_len < P.total) return FB_INVALID;
             char* b = static_cast<char*>(d_scratch);
             int2* keys = reinterpret_cast<int2*>(b + P.keys);
