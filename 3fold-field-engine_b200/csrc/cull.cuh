@@ -407,11 +407,94 @@ __device__ int warp_walk_ball(int n_in, const FbInsn* __restrict__ chain, const 
     return n;
 }
 
+// x -> min(max(x + c, a), b) with a <= b: what a boolean does to a bound of the accumulator.  Closed under
+// composition, so the bounds before each element of a stretch come from one scan over the warp.
+struct Clamp {
+    float c, a, b;
+    __device__ __forceinline__ float operator()(float x) const { return fminf(fmaxf(x + c, a), b); }
+};
+
+// g applied to f's result.
+__device__ __forceinline__ Clamp then(const Clamp& f, const Clamp& g) { return Clamp{f.c + g.c, g(f.a), g(f.b)}; }
+
+__device__ __forceinline__ Clamp shfl_up(const Clamp& f, int o) {
+    return Clamp{__shfl_up_sync(0xffffffffu, f.c, o), __shfl_up_sync(0xffffffffu, f.a, o),
+                 __shfl_up_sync(0xffffffffu, f.b, o)};
+}
+
+// Booleans that form no run of kRunLeast go by the stretch from kStretch of them on: one at a time a step is a
+// chain of shuffles and comparisons of about 40 instructions, a stretch of up to 32 takes about 250.
+constexpr int kRunLeast = 9, kStretch = 5;
+
+struct Walk {  // accumulator's bounds, kept entries, elements taken (0: no stretch here)
+    float alo, ahi;
+    int n, taken;
+};
+
+// The warp's elements E from `pos` on in one stretch, up to where a run of kRunLeast starts, or one that
+// reaches the end of a full 32, or an offset or set: every element decides by interval_step on the bounds
+// before it.
+__device__ __forceinline__ Walk walk_stretch(uint32_t entry, int op, float width, float elo, float ehi, int cnt,
+                                                 int pos, float alo, float ahi, int n, uint32_t* ent, int cap) {
+    const int lane = threadIdx.x & 31;
+    const bool hard = runnable(op, width);
+    const int next = __shfl_down_sync(0xffffffffu, hard ? op : -1, 1);
+    const unsigned pairs = __ballot_sync(0xffffffffu, lane < 31 && hard && next == op);
+    const unsigned hards = __ballot_sync(0xffffffffu, hard);
+    unsigned stops = pairs & pairs >> 1;
+    stops &= stops >> 2;
+    stops &= stops >> 4;
+    static_assert(kRunLeast == 9, "eight pairs in a row");
+    if (cnt == 32 && hards >> 31) stops |= 1u << (31 - __clz(~(pairs << 1)));
+    stops |= __ballot_sync(0xffffffffu, lane >= cnt || op == CH_OFFSET || op == CH_SET || op == CH_SETNEG);
+    stops >>= pos;
+    const int length = stops ? __ffs(stops) - 1 : 32 - pos;
+    if (length < kStretch) return Walk{alo, ahi, n, 0};
+    const bool mine = lane >= pos && lane < pos + length;
+    const float q = 0.2500025f * width;  // the blend's deepest, a little widened for the sums' rounding
+    constexpr float kInf = 3.0e38f;
+    Clamp lo{0.f, -kInf, kInf}, hi{0.f, -kInf, kInf};
+    if (mine && op == CH_UNION) {
+        lo = Clamp{-q, -kInf, elo - q};
+        hi.b = ehi;
+    } else if (mine) {
+        lo.a = elo;
+        hi = Clamp{q, ehi + q, kInf};
+    }
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const Clamp a = shfl_up(lo, o), b = shfl_up(hi, o);
+        if (lane >= o) {
+            lo = then(a, lo);
+            hi = then(b, hi);
+        }
+    }
+    const Clamp lo_before = shfl_up(lo, 1), hi_before = shfl_up(hi, 1);
+    float l = lane > pos ? lo_before(alo) : alo, h = lane > pos ? hi_before(ahi) : ahi;
+    int act = 0;
+    const bool neg = op == CH_SUBTRACT;  // back to the primitive's own bounds
+    if (mine) act = interval_step(op, width, neg ? -ehi : elo, neg ? -elo : ehi, l, h);
+    unsigned kept = __ballot_sync(0xffffffffu, act != 0);
+    const unsigned resets = __ballot_sync(0xffffffffu, act >= 2);
+    if (resets) {  // what lies before the last reset is dominated
+        n = 0;
+        kept &= ~0u << (31 - __clz(resets));
+    }
+    if (n + __popc(kept) <= cap && ((kept >> lane) & 1u))
+        ent[n + __popc(kept & ((1u << lane) - 1u))] = act >= 2 ? (entry & ~3u) | (unsigned)(act - 1) : entry;
+    __syncwarp();
+    return Walk{__shfl_sync(0xffffffffu, lo(alo), pos + length - 1), __shfl_sync(0xffffffffu, hi(ahi), pos + length - 1),
+                n + __popc(kept), length};
+}
+
 // The same walk with every element bounded once, for lists that fit shared memory: candidates of a run
 // (elements not beaten by the bound so far) are kept with their bounds in `ent`, `blo`, `bhi` (shared,
 // `cap` each) and compacted in place when the run ends and its bound is final.  One copy of the code:
-// inlined at each call it missed the instruction cache.  Returns the kept count, or cap + 1 where the
+// inlined at each call it missed the instruction cache.  kStretches: also by the stretch, for chains that
+// are no few long runs (in the usual chains' walk it cost 10^6 queries on a 256^3 field 3 %, through the
+// registers that a caller spills around it).  Returns the kept count, or cap + 1 where the
 // candidates did not fit; every lane of the warp calls it, and the list is readable after it.
+template <bool kStretches>
 static __device__ __noinline__ int warp_walk_once(const uint32_t* in, int n_in, const FbInsn* __restrict__ chain,
                                                   const PrimF* __restrict__ primf, float cx, float cy, float cz,
                                                   float R, float eps, uint32_t* ent, float* blo, float* bhi, int cap) {
@@ -465,6 +548,20 @@ static __device__ __noinline__ int warp_walk_once(const uint32_t* in, int n_in, 
             const bool same = hard && E.op == op && lane >= pos && lane < cnt;
             const unsigned run_mask = __ballot_sync(0xffffffffu, same);
             if (run >= 0 && (run != op || !((run_mask >> pos) & 1u))) finish();
+            const unsigned gap = ~(run_mask >> pos);
+            const int end = gap ? min(pos + __ffs(gap) - 1, cnt) : cnt;  // of the run here, if any
+            if (kStretches && run < 0 && end - pos < kRunLeast && cnt - pos >= kStretch && op >= CH_UNION &&
+                op <= CH_SUBTRACT) {
+                const Walk w = walk_stretch(E.ent, E.op, E.k, E.lo, E.hi, cnt, pos, alo, ahi, n, ent, cap);
+                if (w.n > cap) return cap + 1;
+                if (w.taken) {
+                    alo = w.alo;
+                    ahi = w.ahi;
+                    n = w.n;
+                    pos += w.taken;
+                    continue;
+                }
+            }
             if (!((run_mask >> pos) & 1u)) {  // offsets, sets, smooth booleans: one at a time
                 const float lo = __shfl_sync(0xffffffffu, E.lo, pos), hi = __shfl_sync(0xffffffffu, E.hi, pos);
                 const float k = __shfl_sync(0xffffffffu, E.k, pos);
@@ -485,8 +582,6 @@ static __device__ __noinline__ int warp_walk_once(const uint32_t* in, int n_in, 
                 n0 = n;
                 agg = op == CH_UNION ? 3.0e38f : -3.0e38f;
             }
-            const unsigned gap = ~(run_mask >> pos);
-            const int end = gap ? min(pos + __ffs(gap) - 1, cnt) : cnt;
             const bool mine = lane >= pos && lane < end;
             float a = mine ? (op == CH_UNION ? E.hi : E.lo) : agg;
             for (int o = 16; o > 0; o >>= 1) {

@@ -407,7 +407,7 @@ __device__ void cull_region(const Geo& G, const FbInsn* __restrict__ chain, cons
         n = warp_walk_ball(plen, chain, primf, balls, cx, cy, cz, R, G.eps, dst, cap, walked.lo, walked.hi, kWalked);
     } else {
         const int lane = threadIdx.x & 31;
-        n = warp_walk_once(pool + poff, plen, chain, primf, cx, cy, cz, R, G.eps, walked.ent, walked.lo, walked.hi, kWalked);
+        n = warp_walk_once<false>(pool + poff, plen, chain, primf, cx, cy, cz, R, G.eps, walked.ent, walked.lo, walked.hi, kWalked);
         if (n > kWalked) {
             n = warp_walk(pool + poff, plen, chain, primf, cx, cy, cz, R, G.eps, dst, cap);
         } else {
@@ -785,7 +785,7 @@ __device__ __forceinline__ void classify_block(const Geo& G, const FbPrim* __res
     } else if (bricks && any) {
         ent = sub.ent;
         const float fb = (float)B;
-        m = warp_walk_once(plist, plen, chain, primf, G.fx0 + ((sx * S + wi) * fb + fb) * G.fpitch,
+        m = warp_walk_once<false>(plist, plen, chain, primf, G.fx0 + ((sx * S + wi) * fb + fb) * G.fpitch,
                            G.fy0 + ((sy * S + wj) * fb + 2.f * fb) * G.fpitch,
                            G.fz0 + ((sz * S + wk) * fb + 2.f * fb) * G.fpitch, 3.0001f * fb * G.fpitch, G.eps, sub.ent,
                            sub.lo, sub.hi, kSubset);

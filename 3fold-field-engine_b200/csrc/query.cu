@@ -6,7 +6,8 @@
 //   points) and k_query_sorted (many) cull the superblock's list once more to the points at hand --
 //   exact, by the same strict-domination argument as the build -- instead of walking the whole chain.
 //   k_gradient_points: central differences with step h along each axis, the six offset points
-//   formed in float64 and rounded to float32 as the reference does.
+//   formed in float64 and rounded to float32 as the reference does.  By sizes (by_items, short_chain)
+//   the offset points of an accelerated query go as points of their own, and short chains whole.
 // Per-block pitch fields (src/field_engine/faltkarna_v1_multires.py:84-104, :384-459):
 //   k_multires_tiles fills each active brick's (B*2^l + 1)^3 lattice at pitch h/2^l;
 //   k_multires_value answers avstand (trilinear at the brick's own pitch, +-margin outside active
@@ -16,6 +17,7 @@
 #include "prims.cuh"
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 namespace {
 
@@ -166,6 +168,19 @@ __device__ __forceinline__ Variants load_variants(const float* __restrict__ pts,
     return V;
 }
 
+// What a query's item is: point i itself with its variants, or (kItems) one evaluation, variant i % 7 of point
+// i / 7.
+template <bool kItems>
+__device__ __forceinline__ Variants load_query(const float* __restrict__ pts, int64_t i, double h) {
+    if (!kItems) return load_variants(pts, i, h);
+    const int64_t at = i / 7;
+    const int v = (int)(i - 7 * at);
+    Variants V = load_variants(pts, at, h);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) V.p[a] = V.at(v, a);
+    return V;
+}
+
 // The superblock nearest a point, the bit mask of the point's variants inside that superblock's ball
 // (0 when the point itself is not), and the point's sorting cell: C^3 cells per superblock.
 struct Place {
@@ -261,11 +276,12 @@ struct Survivors {
 
 // `list` (nullptr: the whole chain) culled to the ball (c, R) of points whose coordinates reach `reach`;
 // left as it is where the survivors do not fit.
+template <bool kStretches>
 __device__ __forceinline__ void cull_to(const uint32_t*& list, int& len, const FbInsn* __restrict__ chain,
                                         const PrimF* __restrict__ primf, const float* c, float R, float reach,
                                         float eps, Survivors& out) {
     const float e = fmaxf(eps, 16.f * 1.2e-7f * reach);  // 16 float32 ulps
-    const int m = warp_walk_once(list, len, chain, primf, c[0], c[1], c[2], R, e, out.ent, out.lo, out.hi, kQueryCap);
+    const int m = warp_walk_once<kStretches>(list, len, chain, primf, c[0], c[1], c[2], R, e, out.ent, out.lo, out.hi, kQueryCap);
     if (m <= kQueryCap) {
         list = out.ent;
         len = m;
@@ -382,7 +398,7 @@ __device__ __forceinline__ void write_point(int64_t i, const float* v, float inv
 // around the point's variants (a handful of elements remain), and lane v evaluates variant v.  Bound by
 // the latency of the culling's loads and reductions: 1000 points of a 64^3 field in 9 us, against 55 us
 // in eight kernels when all 7000 evaluations were sorted by the list that each walked.
-template <int NV>
+template <int NV, bool kStretches, bool kItems = false>
 __global__ void __launch_bounds__(32 * kQueryWarps) k_query_warp(const PrimF* __restrict__ primf,
                                                                  const FbInsn* __restrict__ chain, int n_chain,
                                                                  Accel A, const float* __restrict__ pts, int64_t n,
@@ -393,7 +409,7 @@ __global__ void __launch_bounds__(32 * kQueryWarps) k_query_warp(const PrimF* __
     const float inv = (float)(2.0 * h);
     const int64_t nwarps = (int64_t)gridDim.x * kQueryWarps;
     for (int64_t i = blockIdx.x * (int64_t)kQueryWarps + warp; i < n; i += nwarps) {
-        const Variants V = load_variants(pts, i, h);
+        const Variants V = load_query<kItems>(pts, i, h);
         const Place P = place_of<NV>(A, V, 1);
         const uint32_t* list = A.pool + A.sb_off[P.s];
         int len = A.sb_len[P.s];
@@ -414,7 +430,7 @@ __global__ void __launch_bounds__(32 * kQueryWarps) k_query_warp(const PrimF* __
                 list = nullptr;
                 len = n_chain;
             }
-            cull_to(list, len, chain, primf, V.p, R, ball ? 0.f : reach, A.eps, s_list[warp]);
+            cull_to<kStretches>(list, len, chain, primf, V.p, R, ball ? 0.f : reach, A.eps, s_list[warp]);
         }
         __syncwarp();
         float r = 0.f;
@@ -431,11 +447,20 @@ __global__ void __launch_bounds__(32 * kQueryWarps) k_query_warp(const PrimF* __
     }
 }
 
-// A point's sorting cell (outside the grid: the nearest one) and its rank among the cell's points.
-__global__ void k_query_keys(Accel A, const float* __restrict__ pts, int64_t n, int C, int2* __restrict__ keys,
-                             int32_t* __restrict__ count) {
+// A point's sorting cell and its rank among the cell's points; outside the grid the nearest cell, or (outside >= 0)
+// that key for all that lie more than half a superblock's edge beyond it.
+template <bool kItems>
+__global__ void k_query_keys(Accel A, const float* __restrict__ pts, int64_t n, double h, int C, int outside,
+                             int2* __restrict__ keys, int32_t* __restrict__ count) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t key = place_of<1>(A, load_variants(pts, i, 0.0), C).cell;
+        const Variants V = load_query<kItems>(pts, i, h);
+        int32_t key = place_of<1>(A, V, C).cell;
+        if (outside >= 0) {
+            const double inv = 1.0 / ((double)A.S * A.B * A.pitch);
+            const double x = (V.p[0] - A.x0) * inv, y = (V.p[1] - A.y0) * inv, z = (V.p[2] - A.z0) * inv;
+            if (!(x >= -0.5 && y >= -0.5 && z >= -0.5 && x <= A.nsx + 0.5 && y <= A.nsy + 0.5 && z <= A.nsz + 0.5))
+                key = outside;
+        }
         keys[i] = make_int2(key, atomicAdd(&count[key], 1));
     }
 }
@@ -521,21 +546,153 @@ __global__ void k_query_scatter(const int2* __restrict__ keys, int64_t n, const 
     }
 }
 
+// Values alone: lists up to this are walked by the lane itself (a block's own list mostly), longer ones culled for
+// the group: one evaluation a point does not repay the cull of a short list.  10^6 values with 12, 24 and 48
+// here (us): 256^3 field of 576 elements 196, 179, 196 (no lane by itself 243), 300 blends 355, 298, 282 (476), 512^3
+// of 3000 419, 384, 347 (405).
+constexpr int kDirectList = 24;
+
+// Centre and radius of the ball around a warp's variants: a lane's are those of `mask`.
+template <int NV>
+__device__ __forceinline__ float ball_of(const Variants& V, unsigned mask, float* c) {
+    float d = 0.f;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const unsigned fixed = mask & ~(6u << (2 * a));  // variants at the point's own coordinate a
+        float lo = fixed ? V.p[a] : 3.0e38f, hi = fixed ? V.p[a] : -3.0e38f;
+        if (NV > 1) {
+            if (mask & (2u << (2 * a))) { lo = fminf(lo, V.plus[a]); hi = fmaxf(hi, V.plus[a]); }
+            if (mask & (4u << (2 * a))) { lo = fminf(lo, V.minus[a]); hi = fmaxf(hi, V.minus[a]); }
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+            hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+        }
+        c[a] = 0.5f * lo + 0.5f * hi;
+        const float e = fmaxf(hi - c[a], c[a] - lo);
+        d = fmaf(e, e, d);
+    }
+    return sqrtf(d) * 1.00001f;
+}
+
+// What the groups in the superblocks' balls leave of a warp's points (lane: item i, nearest superblock s):
+// `beyond` the variants outside the grid, `left` the others; their values in vals[NV * lane + variant].
+// Rare, and out of line: the groups' loop keeps its registers.
+// Variants beyond the grid go by the superblock nearest to their point, the whole chain culled to the ball
+// around the group.  Groups of which that keeps too much (scattered points) are put together: many points
+// evaluate the whole chain side by side, few go one after another, each culled to a ball of its own as in
+// k_query_warp.  The lines between them are measured costs in issue slots: about 100 for one evaluation of an
+// element by the warp, 45 for one element's part in a cull (its record is gathered from L2).
+// The rest are handed out to the lanes, each on its own list.
+template <int NV, bool kStretches, bool kItems>
+static __device__ __noinline__ void eval_rest(const PrimF* __restrict__ primf, const FbInsn* __restrict__ chain,
+                                              int n_chain, const Accel& A, const float* __restrict__ pts, int64_t i,
+                                              double h, int s, unsigned beyond, unsigned left, Survivors& survivors,
+                                              uint8_t* items, float* vals) {
+    const int lane = threadIdx.x & 31;
+    const Variants V = load_query<kItems>(pts, i, h);
+    const float reach = finite_reach<NV>(V);
+    const int whole_cost = 100 * (NV + 1), point_cost = 45 * n_chain + 1500;
+    unsigned scattered = 0u;
+    for (unsigned todo = __ballot_sync(0xffffffffu, beyond != 0u); todo;) {
+        const int group_s = __shfl_sync(0xffffffffu, s, __ffs(todo) - 1);
+        const bool in = beyond != 0u && s == group_s;
+        const unsigned group = __ballot_sync(0xffffffffu, in), mask = in ? beyond : 0u;
+        todo &= ~group;
+        float c[3], far = in ? reach : 0.f;
+        const float R = ball_of<NV>(V, mask, c);
+        for (int o = 16; o > 0; o >>= 1) far = fmaxf(far, __shfl_xor_sync(0xffffffffu, far, o));
+        const uint32_t* list = nullptr;  // the whole chain
+        int len = n_chain;
+        cull_to<kStretches>(list, len, chain, primf, c, R, far, A.eps, survivors);
+        if ((int64_t)len * whole_cost > (int64_t)__popc(group) * point_cost) {
+            scattered |= group;
+        } else {
+            float acc[NV];
+            eval_variants<NV>(primf, chain, list, len, V, acc);
+#pragma unroll
+            for (int k = 0; k < NV; ++k)
+                if ((mask >> k) & 1u) vals[lane * NV + k] = acc[k];
+        }
+        __syncwarp();
+    }
+    if ((int64_t)n_chain * whole_cost <= (int64_t)__popc(scattered) * point_cost) {
+        const unsigned mask = (scattered >> lane) & 1u ? beyond : 0u;
+        if (NV == 1) {
+            if (mask) vals[lane] = eval_list(primf, chain, nullptr, n_chain, V.p[0], V.p[1], V.p[2]);
+        } else {
+            float acc[NV];
+            eval_variants<NV>(primf, chain, nullptr, n_chain, V, acc);
+#pragma unroll
+            for (int k = 0; k < NV; ++k)
+                if ((mask >> k) & 1u) vals[lane * NV + k] = acc[k];
+        }
+        scattered = 0u;
+    }
+    __syncwarp();
+    for (; scattered; scattered &= scattered - 1) {
+        const int o = __ffs(scattered) - 1;
+        const unsigned his = __shfl_sync(0xffffffffu, beyond, o);
+        const int64_t at = __shfl_sync(0xffffffffu, i, o);
+        const float far = __shfl_sync(0xffffffffu, reach, o);
+        const Variants W = load_query<kItems>(pts, at, h);
+        float r = 0.f;
+        if (NV > 1) {
+#pragma unroll
+            for (int a = 0; a < 3; ++a) r = fmaxf(r, fmaxf(fabsf(W.plus[a] - W.p[a]), fabsf(W.minus[a] - W.p[a])));
+        }
+        const uint32_t* list = nullptr;
+        int len = n_chain;
+        cull_to<kStretches>(list, len, chain, primf, W.p, r * 1.00001f, far, A.eps, survivors);
+        __syncwarp();
+        if (lane < NV && ((his >> lane) & 1u))
+            vals[o * NV + lane] = eval_list(primf, chain, list, len, W.at(lane, 0), W.at(lane, 1), W.at(lane, 2));
+        __syncwarp();
+    }
+    int before = __popc(left);
+    const int mine = before;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, before, o);
+        if (lane >= o) before += y;
+    }
+    const int total = __shfl_sync(0xffffffffu, before, 31);
+    before -= mine;
+    for (unsigned b = left; b; b &= b - 1) items[before++] = (uint8_t)(lane * 8 + __ffs(b) - 1);
+    __syncwarp();
+    for (int t = 0; t < total; t += 32) {
+        const int item = t + lane < total ? items[t + lane] : 0;
+        const int own = item >> 3, v = item & 7;
+        const int64_t at = __shfl_sync(0xffffffffu, i, own);
+        if (t + lane < total) {
+            const Variants W = load_query<kItems>(pts, at, h);
+            const float x = W.at(v, 0), y = W.at(v, 1), z = W.at(v, 2);
+            const uint32_t* list;
+            int len;
+            accel_list(A, n_chain, x, y, z, list, len);
+            vals[own * NV + v] = eval_list(primf, chain, list, len, x, y, z);
+        }
+    }
+    __syncwarp();
+}
+
 // A thread per point in sorted order.  The warp's points of one superblock form a group: its list is
 // culled to the ball around the group's variants, then every lane evaluates its NV variants on what is
-// left.  Variants outside the ball are handed out to the lanes afterwards, each on its own list.
+// left.  Variants outside the ball follow in eval_rest.
 // Bound by instruction issue and the latencies of 20 warps per SM (52 % of issue slots, 30 of 32
 // lanes): 10^6 points with gradients on a 256^3 field of 576 elements in 445 us, against 2680 us for
 // 7 10^6 sorted evaluations on the whole superblock lists (and 1100 us for their keys and scatter, which
 // go by points now: 24 us).  Groups are kept to one superblock: one group of far points in a warp, whose
 // ball nothing is culled from, took 600 us by itself.
-template <int NV>
+template <int NV, bool kStretches, bool kItems = false>
 __global__ void __launch_bounds__(32 * kQueryWarps, 5) k_query_sorted(const PrimF* __restrict__ primf,
                                                                    const FbInsn* __restrict__ chain, int n_chain,
-                                                                   Accel A, const float* __restrict__ pts, int64_t n,
-                                                                   double h, const int32_t* __restrict__ order,
+                                                                   const __grid_constant__ Accel A,
+                                                                   const float* __restrict__ pts, int64_t n, double h,
+                                                                   const int32_t* __restrict__ order,
+                                                                   const int32_t* __restrict__ inside,
                                                                    float* __restrict__ grad,
                                                                    float* __restrict__ value) {
+    if (inside) n = *inside;  // the rest is k_query_outside's
     __shared__ Survivors s_list[kQueryWarps];
     __shared__ uint8_t s_item[kQueryWarps][32 * NV];
     __shared__ float s_val[kQueryWarps][32 * NV];
@@ -545,104 +702,80 @@ __global__ void __launch_bounds__(32 * kQueryWarps, 5) k_query_sorted(const Prim
     for (int64_t w = blockIdx.x * (int64_t)kQueryWarps + warp; w * 32 < n; w += nwarps) {
         const bool live = w * 32 + lane < n;
         const int64_t i = live ? order[w * 32 + lane] : 0;
-        const Variants V = load_variants(pts, i, h);
+        const Variants V = load_query<kItems>(pts, i, h);
         const Place P = place_of<NV>(A, V, 1);
         float r[NV];
 #pragma unroll
         for (int k = 0; k < NV; ++k) r[k] = 0.f;
-        // groups: the variants in one superblock's ball, then those beyond the grid nearest to one
-        const float reach = finite_reach<NV>(V);
-        const bool ball = P.inside & 1u;
-        const unsigned beyond = live && reach >= 0.f ? P.beyond : 0u;
-        unsigned todo = __ballot_sync(0xffffffffu, live && ball), after = __ballot_sync(0xffffffffu, beyond != 0u);
-        while (todo | after) {
-            const bool whole = !todo;
-            const int s = __shfl_sync(0xffffffffu, P.s, __ffs(whole ? after : todo) - 1);
-            const bool in = (whole ? beyond != 0u : live && ball) && P.s == s;
-            const unsigned mask = !in ? 0u : (whole ? beyond : P.inside);
-            float lo[3], hi[3];
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                const unsigned fixed = mask & ~(6u << (2 * a));  // variants at the point's own coordinate a
-                lo[a] = fixed ? V.p[a] : 3.0e38f;
-                hi[a] = fixed ? V.p[a] : -3.0e38f;
-                if (NV > 1) {
-                    if (mask & (2u << (2 * a))) { lo[a] = fminf(lo[a], V.plus[a]); hi[a] = fmaxf(hi[a], V.plus[a]); }
-                    if (mask & (4u << (2 * a))) { lo[a] = fminf(lo[a], V.minus[a]); hi[a] = fmaxf(hi[a], V.minus[a]); }
-                }
+        bool open = live;  // not evaluated yet
+        if (NV == 1) {
+            const uint32_t* list;
+            int len;
+            accel_list(A, n_chain, V.p[0], V.p[1], V.p[2], list, len);
+            if (live && len <= kDirectList) {
+                r[0] = eval_list(primf, chain, list, len, V.p[0], V.p[1], V.p[2]);
+                open = false;
             }
-            float c[3], d = 0.f;
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                for (int o = 16; o > 0; o >>= 1) {
-                    lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
-                    hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
-                }
-                c[a] = 0.5f * lo[a] + 0.5f * hi[a];
-                const float e = fmaxf(hi[a] - c[a], c[a] - lo[a]);
-                d = fmaf(e, e, d);
-            }
-            const float R = sqrtf(d) * 1.00001f;
-            const uint32_t* list = nullptr;  // the whole chain
-            int len = n_chain;
-            float far = 0.f;
-            if (whole) {
-                far = in ? reach : 0.f;
-                for (int o = 16; o > 0; o >>= 1) far = fmaxf(far, __shfl_xor_sync(0xffffffffu, far, o));
-            } else {
-                list = A.pool + A.sb_off[s];
-                len = A.sb_len[s];
-            }
-            cull_to(list, len, chain, primf, c, R, far, A.eps, s_list[warp]);
+            __syncwarp();
+        }
+        const bool ball = open && (P.inside & 1u);
+        for (unsigned todo = __ballot_sync(0xffffffffu, ball); todo;) {  // groups: the variants in one superblock's ball
+            const int s = __shfl_sync(0xffffffffu, P.s, __ffs(todo) - 1);
+            const bool in = ball && P.s == s;
+            todo &= ~__ballot_sync(0xffffffffu, in);
+            // a lone variant is inside where its lane is in (written so: from `in ? P.inside : 0u` nvcc 12.9 made
+            // 0 for NV = 1 with both set)
+            const unsigned mask = in ? (NV == 1 ? 1u : P.inside) : 0u;
+            float c[3];
+            const float R = ball_of<NV>(V, mask, c);
+            const uint32_t* list = A.pool + A.sb_off[s];
+            int len = A.sb_len[s];
+            cull_to<kStretches>(list, len, chain, primf, c, R, 0.f, A.eps, s_list[warp]);
             float acc[NV];
             eval_variants<NV>(primf, chain, list, len, V, acc);
 #pragma unroll
             for (int k = 0; k < NV; ++k)
                 if ((mask >> k) & 1u) r[k] = acc[k];
-            const unsigned done = __ballot_sync(0xffffffffu, in);
-            if (whole) after &= ~done;
-            else todo &= ~done;
             __syncwarp();
         }
-        // variants left over
-        const unsigned left = live ? ~(P.inside | beyond) & ((1u << NV) - 1u) : 0u;
-        int before = __popc(left);
-        const int mine = before;
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, before, o);
-            if (lane >= o) before += y;
-        }
-        const int total = __shfl_sync(0xffffffffu, before, 31);
-        if (total) {
-            before -= mine;
-            for (unsigned b = left; b; b &= b - 1) s_item[warp][before++] = (uint8_t)(lane * 8 + __ffs(b) - 1);
-            __syncwarp();
-            for (int t = 0; t < total; t += 32) {
-                const int item = t + lane < total ? s_item[warp][t + lane] : 0;
-                const int own = item >> 3, v = item & 7;
-                float q[3];
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    q[a] = __shfl_sync(0xffffffffu, V.p[a], own);
-                    const float qp = __shfl_sync(0xffffffffu, V.plus[a], own), qm = __shfl_sync(0xffffffffu, V.minus[a], own);
-                    if (v == 1 + 2 * a) q[a] = qp;
-                    if (v == 2 + 2 * a) q[a] = qm;
-                }
-                if (t + lane < total) {
-                    const uint32_t* list;
-                    int len;
-                    accel_list(A, n_chain, q[0], q[1], q[2], list, len);
-                    s_val[warp][own * NV + v] = eval_list(primf, chain, list, len, q[0], q[1], q[2]);
-                }
-                __syncwarp();
-            }
+        const unsigned rest = open ? ~P.inside & ((1u << NV) - 1u) : 0u;
+        if (__any_sync(0xffffffffu, rest != 0u)) {
+            const unsigned beyond = finite_reach<NV>(V) >= 0.f ? rest & P.beyond : 0u;
+            eval_rest<NV, kStretches, kItems>(primf, chain, n_chain, A, pts, i, h, P.s, beyond, rest & ~beyond, s_list[warp],
+                                              s_item[warp], s_val[warp]);
 #pragma unroll
             for (int k = 0; k < NV; ++k)
-                if ((left >> k) & 1u) r[k] = s_val[warp][lane * NV + k];
+                if ((rest >> k) & 1u) r[k] = s_val[warp][lane * NV + k];
             __syncwarp();
         }
         if (live) write_point(i, r, inv, NV > 1 ? grad : nullptr, value);
     }
+}
+
+// The sorted points from *inside on, which lie far outside the grid, on the whole chain: a thread each.
+template <bool kItems>
+__global__ void __launch_bounds__(256) k_query_outside(const PrimF* __restrict__ primf, const FbInsn* __restrict__ chain,
+                                                       int n_chain, const float* __restrict__ pts, int64_t n, double h,
+                                                       const int32_t* __restrict__ order,
+                                                       const int32_t* __restrict__ inside, float* __restrict__ value) {
+    for (int64_t t = *inside + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t i = order[t];
+        const Variants V = load_query<kItems>(pts, i, h);
+        value[i] = eval_point(primf, chain, n_chain, 1, nullptr, n_chain, V.p[0], V.p[1], V.p[2]);
+    }
+}
+
+// Chains longer than this (about what L1 holds of their records) are not culled for points far outside the grid
+// where each is one evaluation: 100 000 of them scattered around a 512^3 field of 3000 elements 8600 us with the groups'
+// and points' culls, 2200 a thread each.
+constexpr int kCulledOutside = 1024;
+
+// From the seven values of every point: the value and the gradient, k_gradient_points' arithmetic.
+__global__ void k_query_combine(const float* __restrict__ vals, int64_t n, double h, float* __restrict__ grad,
+                                float* __restrict__ value) {
+    const float inv = (float)(2.0 * h);
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        write_point(i, vals + 7 * i, inv, grad, value);
 }
 
 // Up to warp_points points go a warp per point, without scratch; more are sorted first.  Values and
@@ -659,36 +792,75 @@ int64_t warp_points(int64_t nsuper, bool grad) {
     return grad ? kWarpPoints : std::min<int64_t>(kWarpPoints, 19000 + 6 * nsuper);
 }
 
-struct SortedPlan {
-    int64_t nsuper, nbins, ntiles;
+// Gradient queries as 7 n points of their own -- the points and their offsets sorted together, values combined
+// at the end -- against a thread per point with its seven variants (us, steps of 1 and 4 voxels):
+//   64^3 field of 60 elements     41 000 points  87, 103 / 118, 194    200 000  263, 310 / 151, 290
+//   256^3, 576                    41 000  99, 142 / 419, 534    400 000  384, 462 / 421, 665    10^6  824, 998 / 630, 1029
+//   512^3, 3000                   41 000  196, 368 / 1064, 1381    400 000  742, 1064 / 982, 1562    10^6  1599, 2177 / 1291, 2369
+//   256^3, 300 blends             41 000  146, 175 / 577, 699    400 000  658, 753 / 646, 984
+// Seven variants in one lane are a long chain of evaluations in few warps; with enough points the groups' culls,
+// seven times as many, outweigh it, the later the more superblocks there are, the longer the step (which takes
+// variants out of their point's ball) and the longer the lists (100 000 points, 16 elements: 97 / 65).  Few points go by the warp (20 480 points of the 64^3 field 64,
+// 32 768 95), except for steps over a quarter of a superblock's edge.
+bool by_items(int64_t nsuper, int64_t n_chain, int64_t n, double edges) {  // edges: the step in superblock edges
+    if (n <= std::min<int64_t>(40960, 24000 + 4 * nsuper)) return edges > 0.25;
+    const double most = 30000.0 + std::min(std::min(400.0 * nsuper, 1000.0 * n_chain), 500000.0);
+    return edges >= 1.0 || (double)n <= most * (1.0 + 8.0 * edges);
+}
+
+// Chains this short are evaluated whole, a thread per point, where the points are many for them (both sides
+// measured on 2 to 64 parts, 1000 to 10^6 points: 4 parts 9 us against 36 for 40 000 values, 19 against 76 with
+// gradients; 12 parts 41 against 88; 8 parts 10^6 with gradients 272 against 183).
+bool short_chain(int n_chain, int64_t n, int64_t warp_most, bool grad) {
+    if (grad) return n <= warp_most ? n > 1700 * (int64_t)n_chain : n_chain <= 12 && n * n_chain <= 3500000;
+    return n <= warp_most ? n > 650 * (int64_t)n_chain : n_chain <= 32 && n * n_chain <= 32000000;
+}
+
+// How a query on an accelerated grid runs and where its scratch lies.
+struct QueryPlan {
+    int64_t nsuper, n;  // n: points, or their evaluations
+    bool items, sorted;
+    int64_t nbins, ntiles;
     int C;  // sorting cells per superblock edge
-    int64_t keys, order, count, tiles, total;
+    int64_t vals, keys, order, count, tiles, total;
 };
 
-constexpr int64_t kMaxBins = int64_t(kScanTile) * kScanTile;  // one tile-sum CTA covers them
+constexpr int64_t kMaxBins = int64_t(kScanTile) * kScanTile;  // one tile-sum CTA covers them (one for points outside)
 constexpr int64_t kMaxSortedPoints = int64_t(1) << 31;        // sorted positions are int32
 
-// false: that grid or that many points are not sorted.
-bool sorted_plan(const int32_t* dims, int64_t n, SortedPlan& p) {
+// edges: the step in superblock edges; negative where it is not known.  n_chain: kAnyChain for the most scratch.
+constexpr int64_t kAnyChain = int64_t(1) << 31;
+
+QueryPlan query_plan(const int32_t* dims, int64_t n_chain, int64_t n, bool grad, double edges) {
+    QueryPlan p{};
     const int B = dims[3];
-    if (B < 1 || n >= kMaxSortedPoints) return false;
     const int64_t nbx = (dims[0] + B - 1) / B, nby = (dims[1] + B - 1) / B, nbz = (dims[2] + B - 1) / B;
     const int64_t S = std::max(1, fb_super_edge(dims[0], dims[1], dims[2]) / B);
-    const int64_t ns = ((nbx + S - 1) / S) * ((nby + S - 1) / S) * ((nbz + S - 1) / S);
-    for (p.C = 4; p.C > 1 && ns * p.C * p.C * p.C > kMaxBins; p.C /= 2) {
+    p.nsuper = ((nbx + S - 1) / S) * ((nby + S - 1) / S) * ((nbz + S - 1) / S);
+    p.items = grad && edges >= 0.0 && n < kMaxSortedPoints / 7 && by_items(p.nsuper, n_chain, n, edges);
+    p.n = p.items ? 7 * n : n;
+    for (p.C = 4; p.C > 1 && p.nsuper * p.C * p.C * p.C >= kMaxBins; p.C /= 2) {
     }
-    p.nsuper = ns;
-    p.nbins = ns * p.C * p.C * p.C;
-    if (ns < 1 || p.nbins > kMaxBins) return false;
+    p.nbins = p.nsuper * p.C * p.C * p.C;
+    p.ntiles = (p.nbins + 1 + kScanTile - 1) / kScanTile;
+    p.sorted = p.nsuper >= 1 && p.nbins < kMaxBins && p.n < kMaxSortedPoints &&
+               p.n > warp_points(p.nsuper, grad && !p.items);
     auto al = [](int64_t b) { return (b + 255) / 256 * 256; };
-    p.ntiles = (p.nbins + kScanTile - 1) / kScanTile;
     int64_t at = 0;
-    p.keys = at; at += al(n * 8);
-    p.order = at; at += al(n * 4);
-    p.count = at; at += al(p.nbins * 4);
-    p.tiles = at; at += al(p.ntiles * 4);
+    p.vals = at; at += p.items ? al(p.n * 4) : 0;
+    if (p.sorted) {
+        p.keys = at; at += al(p.n * 8);
+        p.order = at; at += al(p.n * 4);
+        p.count = at; at += al((p.nbins + 1) * 4);
+        p.tiles = at; at += al(p.ntiles * 4);
+    }
     p.total = at;
-    return true;
+    return p;
+}
+
+double step_edges(const double* grid, const int32_t* dims, double h) {
+    const int S = std::max(1, fb_super_edge(dims[0], dims[1], dims[2]) / dims[3]);
+    return std::fabs(h) / (S * dims[3] * grid[3]);
 }
 
 // ------------------------------------------------------------------------------------ multires
@@ -1046,12 +1218,19 @@ int fb_grid_pairs_device(const float* d_params, int32_t n_leaves, const float* d
 // whole chain / program.
 int fb_query_prepare(const FbPrim* d_prims, int32_t n_prims, void* d_primf, void* stream) noexcept;
 
-// Scratch bytes of the sorted query path for n points on an accelerated grid of dims (nx, ny, nz, B); 0
-// or -1: the query takes a path without scratch (few points; a grid that is not sorted).
+// Scratch bytes of a query of n points (with_grad: gradients, a thread or a warp per point whatever the step)
+// on an accelerated grid of dims (nx, ny, nz, B); 0 where it takes a path without scratch, -1 for
+// invalid arguments.
 int64_t fb_query_scratch_bytes(const int32_t* accel_dims, int64_t n, int32_t with_grad) noexcept {
-    SortedPlan P;
-    if (!accel_dims || n < 0 || !sorted_plan(accel_dims, n, P)) return -1;
-    return n <= warp_points(P.nsuper, with_grad != 0) ? 0 : P.total;
+    if (!accel_dims || accel_dims[3] < 1 || n < 0) return -1;
+    return query_plan(accel_dims, kAnyChain, n, with_grad != 0, -1.0).total;
+}
+
+// The same for gradients of step h on a grid of x0, y0, z0, pitch (accel_grid).
+int64_t fb_query_scratch_bytes_h(const double* accel_grid, const int32_t* accel_dims, int64_t n, int32_t with_grad,
+                                 double h) noexcept {
+    if (!accel_grid || !accel_dims || accel_dims[3] < 1 || n < 0) return -1;
+    return query_plan(accel_dims, kAnyChain, n, with_grad != 0, step_edges(accel_grid, accel_dims, h)).total;
 }
 
 int fb_query_points_device(const void* d_primf, const FbInsn* d_chain, int32_t n_chain, int32_t mode,
@@ -1064,7 +1243,7 @@ int fb_query_points_device(const void* d_primf, const FbInsn* d_chain, int32_t n
     if (!d_primf || !d_chain || n_chain < 1 || !d_points || n < 0 || (!d_value && !d_grad)) return FB_INVALID;
     if (n == 0) return FB_OK;
     Accel A{};
-    if (accel_pool && accel_off && accel_len && accel_grid && accel_dims && mode == 1) {
+    if (accel_pool && accel_off && accel_len && accel_grid && accel_dims && (mode == 1 || mode == 3) && accel_dims[3] >= 1) {
         A.pool = static_cast<const uint32_t*>(accel_pool);
         A.sb_off = accel_off;
         A.sb_len = accel_len;
@@ -1086,7 +1265,15 @@ int fb_query_points_device(const void* d_primf, const FbInsn* d_chain, int32_t n
     }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const PrimF* primf = static_cast<const PrimF*>(d_primf);
+    QueryPlan P{};
+    bool whole = !A.pool;
     if (A.pool) {
+        P = query_plan(accel_dims, n_chain, n, d_grad != nullptr, step_edges(accel_grid, accel_dims, h));
+        // scratch that was sized without the step, or none: its points in place of their evaluations
+        if (P.items && (!d_scratch || scratch_len < P.total)) P = query_plan(accel_dims, n_chain, n, true, -1.0);
+        whole = short_chain(n_chain, n, warp_points(P.nsuper, d_grad != nullptr), d_grad != nullptr);
+    }
+    if (!whole) {
         // 16 float32 ulps of the largest coordinate a superblock's ball reaches: the default guard's slack
         float far = 0.f;
         const double reach = (A.S * A.B + 1) * A.pitch;
@@ -1095,44 +1282,77 @@ int fb_query_points_device(const void* d_primf, const FbInsn* d_chain, int32_t n
         for (int a = 0; a < 3; ++a)
             far = std::max(far, (float)std::max(std::fabs(lo[a] - reach), std::fabs(lo[a] + ext[a] * A.pitch + reach)));
         A.eps = 16.f * (std::nextafter(far, 3.4e38f) - far);
-        SortedPlan P;
-        if (d_scratch && sorted_plan(accel_dims, n, P) && n > warp_points(P.nsuper, d_grad != nullptr)) {
-            if (scratch_len < P.total) return FB_INVALID;
-            char* b = static_cast<char*>(d_scratch);
+        const bool sorted = P.sorted && d_scratch;
+        if (sorted && scratch_len < P.total) return FB_INVALID;
+        char* b = static_cast<char*>(d_scratch);
+        float* out = P.items ? reinterpret_cast<float*>(b + P.vals) : d_value;
+        int32_t* order = nullptr;
+        const int32_t* inside = nullptr;
+        if (sorted) {
             int2* keys = reinterpret_cast<int2*>(b + P.keys);
-            int32_t* order = reinterpret_cast<int32_t*>(b + P.order);
+            order = reinterpret_cast<int32_t*>(b + P.order);
             int32_t* count = reinterpret_cast<int32_t*>(b + P.count);
             int32_t* tiles = reinterpret_cast<int32_t*>(b + P.tiles);
-            const int ge = (int)std::min<int64_t>((n + 255) / 256, (int64_t)fb_sm_count() * 16);
-            FB_CUDA(cudaMemsetAsync(count, 0, P.nbins * 4, st));
-            k_query_keys<<<ge, 256, 0, st>>>(A, d_points, n, P.C, keys, count);
+            const int ge = (int)std::min<int64_t>((P.n + 255) / 256, (int64_t)fb_sm_count() * 16);
+            const bool apart = n_chain > kCulledOutside && (P.items || !d_grad);
+            if (apart) inside = count + P.nbins;
+            const int outside = apart ? (int)P.nbins : -1;
+            FB_CUDA(cudaMemsetAsync(count, 0, (P.nbins + 1) * 4, st));
+            if (P.items) k_query_keys<true><<<ge, 256, 0, st>>>(A, d_points, P.n, h, P.C, outside, keys, count);
+            else k_query_keys<false><<<ge, 256, 0, st>>>(A, d_points, P.n, 0.0, P.C, outside, keys, count);
             FB_LAUNCH();
-            k_scan_tiles<<<(unsigned)P.ntiles, kScanThreads, 0, st>>>(count, P.nbins, tiles);
+            k_scan_tiles<<<(unsigned)P.ntiles, kScanThreads, 0, st>>>(count, P.nbins + 1, tiles);
             FB_LAUNCH();
             k_scan_sums<<<1, kScanThreads, 0, st>>>(tiles, (int)P.ntiles);
             FB_LAUNCH();
-            k_scan_add<<<(int)std::min<int64_t>((P.nbins + 255) / 256, (int64_t)fb_sm_count() * 16), 256, 0, st>>>(
-                count, P.nbins, tiles);
+            k_scan_add<<<(int)std::min<int64_t>((P.nbins + 256) / 256, (int64_t)fb_sm_count() * 16), 256, 0, st>>>(
+                count, P.nbins + 1, tiles);
             FB_LAUNCH();
-            k_query_scatter<<<ge, 256, 0, st>>>(keys, n, count, order);
+            k_query_scatter<<<ge, 256, 0, st>>>(keys, P.n, count, order);
             FB_LAUNCH();
-            const int gs = (int)std::min<int64_t>((n + 127) / 128, (int64_t)fb_sm_count() * 64);
-            if (d_grad)
-                k_query_sorted<7><<<gs, 32 * kQueryWarps, 0, st>>>(primf, d_chain, n_chain, A, d_points, n, h, order,
-                                                                   d_grad, d_value);
-            else
-                k_query_sorted<1><<<gs, 32 * kQueryWarps, 0, st>>>(primf, d_chain, n_chain, A, d_points, n, 0.0, order,
-                                                                   nullptr, d_value);
-            FB_LAUNCH();
-            return FB_OK;
         }
-        const int gw = (int)std::min<int64_t>((n + kQueryWarps - 1) / kQueryWarps, (int64_t)fb_sm_count() * 64);
-        if (d_grad)
-            k_query_warp<7><<<gw, 32 * kQueryWarps, 0, st>>>(primf, d_chain, n_chain, A, d_points, n, h, d_grad, d_value);
-        else
-            k_query_warp<1><<<gw, 32 * kQueryWarps, 0, st>>>(primf, d_chain, n_chain, A, d_points, n, 0.0, nullptr,
-                                                             d_value);
+        const int per = sorted ? 32 * kQueryWarps : kQueryWarps;  // points a CTA takes at a time
+        const int gs = (int)std::min<int64_t>((P.n + per - 1) / per, (int64_t)fb_sm_count() * 64);
+        auto run = [&](auto nv, auto stretches, auto items) {
+            constexpr int NV = decltype(nv)::value;
+            constexpr bool kS = decltype(stretches)::value, kI = decltype(items)::value;
+            const double step = NV > 1 || kI ? h : 0.0;
+            float* grad = NV > 1 ? d_grad : nullptr;
+            if (sorted)
+                k_query_sorted<NV, kS, kI><<<gs, 32 * kQueryWarps, 0, st>>>(primf, d_chain, n_chain, A, d_points, P.n, step,
+                                                                            order, inside, grad, out);
+            else
+                k_query_warp<NV, kS, kI><<<gs, 32 * kQueryWarps, 0, st>>>(primf, d_chain, n_chain, A, d_points, P.n, step,
+                                                                          grad, out);
+        };
+        const std::integral_constant<int, 1> one;
+        const std::integral_constant<int, 7> seven;
+        const std::true_type yes;
+        const std::false_type no;
+        if (P.items) {
+            if (mode == 3) run(one, yes, yes);
+            else run(one, no, yes);
+        } else if (d_grad) {
+            if (mode == 3) run(seven, yes, no);
+            else run(seven, no, no);
+        } else {
+            if (mode == 3) run(one, yes, no);
+            else run(one, no, no);
+        }
         FB_LAUNCH();
+        if (inside) {
+            const int go = (int)std::min<int64_t>((P.n + 255) / 256, (int64_t)fb_sm_count() * 16);
+            if (P.items)
+                k_query_outside<true><<<go, 256, 0, st>>>(primf, d_chain, n_chain, d_points, P.n, h, order, inside, out);
+            else
+                k_query_outside<false><<<go, 256, 0, st>>>(primf, d_chain, n_chain, d_points, P.n, 0.0, order, inside, out);
+            FB_LAUNCH();
+        }
+        if (P.items) {
+            k_query_combine<<<(int)std::min<int64_t>((n + 255) / 256, (int64_t)fb_sm_count() * 16), 256, 0, st>>>(
+                out, n, h, d_grad, d_value);
+            FB_LAUNCH();
+        }
         return FB_OK;
     }
     const int grid = (int)std::min<int64_t>((n + 127) / 128, (int64_t)fb_sm_count() * 16);

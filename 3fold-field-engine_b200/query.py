@@ -18,10 +18,21 @@ import ctypes as ct
 import numpy as np
 
 from . import _lib
+from . import expr as X
 from .expr import Compiled, compile_recipe
 from .build import device_tables
 
 PRIMF_BYTES = 128
+
+
+def _many_steps(chain):
+    """Whether a chain is many short runs of one hard boolean, blends and offsets rather than a few long runs:
+    more than 12 of them that are no run of at least 9."""
+    op, k = chain["op"], chain["k"]
+    hard = (k <= 0) & np.isin(op, (X.CH_UNION, X.CH_INTERSECT, X.CH_SUBTRACT))
+    key = np.where(hard, op, -1 - np.arange(len(op)))  # every other element a run of its own
+    runs = np.diff(np.flatnonzero(np.concatenate(([True], key[1:] != key[:-1], [True]))))
+    return int((runs < 9).sum()) > 12
 
 
 class RecipeQueries:
@@ -35,6 +46,7 @@ class RecipeQueries:
         c = self.compiled
         self.mode = 1 if c.chain is not None else 0
         insns = c.chain if self.mode == 1 else c.program
+        self._walk = 3 if self.mode == 1 and _many_steps(c.chain) else self.mode
         self.n_chain = len(insns)
         self.prims, self.chain = device_tables(c, self.device, torch.cuda.current_stream(self.device))
         self.primf = torch.empty(len(c.prims) * PRIMF_BYTES, dtype=torch.uint8, device=self.device)
@@ -66,7 +78,8 @@ class RecipeQueries:
         a = self._accel
         scratch, nscratch = None, 0
         if a is not None and pts.shape[0] > 0:
-            nbytes = int(self.lib.fb_query_scratch_bytes(a[4].ctypes.data, pts.shape[0], 1 if grad is not None else 0))
+            nbytes = int(self.lib.fb_query_scratch_bytes_h(a[3].ctypes.data, a[4].ctypes.data, pts.shape[0],
+                                                           1 if grad is not None else 0, float(h)))
             if nbytes > 0:
                 nscratch = nbytes
                 if alloc is not None:
@@ -77,7 +90,7 @@ class RecipeQueries:
                         scratch.record_stream(stream)
         args = (a[0], a[1], a[2], a[3].ctypes.data, a[4].ctypes.data, *a[5]) if a else (None,) * 5 + (None, None,
                                                                                                      None, None, 0, 0)
-        st = self.lib.fb_query_points_device(self.primf.data_ptr(), self.chain.data_ptr(), self.n_chain, self.mode,
+        st = self.lib.fb_query_points_device(self.primf.data_ptr(), self.chain.data_ptr(), self.n_chain, self._walk,
                                              *args, pts.data_ptr(), pts.shape[0], float(h),
                                              value.data_ptr() if value is not None else None,
                                              grad.data_ptr() if grad is not None else None,

@@ -308,7 +308,8 @@ int fb_grid_pairs_device(const float* d_params, int32_t n_leaves, const float* d
  * fb_query_prepare fills the 128-byte float32 primitive mirror; fb_field_accel exposes a
  * classification's culling lists inside its scratch (superblock and per-block) so that points
  * inside that grid walk only their block's list (where the classification kept one; blk_all = 1:
- * every block, else blocks of kind 0) or their superblock's list. */
+ * every block, else blocks of kind 0) or their superblock's list.  mode: 0 a program, 1 a chain, 3 a chain of
+ * many short runs or blends (its lists are then culled by the stretch; the results are the same). */
 int fb_query_prepare(const fb_prim* d_prims, int32_t n_prims, void* d_primf, void* stream);
 int fb_field_accel(const fb_geom* g, int32_t n_prims, int32_t n_chain, const void* d_scratch, const void** pool,
                    const int64_t** sb_off, const int32_t** sb_len, const int32_t** blk_off, const int32_t** blk_len,
@@ -319,10 +320,14 @@ int fb_query_points_device(const void* d_primf, const fb_insn* d_chain, int32_t 
                            const int32_t* blk_off, const int32_t* blk_len, const uint32_t* blk_pool, int64_t blk_cap,
                            int32_t blk_all, const float* d_points, int64_t n, double h, float* d_value, float* d_grad,
                            void* d_scratch, int64_t scratch_len, void* stream);
-/* Scratch of the sorted query path (points sorted by cell, so a warp's points share one culled list);
- * 0 or -1 when that query takes a path without scratch (few points; a grid that is not sorted).  No
- * reference counterpart: an execution strategy of fb_query_points_device, same results bit for bit. */
+/* Scratch of the query (points sorted by cell, so a warp's points share one culled list); 0 when it takes a
+ * path without scratch (few points; a grid that is not sorted).  fb_query_scratch_bytes_h knows the step: where
+ * that is faster the offset points are then queried as points of their own, which takes more scratch (with the
+ * scratch of the other they are not).  No reference counterpart: execution strategies of
+ * fb_query_points_device, same results bit for bit. */
 int64_t fb_query_scratch_bytes(const int32_t* accel_dims, int64_t n, int32_t with_grad);
+int64_t fb_query_scratch_bytes_h(const double* accel_grid, const int32_t* accel_dims, int64_t n, int32_t with_grad,
+                                 double h);
 
 /* Replace the per-block-pitch field's lattices and its avstand / gradient queries,
  * src/field_engine/faltkarna_v1_multires.py:84-104,384-459 (lattices built from a recipe). */
