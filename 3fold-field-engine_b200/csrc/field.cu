@@ -2016,7 +2016,6 @@ __device__ __forceinline__ void leaf_block(const Geo& G, const FbPrim* __restric
     if (near) recheck_near<B, VG>(near, lane, out, list, len, chain, prims, G, bi, bj, bk);
 }
 
-// Leaf tiles of a chain recipe: a warp per active block (leaf_block).
 // Up to kLeafGroupMost active blocks of one recipe by one warp: their ids, list places and list entries are
 // read by the lanes side by side and the elements of their lists localised in rounds of lanes, so the
 // dependent loads in front of a block's first evaluation (id, list place, entry, instruction,
@@ -2024,14 +2023,24 @@ __device__ __forceinline__ void leaf_block(const Geo& G, const FbPrim* __restric
 // outside the grid are left to leaf_alone, a warp per block in a second loop: their lists are long, and
 // four of them in one group's warp took as long as all the rest.  Measured: 1024^3 part 1380 -> 1109 us
 // (8^3, 2.3 elements a block); the 4^3 recipes of a batch of 20 2420 -> 1008 us.
-// Blocks a group takes: as many as still leave a group for each of the ~3000 warps the GPU holds.
-constexpr int64_t kLeafResident = 3000;
+// Only for many blocks of short lists: few blocks' groups fill the ~3000 resident warps in two or three uneven
+// waves, and with longer lists the evaluation is the time (8^3 blocks, grouped against alone: 28 000 of 6.2 elements in
+// the mean 490 / 328 us, 220 000 of 6.0 2549 / 2096, 34 000 of 1.8 154 / 131, 43 000 of 2.7 86 / 97, 105 000 of 2.7
+// 173 / 208; 4^3: 163 000 of 2.8 216 / 242, 137 000 of 1.1 90 / 166, 12 600 of 1.4 26 / 29).  The lists' lengths are on
+// the device: where they turn out long the grouped kernel takes the blocks alone as well, at its 5 CTAs per SM (8 %
+// behind k_leaf's 6; an empty launch of k_leaf beside it cost every build 8 us).
+constexpr int kLeafGroupMost = 8;
 
 template <int B>
-__device__ __forceinline__ int leaf_group_size(int64_t n) {
-    return (int)min(max(n / kLeafResident, (int64_t)1), (int64_t)(B == 4 ? 8 : 4));
+__host__ __device__ constexpr int64_t group_least() { return B == 4 ? 10000 : 40000; }
+
+// Blocks a group takes, 1: alone.  entries: list entries of all n blocks.
+template <int B>
+__device__ __forceinline__ int leaf_group_size(int64_t n, int64_t entries) {
+    const int64_t most = n >= 40000 ? 4 * n : 2 * n;
+    if (n < group_least<B>() || entries > most) return 1;
+    return (int)min(max(n / (n >= 40000 ? 10000 : 4000), (int64_t)2), (int64_t)(B == 4 ? 8 : 4));
 }
-constexpr int kLeafGroupMost = 8;
 
 // leaf_block out of line, for the blocks that do not go in groups.
 template <int B, bool kEdge>
@@ -2169,6 +2178,7 @@ __device__ __forceinline__ void leaf_group(const Geo& G, const FbPrim* __restric
     __syncwarp();  // `sp` is staged again by the next group
 }
 
+// Leaf tiles of a chain recipe: a warp per active block (leaf_block).
 template <int B, bool kEdge>
 __global__ void __launch_bounds__(32 * kLeafWarps, 6) k_leaf(Geo G, const FbPrim* __restrict__ prims,
                                                              const PrimF* __restrict__ primf,
@@ -2205,7 +2215,7 @@ __global__ void __launch_bounds__(32 * kLeafWarps, 5) k_leaf_groups(Geo G, const
                                                              const int32_t* __restrict__ sb_len,
                                                              const int32_t* __restrict__ active,
                                                              const int32_t* __restrict__ count, int64_t capacity,
-                                                             float* __restrict__ tiles,
+                                                             float* __restrict__ tiles, const int* __restrict__ entries,
                                                              const int32_t* __restrict__ kind,
                                                              const int32_t* __restrict__ blk_off,
                                                              const int32_t* __restrict__ blk_len,
@@ -2217,7 +2227,7 @@ __global__ void __launch_bounds__(32 * kLeafWarps, 5) k_leaf_groups(Geo G, const
     const int64_t gwarp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const int64_t n_active = min((int64_t)count[0], capacity);
-    const int K = leaf_group_size<B>(n_active), lane = threadIdx.x & 31;
+    const int K = leaf_group_size<B>(n_active, *entries), lane = threadIdx.x & 31;
     if (K == 1) {
         for (int64_t a = gwarp; a < n_active; a += nwarps)
             leaf_block<B, kEdge>(G, prims, primf, chain, pool, sb_off, sb_len, active[a], tiles + a * (B * B * B),
@@ -2480,7 +2490,7 @@ int launch_compact(const int32_t* kind, int64_t nblocks, int32_t* active, int32_
                    int* misc, cudaStream_t st) {
     const int64_t ntiles = (nblocks + kTile - 1) / kTile;
     FB_CUDA(cudaMemsetAsync(status, 0, ntiles * 8, st));
-    FB_CUDA(cudaMemsetAsync(misc, 0, 256, st));
+    FB_CUDA(cudaMemsetAsync(misc, 0, 8, st));  // the list entries' count behind stays
     k_compact<<<(unsigned)ntiles, 256, 0, st>>>(kind, nblocks, active, count, status, misc, ntiles, kLookbackSpins);
     FB_LAUNCH();
     return FB_OK;
@@ -2530,10 +2540,10 @@ int classify_impl(const FbGeom& g, const FbPrim* prims, int n_prims, const FbIns
     return FB_OK;
 }
 
-// Whether a leaf pass over at most `most` blocks may take groups: the host knows no more than that (the
-// kernel decides the group size from the count), and the kernel without the grouped path is the faster
-// one where every group would be a single block (the 169 x 129 x 89 plate: 17.8 against 20.7 us).
-bool leaf_in_groups(int64_t most, const void* work) { return !work && most >= 2 * kLeafResident; }
+// Whether a leaf pass over at most `most` blocks may take groups: the host knows no more than that.
+bool leaf_in_groups(int B, int64_t most, const void* work) {
+    return !work && B < 16 && most >= (B == 4 ? group_least<4>() : group_least<8>());
+}
 
 int leaf_impl(const FbGeom& g, const FbPrim* prims, int n_prims, const FbInsn* chain, int n_chain, int mode,
               const int32_t* kind, const int32_t* active, const int32_t* count, float* tiles, int64_t capacity,
@@ -2565,9 +2575,9 @@ int leaf_impl(const FbGeom& g, const FbPrim* prims, int n_prims, const FbInsn* c
                                                        S.blk_pool, P.blk_cap)
 #define FB_LEAF_GROUPS(BB, EDGE)                                                                                   \
     k_leaf_groups<BB, EDGE><<<grid, 32 * kLeafWarps, 0, st>>>(G, prims, S.primf, chain, S.pool, sb_off, sb_len, active, \
-                                                              count, capacity, tiles, kind, S.blk_off, S.blk_len,      \
+                                                              count, capacity, tiles, S.misc + 2, kind, S.blk_off, S.blk_len, \
                                                               S.blk_pool, P.blk_cap)
-        const bool edge = G.special != 0, groups = leaf_in_groups(std::min(G.nblocks, capacity), work);
+        const bool edge = G.special != 0, groups = leaf_in_groups(G.B, std::min(G.nblocks, capacity), work);
         switch (G.B) {
         case 4:
             if (groups) { if (edge) FB_LEAF_GROUPS(4, true); else FB_LEAF_GROUPS(4, false); }
@@ -2807,7 +2817,8 @@ __global__ void __launch_bounds__(32 * kLeafWarps, 5) k_b_leaf(const RecDesc* __
 template <int B, bool kEdge>
 __global__ void __launch_bounds__(32 * kLeafWarps, 5) k_b_leaf_groups(const RecDesc* __restrict__ D, Group W,
                                                                float* __restrict__ tiles,
-                                                               const int64_t* __restrict__ tile_off) {
+                                                               const int64_t* __restrict__ tile_off,
+                                                               const int* __restrict__ cursors) {
     __shared__ LocalPrim s_prim[kLeafWarps][kCapBlock];
     __shared__ uint32_t s_list[kLeafWarps][kCapBlock];
     __shared__ float4 s_acc[kLeafWarps][B == 8 ? 128 : 1];  // 8^3 tiles: running values, 4 groups x 32 lanes
@@ -2815,7 +2826,11 @@ __global__ void __launch_bounds__(32 * kLeafWarps, 5) k_b_leaf_groups(const RecD
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const int64_t total = W.pre[W.m];
     const int64_t gwarp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int K = leaf_group_size<B>(total), lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31;
+    int64_t entries = 0;  // of all the group's recipes
+    for (int j = lane; j < W.m; j += 32) entries += cursors[W.rec[j]];
+    for (int o = 16; o > 0; o >>= 1) entries += __shfl_xor_sync(0xffffffffu, entries, o);
+    const int K = leaf_group_size<B>(total, entries);
     if (K == 1) {
         for (int64_t g = gwarp; g < total; g += nwarps) {
             const int j = group_find(W, g);
@@ -3134,23 +3149,23 @@ int fb_batch_build_timed_device(void* batch, float* d_tiles, int64_t capacity, i
     for (int q = 0; q < kLeafGroups; ++q) {
         if (!H->leaf[q].m) continue;
         const Group& W = H->leaf[q];
-        const bool groups = leaf_in_groups(H->leaf_blocks[q], work);
+        const bool groups = leaf_in_groups(q % 3 == 0 ? 4 : (q % 3 == 1 ? 8 : 16), H->leaf_blocks[q], work);
         switch (q) {
         case 0:
-            if (groups) k_b_leaf_groups<4, false><<<dyn, 32 * kLeafWarps, 0, st>>>(D, W, d_tiles, H->tile_off);
+            if (groups) k_b_leaf_groups<4, false><<<dyn, 32 * kLeafWarps, 0, st>>>(D, W, d_tiles, H->tile_off, H->cursors);
             else k_b_leaf<4, false><<<dyn, 32 * kLeafWarps, 0, st>>>(D, W, d_tiles, H->tile_off, work);
             break;
         case 1:
-            if (groups) k_b_leaf_groups<8, false><<<dyn, 32 * kLeafWarps, 0, st>>>(D, W, d_tiles, H->tile_off);
+            if (groups) k_b_leaf_groups<8, false><<<dyn, 32 * kLeafWarps, 0, st>>>(D, W, d_tiles, H->tile_off, H->cursors);
             else k_b_leaf<8, false><<<dyn, 32 * kLeafWarps, 0, st>>>(D, W, d_tiles, H->tile_off, work);
             break;
         case 2: k_b_leaf<16, false><<<dyn, 32 * kLeafWarps, 0, st>>>(D, W, d_tiles, H->tile_off, work); break;
         case 3:
-            if (groups) k_b_leaf_groups<4, true><<<dyn, 32 * kLeafWarps, 0, st>>>(D, W, d_tiles, H->tile_off);
+            if (groups) k_b_leaf_groups<4, true><<<dyn, 32 * kLeafWarps, 0, st>>>(D, W, d_tiles, H->tile_off, H->cursors);
             else k_b_leaf<4, true><<<dyn, 32 * kLeafWarps, 0, st>>>(D, W, d_tiles, H->tile_off, work);
             break;
         case 4:
-            if (groups) k_b_leaf_groups<8, true><<<dyn, 32 * kLeafWarps, 0, st>>>(D, W, d_tiles, H->tile_off);
+            if (groups) k_b_leaf_groups<8, true><<<dyn, 32 * kLeafWarps, 0, st>>>(D, W, d_tiles, H->tile_off, H->cursors);
             else k_b_leaf<8, true><<<dyn, 32 * kLeafWarps, 0, st>>>(D, W, d_tiles, H->tile_off, work);
             break;
         default: k_b_leaf<16, true><<<dyn, 32 * kLeafWarps, 0, st>>>(D, W, d_tiles, H->tile_off, work);
