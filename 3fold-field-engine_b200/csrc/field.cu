@@ -2830,7 +2830,9 @@ __global__ void __launch_bounds__(32 * kLeafWarps, 5) k_b_leaf_groups(const RecD
     int64_t entries = 0;  // of all the group's recipes
     for (int j = lane; j < W.m; j += 32) entries += cursors[W.rec[j]];
     for (int o = 16; o > 0; o >>= 1) entries += __shfl_xor_sync(0xffffffffu, entries, o);
-    const int K = leaf_group_size<B>(total, entries);
+    // A batch's many recipes fill the waves, so groups pay up to longer lists than in one recipe (256 recipes: leaves
+    // 13.0 ms by leaf_group_size, 12.6 so).
+    const int K = entries > 8 * total ? 1 : (int)min(max(total / 3000, (int64_t)1), (int64_t)(B == 4 ? 8 : 4));
     if (K == 1) {
         for (int64_t g = gwarp; g < total; g += nwarps) {
             const int j = group_find(W, g);
@@ -3149,7 +3151,7 @@ int fb_batch_build_timed_device(void* batch, float* d_tiles, int64_t capacity, i
     for (int q = 0; q < kLeafGroups; ++q) {
         if (!H->leaf[q].m) continue;
         const Group& W = H->leaf[q];
-        const bool groups = leaf_in_groups(q % 3 == 0 ? 4 : (q % 3 == 1 ? 8 : 16), H->leaf_blocks[q], work);
+        const bool groups = !work && H->leaf_blocks[q] >= 6000;  // two blocks a group or more
         switch (q) {
         case 0:
             if (groups) k_b_leaf_groups<4, false><<<dyn, 32 * kLeafWarps, 0, st>>>(D, W, d_tiles, H->tile_off, H->cursors);
