@@ -137,10 +137,11 @@ void launch_bits(int grid, cudaStream_t stream, const uint8_t* mask, uint32_t* b
 // fifth).  A lower envelope built as a hull per column (one push, its pops and one walk step per voxel,
 // band hulls joined pairwise) took 107 (x) and 149 (zy) warp instructions per 32 voxels of the 512^3
 // obstacle grid (2000 boxes, 8 % filled), its loops diverging over the lanes; here it is 74 and 92, and
-// the work depends on the data only through votes: x 637 -> 402 us, zy 858 -> 545 us, the transform
-// 1515 -> 979 us (30 % random voxels 1640 -> 772, one box edge or ball far from most voxels 0 - 40 %
-// less).  The hulls remain faster only where a smooth surface lies hundreds of voxels away from most of
-// the grid along its diagonal (a half-space x + y + z < 350 of 512^3: 984 against 1584 us).
+// the work depends on the data only through votes: x 638 -> 395 us, zy 851 -> 559 us, the transform
+// 1515 -> 986 us (30 % random voxels 1640 -> 773, one box or ball far from most voxels 14 - 18 % less).
+// The hulls remain faster where a smooth surface lies hundreds of voxels away from most of the grid along
+// its diagonal (half-spaces of 512^3: x + y + z < 350 986 against 1273 us, < 700 1138 / 1414, z < 100
+// 1058 / 1123; a shell of radius 240 1472 / 1560).
 // ------------------------------------------------------------------------------------------
 constexpr int kWarps = 8;
 constexpr int kThreads = 32 * kWarps;
@@ -223,7 +224,7 @@ __device__ __forceinline__ void group_minima(const float* __restrict__ rows, flo
     }
 }
 
-// The strips [g0, g1) of one warp in ascending order, an axis of n rows: store(strip, g) for each, columns
+// The strips [g0, g1) of one warp, an axis of n rows: store(strip, g) for each, columns
 // inside the grid.  All rows and minima of the CTA are in place (the caller has synchronised); `mins`
 // holds kNear groups of kPadValue before the first and after the last group, which therefore fail every
 // test.  Columns outside the grid hold kPadValue in every row and take no part in the decisions.
@@ -232,7 +233,12 @@ __device__ __forceinline__ void group_minima(const float* __restrict__ rows, flo
 // ended there hands the place to the next one, which begins with that group instead of its own.  The
 // site of an output never lies before the previous output's, so groups before the least such place of
 // the columns are left out, and groups beyond a column's own are tested at the strip's last output.
-template <int LD, typename Store>
+// kLastFirst: the last strip goes before the others, whose groups then end at its first output's minimum, and
+// groups that can only gain on a column's last or first output are tried on that output alone before they are
+// taken.  Smooth masks far away leave tens of groups within the bounds of 32 columns; the x pass, 512^3:
+// half-spaces x + y + z < 350 and < 700 968 -> 699 and 691 -> 584 us, z < 100 564 -> 450, boxes unchanged.  In
+// the zy pass it gains a twelfth there and costs the boxes a twentieth (its registers spill).
+template <int LD, bool kLastFirst, typename Store>
 __device__ __forceinline__ void strips(const float* __restrict__ rows, const float* __restrict__ mins,
                                        const float* __restrict__ low, int n, int g0, int g1, bool in, Store store) {
     const int lane = threadIdx.x & 31;
@@ -243,9 +249,13 @@ __device__ __forceinline__ void strips(const float* __restrict__ rows, const flo
     float2 ahead = make_float2((float)kGroup, (float)kGroup), behind = make_float2(-(float)kGroup, -(float)kGroup);
     asm volatile("" : "+f"(origin.x), "+f"(origin.y), "+f"(back2.x), "+f"(back2.y));
     asm volatile("" : "+f"(ahead.x), "+f"(ahead.y), "+f"(behind.x), "+f"(behind.y));
+    const int middle = kLastFirst ? __popc(__ballot_sync(0xffffffffu, in)) >> 1 : 0;  // of the columns inside the grid
     int seed = 0;   // offset of the group to begin with
     int least = 0;  // groups before it hold no minimum of this and later strips
-    for (int g = g0; g < g1; ++g) {
+    int greatest = ng;  // groups behind it hold none of the strips before the last one
+    const bool ends = kLastFirst && g1 - g0 > 5;  // worth it
+    for (int t = ends ? g0 - 1 : g0; t < (ends ? g1 - 1 : g1); ++t) {
+        const int g = kLastFirst && t < g0 ? g1 - 1 : t;
         const float* const own = rows + g * kGroup * LD + lane;
         const float* const near = mins + g * 32 + lane;
         Strip s;
@@ -278,10 +288,11 @@ __device__ __forceinline__ void strips(const float* __restrict__ rows, const flo
             float top = warp_max(most);  // of all columns
             const int skip = seed == 0 ? kNear : -1;
             int at = seed == 0 ? -kNear : ng;  // a group no later than the last output's minimum, as an offset
+            int first = seed == 0 ? kNear : -ng;  // and one no earlier than the first output's
             const int o0 = abs(lane - g), o1 = abs(lane + 32 - g);
             const float d0 = fmaxf((float)(kGroup * o0 - (kGroup - 1)), 0.f), d1 = fmaxf((float)(kGroup * o1 - (kGroup - 1)), 0.f);
-            float b0 = o0 > skip && lane >= least && lane < ng ? fmaf(d0, d0, low[lane]) : kPadValue;
-            float b1 = o1 > skip && lane + 32 >= least && lane + 32 < ng ? fmaf(d1, d1, low[lane + 32]) : kPadValue;
+            float b0 = o0 > skip && lane >= least && (!kLastFirst || lane <= greatest) && lane < ng ? fmaf(d0, d0, low[lane]) : kPadValue;
+            float b1 = o1 > skip && lane + 32 >= least && (!kLastFirst || lane + 32 <= greatest) && lane + 32 < ng ? fmaf(d1, d1, low[lane + 32]) : kPadValue;
             int next = g + seed;
             bool begin = seed != 0;
             for (;;) {  // each turn takes one group out
@@ -303,17 +314,38 @@ __device__ __forceinline__ void strips(const float* __restrict__ rows, const flo
                 const float e = beyond ? dl : d;
                 const float lim = beyond && in ? s.value(kGroup - 1) : most;
                 if (!begin && !__any_sync(0xffffffffu, near[o * 32] < fmaf(-e, e, lim))) continue;
+                if (kLastFirst && !begin) {
+                    const bool may = near[o * 32] < fmaf(-e, e, lim);
+                    const bool before = o < first;
+                    const float* const col = own + o * (kGroup * LD);
+                    const float x = beyond ? D + (float)(kGroup - 1) : D, end = beyond ? s.value(kGroup - 1) : s.value(0);
+                    float2 q = make_float2(x, x - 1.f);
+                    float v = kPadValue;
+#pragma unroll
+                    for (int i = 0; i < kGroup; i += 2) {
+                        const float2 c = __ffma2_rn(q, q, make_float2(col[i * LD], col[(i + 1) * LD]));
+                        v = min3(v, c.x, c.y);
+                        q = __fadd2_rn(q, back2);
+                    }
+                    if (!__any_sync(0xffffffffu, may && in && (!(beyond || before) || v < end))) continue;
+                }
                 begin = false;
                 const float was = s.a[kGroup - 1];
+                [[maybe_unused]] const float was0 = s.a[0];
                 s.group<LD>(own + o * (kGroup * LD), make_float2(D, D - 1.f), back2);
                 if (s.a[kGroup - 1] < was) at = o;
+                if (kLastFirst && s.a[0] < was0) first = o;
                 most = in ? s.largest() : 0.f;
                 top = warp_max(most);
             }
             least = g + __reduce_min_sync(0xffffffffu, in ? at : ng);
-            seed = __shfl_sync(0xffffffffu, at, 0) - 1;
+            seed = __shfl_sync(0xffffffffu, at, middle) - 1;
             if (seed >= -kNear - 1 && seed <= kNear) seed = 0;
+            if (kLastFirst && t < g0) greatest = g + __reduce_max_sync(0xffffffffu, in ? first : -ng);
+        } else if (kLastFirst && t < g0) {
+            greatest = g + kNear;
         }
+        if (kLastFirst && t < g0) seed = least = 0;
         if (in) store(s, g);
     }
 }
@@ -449,7 +481,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_edt_zy(const uint32_t* __restri
     __syncwarp();
     group_minima<kZyLd>(rows, mins, low, g0, g1);
     __syncthreads();
-    strips<kZyLd>(rows, mins, low, ny, g0, g1, in, [&](const Strip& s, int gr) { put<float>(s, out, nz, ny, gr); });
+    strips<kZyLd, false>(rows, mins, low, ny, g0, g1, in, [&](const Strip& s, int gr) { put<float>(s, out, nz, ny, gr); });
 }
 
 // x pass.  grid = (W, ny, polarities), block = kThreads, dynamic smem = pass_smem_bytes(nx, 32).
@@ -496,7 +528,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_edt_x(const float* g, int32_t* 
     __syncthreads();
     int32_t* const dst = out + col + lane;
     const bool in = lane < live;
-    strips<32>(rows, mins, low, nx, g0, g1, in, [&](const Strip& s, int gr) { put<int32_t>(s, dst, stride, nx, gr); });
+    strips<32, true>(rows, mins, low, nx, g0, g1, in, [&](const Strip& s, int gr) { put<int32_t>(s, dst, stride, nx, gr); });
 }
 
 // Correctly rounded signed distance of one voxel from its two squared distances, the reference's
