@@ -335,7 +335,10 @@ __device__ __forceinline__ double write_triangle(int64_t at, int64_t end, const 
 // signs, the emit pass at the counts); index arithmetic is 32-bit with the block edge a constant;
 // corner signs are bytes; loops come from a table except where a face needs its decision; and the emit
 // pass hands out triangles, not cubes, to the threads.  27 balls on 256 x 256 x 250: count 301 -> 61 us,
-// emit 414 -> 60 us.
+// emit 414 -> 60 us.  Blocks of more than kMcDense triangles, or two a cube, have enough for all threads either
+// way: a cube then goes to one thread, which forms each vertex of its loops once instead of once a triangle
+// (128^3 noise, blocks of 8: emit 1759 -> 750 us, 1256 when every cube went to one; of 16 2464 -> 1047, 1302).
+constexpr int kMcDense = 1024;
 constexpr int kMcItems = 1024;  // triangles (or undecided cubes) handed out at a time
 constexpr size_t kMcStatic = kMcItems * sizeof(uint2) + 1024;  // k_mc's static shared memory is below it
 static_assert(kMcItems >= kMcThreads * kMaxTableTris, "one round of cubes must fit");
@@ -483,6 +486,7 @@ __global__ void __launch_bounds__(kMcThreads) k_mc(McField F, const int32_t* __r
         const int C = B + 1, ncube = C * C * C;
         int run = 0, items = 0, tri_sum = 0;
         double vol = 0.0;
+        const bool whole_cubes = kEmit && tcount[sa + 1] - tcount[sa] > min(kMcDense, 2 * ncube);
         auto corners = [&](int r, double* g) {
 #pragma unroll
             for (int c = 0; c < 8; ++c) g[c] = val(r + ((c & 1) ? R * R : 0) + ((c & 2) ? R : 0) + ((c & 4) ? 1 : 0));
@@ -538,13 +542,17 @@ __global__ void __launch_bounds__(kMcThreads) k_mc(McField F, const int32_t* __r
                     int c = 0;
                     while (c < len && (edge_faces(el[c]) & twice)) ++c;
                     if (c == len) c = 0;
-                    for (int i2 = 1; i2 + 1 < len; ++i2) {
-                        int64_t vid[3];
-                        float q[3][3];
-                        edge_point(m, el[c], vid[0], q[0]);
-                        edge_point(m, el[(c + i2 + 1) % len], vid[1], q[1]);
-                        edge_point(m, el[(c + i2) % len], vid[2], q[2]);
+                    int64_t vid[3];
+                    float q[3][3];
+                    edge_point(m, el[c], vid[0], q[0]);
+                    edge_point(m, el[c + 1 < len ? c + 1 : c + 1 - len], vid[2], q[2]);
+                    for (int i2 = 2; i2 < len; ++i2) {  // each vertex of the loop once
+                        const int j = c + i2 < len ? c + i2 : c + i2 - len;
+                        edge_point(m, el[j], vid[1], q[1]);
                         vol += write_triangle(to++, end, vid, q, faces, err);
+                        vid[2] = vid[1];
+#pragma unroll
+                        for (int a = 0; a < 3; ++a) q[2][a] = q[1][a];
                     }
                 }
             }
@@ -584,6 +592,8 @@ __global__ void __launch_bounds__(kMcThreads) k_mc(McField F, const int32_t* __r
                         corners(r, g);
                         ntri = cube_triangles(cube_loops(g));
                         n_items = ntri ? kMaxTableTris + 1 : 0;  // marks one item for the whole cube
+                    } else if (kEmit && whole_cubes && ntri) {
+                        n_items = kMaxTableTris + 1;
                     }
                 }
             }
