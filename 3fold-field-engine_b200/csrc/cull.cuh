@@ -307,7 +307,7 @@ __device__ int warp_walk_ball(int n_in, const FbInsn* __restrict__ chain, const 
         float agg = op == CH_UNION ? 3.0e38f : -3.0e38f;
         int j = n_in;
         const int n0 = n;
-        for (int b = i; b < n_in; b += 32 * kBallChunks) {
+        for (int b = i, chunks = 1; b < n_in; b += 32 * chunks, chunks = kBallChunks) {  // a short run loads one
             Elem E[kBallChunks];
 #pragma unroll
             for (int c = 0; c < kBallChunks; ++c) {
@@ -315,15 +315,15 @@ __device__ int warp_walk_ball(int n_in, const FbInsn* __restrict__ chain, const 
                 E[c].op = -1;
                 E[c].k = E[c].lo = E[c].hi = 0.f;
                 E[c].ent = 0u;
-                if (e < n_in) E[c] = load_elem(nullptr, e, chain, primf, cx, cy, cz, R, eps, true, balls);
+                if (c < chunks && e < n_in) E[c] = load_elem(nullptr, e, chain, primf, cx, cy, cz, R, eps, true, balls);
             }
-            int end = min(b + 32 * kBallChunks, n_in);
+            int end = min(b + 32 * chunks, n_in);
             bool stopped = false;
 #pragma unroll
             for (int c = 0; c < kBallChunks; ++c) {
                 const int e = b + 32 * c + lane;
                 const bool same = e == i || (E[c].op == op && runnable(E[c].op, E[c].k));
-                const unsigned stop = __ballot_sync(0xffffffffu, e < n_in && !same);
+                const unsigned stop = __ballot_sync(0xffffffffu, c < chunks && e < n_in && !same);
                 if (stop && !stopped) {
                     stopped = true;
                     end = b + 32 * c + __ffs(stop) - 1;

@@ -669,7 +669,7 @@ __device__ __forceinline__ void subset_walk(const uint32_t* ent, int m, const Fb
 
 // Where threads' blocks do not share a subset (superblocks of 1 or 8 blocks, several to a warp, or a
 // subset that did not fit): each block culls its superblock's list itself (seq_walk).
-__device__ __noinline__ void classify_alone(const Geo& G, const BlockAt& A, const FbPrim* __restrict__ prims,
+__device__ __forceinline__ void classify_alone_body(const Geo& G, const BlockAt& A, const FbPrim* __restrict__ prims,
                                             const PrimF* __restrict__ primf, const FbInsn* __restrict__ chain,
                                             const uint32_t* __restrict__ plist, int plen, int32_t* __restrict__ kind,
                                             float* __restrict__ cma, int32_t* __restrict__ blk_off,
@@ -728,6 +728,43 @@ __device__ __noinline__ void classify_alone(const Geo& G, const BlockAt& A, cons
         }
         blk_len[A.b] = len_b;  // -1: the leaf pass culls the block itself
     }
+}
+
+__device__ __noinline__ void classify_alone(const Geo& G, const BlockAt& A, const FbPrim* __restrict__ prims,
+                                            const PrimF* __restrict__ primf, const FbInsn* __restrict__ chain,
+                                            const uint32_t* __restrict__ plist, int plen, int32_t* __restrict__ kind,
+                                            float* __restrict__ cma, int32_t* __restrict__ blk_off,
+                                            int32_t* __restrict__ blk_len, uint32_t* __restrict__ blk_pool,
+                                            int64_t blk_cap, int* __restrict__ cursor) {
+    classify_alone_body(G, A, prims, primf, chain, plist, plen, kind, cma, blk_off, blk_len, blk_pool, blk_cap, cursor);
+}
+
+// Superblocks of 1 or 8 blocks: every block by itself, in a kernel of its own.  Behind the bricks' branch their
+// walk is a call out of line beside the bricks' registers and shared memory (512^3 of 3000 elements in blocks of
+// 16: 1230 us, 1082 here; 64^3 of 2 elements 10.9 and 7.9).  A batch keeps one kernel for all of its recipes: two
+// after one another left the GPU idle at the end of each (20 recipes 3540 -> 3710 us).
+__device__ __forceinline__ void classify_block_alone(const Geo& G, const FbPrim* __restrict__ prims,
+                                                     const PrimF* __restrict__ primf, const FbInsn* __restrict__ chain,
+                                                     const uint32_t* __restrict__ pool,
+                                                     const int64_t* __restrict__ sb_off,
+                                                     const int32_t* __restrict__ sb_len, int32_t* __restrict__ kind,
+                                                     float* __restrict__ cma, int32_t* __restrict__ blk_off,
+                                                     int32_t* __restrict__ blk_len, uint32_t* __restrict__ blk_pool,
+                                                     int64_t blk_cap, int* __restrict__ cursor, int64_t t) {
+    const int S = G.S;
+    const int T = threads_per_super(S);  // 1 or 8
+    const int64_t s_id = t / T;
+    const int local = (int)(t % T);
+    const int sz = (int)(s_id % G.nsz), sy = (int)((s_id / G.nsz) % G.nsy), sx = (int)(s_id / ((int64_t)G.nsz * G.nsy));
+    BlockAt A;
+    A.bi = sx * S + local / (S * S);
+    A.bj = sy * S + (local / S) % S;
+    A.bk = sz * S + local % S;
+    const bool any = s_id < G.nsuper;
+    A.valid = any && A.bi < G.nbx && A.bj < G.nby && A.bk < G.nbz;
+    A.b = ((int64_t)A.bi * G.nby + A.bj) * G.nbz + A.bk;
+    classify_alone_body(G, A, prims, primf, chain, any ? pool + sb_off[s_id] : pool, any ? sb_len[s_id] : 0, kind, cma,
+                        blk_off, blk_len, blk_pool, blk_cap, cursor);
 }
 
 // Thread-per-block classification of a chain recipe: thread t of the superblock-major order --
@@ -870,6 +907,21 @@ __global__ void __launch_bounds__(128, 6) k_classify_blocks(Geo G, const FbPrim*
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     classify_block(G, prims, primf, chain, pool, sb_off, sb_len, kind, cma, blk_off, blk_len, blk_pool, blk_cap, cursor,
                    t, s_sub[threadIdx.x >> 5]);
+}
+
+__global__ void __launch_bounds__(128, 6) k_classify_alone(Geo G, const FbPrim* __restrict__ prims,
+                                                           const PrimF* __restrict__ primf,
+                                                           const FbInsn* __restrict__ chain,
+                                                           const uint32_t* __restrict__ pool,
+                                                           const int64_t* __restrict__ sb_off,
+                                                           const int32_t* __restrict__ sb_len,
+                                                           int32_t* __restrict__ kind, float* __restrict__ cma,
+                                                           int32_t* __restrict__ blk_off, int32_t* __restrict__ blk_len,
+                                                           uint32_t* __restrict__ blk_pool, int64_t blk_cap,
+                                                           int* __restrict__ cursor) {
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    classify_block_alone(G, prims, primf, chain, pool, sb_off, sb_len, kind, cma, blk_off, blk_len, blk_pool, blk_cap, cursor,
+                         t);
 }
 
 // ------------------------------------------------------------------------------------ general programs
@@ -2523,9 +2575,13 @@ int classify_impl(const FbGeom& g, const FbPrim* prims, int n_prims, const FbIns
         FB_LAUNCH();
         FB_CUDA(cudaMemsetAsync(S.misc, 0, 256, st));
         // a thread per block: its own cull of the superblock list, kept for the active blocks
-        k_classify_blocks<<<fb_div_up(G.nsuper * threads_per_super(G.S), 128), 128, 0, st>>>(
-            G, prims, S.primf, chain, S.pool, S.off + G.ncoarse, S.len + G.ncoarse, kind, cma, S.blk_off, S.blk_len,
-            S.blk_pool, P.blk_cap, S.misc + 2);
+        const unsigned ctas = fb_div_up(G.nsuper * threads_per_super(G.S), 128);
+        if (G.S >= 4)
+            k_classify_blocks<<<ctas, 128, 0, st>>>(G, prims, S.primf, chain, S.pool, S.off + G.ncoarse, S.len + G.ncoarse,
+                                                    kind, cma, S.blk_off, S.blk_len, S.blk_pool, P.blk_cap, S.misc + 2);
+        else
+            k_classify_alone<<<ctas, 128, 0, st>>>(G, prims, S.primf, chain, S.pool, S.off + G.ncoarse, S.len + G.ncoarse,
+                                                   kind, cma, S.blk_off, S.blk_len, S.blk_pool, P.blk_cap, S.misc + 2);
     } else {
         k_cull_program<<<fb_div_up(G.nsuper, kProgWarps), 32 * kProgWarps, 0, st>>>(
             G, prims, S.primf, chain, n_chain, S.pool, P.pool_super, P.cap_super, S.off + G.ncoarse, S.len + G.ncoarse);
