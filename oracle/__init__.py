@@ -284,6 +284,10 @@ def tiles_program(prims, prog, meta, active_ids):
 
 
 # ----------------------------------------------------------------------------------------- reference libs
+class NotBuilt(RuntimeError):
+    """A reference library that was not compiled on this machine (its sources are absent here)."""
+
+
 def ref_library(name):
     """A reference CPU library compiled from the reference's own sources into oracle/_ref/
     (``pack``, ``csg_batch`` or ``mesh_sdf``); None when it was not built on this machine."""
@@ -299,7 +303,7 @@ def ref_classify_dense(dense, pitch, block, nthreads=0):
     import math
     L = ref_library("mesh_sdf")
     if L is None:
-        raise RuntimeError("oracle/_ref/libref_mesh_sdf.so is not built")
+        raise NotBuilt("oracle/_ref/libref_mesh_sdf.so is not built")
     P, I64 = ct.c_void_p, ct.c_int64
     L.meshsdf_classify_cpu.argtypes = [P, I64, I64, I64, I64, ct.c_float, P, ct.c_int]
     L.meshsdf_classify_cpu.restype = ct.c_int
@@ -329,7 +333,7 @@ def ref_pack(samples, threshold=512):
     """The reference's adaptive_pack compiled from pack.cpp: (nodes, payload)."""
     L = ref_library("pack")
     if L is None:
-        raise RuntimeError("oracle/_ref/libref_pack.so is not built")
+        raise NotBuilt("oracle/_ref/libref_pack.so is not built")
     L.adaptive_pack.argtypes = [ct.c_void_p, ct.c_void_p, ct.c_int]
     L.adaptive_pack.restype = ct.c_void_p
     for name in ("adaptive_nodes", "adaptive_samples"):
@@ -505,7 +509,7 @@ def ref_mesh_field(V, T, origin, pitch, jitter, shape, surface_correction=True, 
     stats int64[4])."""
     L = ref_library("mesh_sdf")
     if L is None:
-        raise RuntimeError("oracle/_ref/libref_mesh_sdf.so is not built")
+        raise NotBuilt("oracle/_ref/libref_mesh_sdf.so is not built")
     P, I64, D, I = ct.c_void_p, ct.c_int64, ct.c_double, ct.c_int
     L.meshsdf_field_cpu.argtypes = [P, I64, P, I64, D, D, D, D, D, D, I64, I64, I64, I, I, P, P, P, P, P]
     L.meshsdf_field_cpu.restype = I
