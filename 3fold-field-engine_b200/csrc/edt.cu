@@ -26,6 +26,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <mutex>
+#include <type_traits>
 #include <new>
 
 namespace {
@@ -356,8 +357,8 @@ __device__ __forceinline__ void put(const Strip& s, T* __restrict__ out, int64_t
     T* p = out + (int64_t)(g * kGroup) * stride;
     const int valid = n - g * kGroup;
     auto one = [&](int k) {
-        if (sizeof(T) == 4 && T(0.5f) == T(0)) *p = (T)s.integer(k);
-        else *p = (T)s.value(k);
+        if constexpr (std::is_same_v<T, int32_t>) *p = s.integer(k);
+        else *p = s.value(k);
         p += stride;
     };
     if (valid >= kGroup) {
@@ -634,7 +635,6 @@ int enqueue(const uint8_t* d_mask, int nx, int ny, int nz, int paired, int sites
         launch_x(g, out_sq, nx, ny, nz, W, 1, stream);
     }
     FB_LAUNCH();
-    (void)size;
     return FB_OK;
 }
 
@@ -669,7 +669,7 @@ struct Pair {
 // its own pool allocator, a real-time loop that must never hit the implicit synchronisation of
 // cudaMalloc/cudaFree, a plugin whose host forbids allocation calls); they can pass input and
 // output buffers but not scratch.  For them the squared EDT below keeps its scratch (bit words
-// and the int32 intermediate) in a fixed array compiled into this library.
+// and the float32 intermediate) in a fixed array compiled into this library.
 //
 // Limit: at most kNoAllocVoxels = 2^20 voxels and 512 per axis -- the reference's own EDT
 // contract (src/field_engine/edt_native_large_v1/edt.cu:34-37).  Every GPU that loads this
@@ -677,7 +677,7 @@ struct Pair {
 // ---------------------------------------------------------------------------------------------
 constexpr int64_t kNoAllocVoxels = int64_t(1) << 20;
 // bit words: nx*ny*ceil(nz/32) <= voxels/32 + nx*ny <= 2^15 + 512*512; plus 256 B of counters and
-// one int32 intermediate per voxel
+// one float32 intermediate per voxel
 constexpr int64_t kNoAllocBitBytes = ((kNoAllocVoxels / 32 + 512 * 512) * 4 + 255) / 256 * 256;
 constexpr int64_t kNoAllocScratchBytes = 256 + kNoAllocBitBytes + kNoAllocVoxels * 4;
 static __device__ __align__(256) unsigned char g_edt_noalloc_scratch[kNoAllocScratchBytes];

@@ -440,7 +440,6 @@ __global__ void k_cull(Geo G, const FbInsn* __restrict__ chain, const PrimF* __r
 }
 
 
-// ------------------------------------------------------------------------------------ localisation
 // ------------------------------------------------------------------------------------ classify
 // float64 value of a block list at a world point (guard-band recheck).
 __device__ __noinline__ double list_eval_d(const uint32_t* __restrict__ list, int n, const FbInsn* __restrict__ chain,
@@ -3299,14 +3298,6 @@ void fb_batch_destroy(void* batch) noexcept {
     delete H;
 }
 
-}  // extern "C"
-
-namespace {
-
-}  // namespace
-
-extern "C" {
-
 // Scratch bytes of one analytic build (classify + leaf) for this geometry and program size.
 int64_t fb_field_scratch_bytes(const FbGeom* g, int32_t n_prims, int32_t n_chain) {
     if (!g || !geom_ok(*g) || n_prims < 1 || n_chain < 1) return -1;
@@ -3315,7 +3306,7 @@ int64_t fb_field_scratch_bytes(const FbGeom* g, int32_t n_prims, int32_t n_chain
 }
 
 // Classification + compaction of an analytic recipe.  mode 1: `chain` is the left-deep chain
-// (CH_* ops, culled); mode 0: `chain` is a general postfix program (OP_* ops, float64, no culling).
+// (CH_* ops, culled); mode 0: `chain` is a general postfix program (OP_* ops, float64, pruned per region).
 // Writes kind[n_blocks], corner_min_abs[n_blocks], active[<= n_blocks] ascending and count[0].
 int fb_field_classify_device(const FbGeom* g, const FbPrim* d_prims, int32_t n_prims, const FbInsn* d_chain,
                              int32_t n_chain, int32_t mode, int32_t* d_kind, float* d_cma, int32_t* d_active,

@@ -13,7 +13,7 @@ leaf's own record, so the device evaluates ``value = s * f(A x + t) - off`` per 
 primitives.  Hard (k == 0) unions, intersections and subtractions of unions are re-associated
 into a left-deep chain ``acc = op_i(acc, prim_i)`` -- exact for min/max -- which is what the
 GPU's Lipschitz culling works on; smooth operators are never re-associated.  Trees that do not
-reduce to a chain run as a general postfix program (every primitive at every voxel).
+reduce to a chain run as a general postfix program, pruned per region to what can matter there.
 """
 from __future__ import annotations
 

@@ -116,8 +116,9 @@ int64_t fb_edt_noalloc_capacity(int64_t* max_voxels);
  * k_classify_testfalt :129-164, host compaction np.where :277, k_eval_tile_testfalt :167-190 -- for any
  * compiled recipe.  mode 1: d_chain is the culled chain form; mode 0: a postfix program (float64).
  * Outputs: kind[n_blocks] (-1/0/+1), corner_min_abs[n_blocks], ascending active ids, count[0],
- * tiles[count][block^3] (C order li, lj, lk).  fb_field_leaf_device reuses the lists that
- * fb_field_classify_device left in d_scratch for the same recipe and grid. */
+ * tiles[count][block^3] (C order li, lj, lk).  fb_field_leaf_device reuses what fb_field_classify_device
+ * left in d_scratch for the same recipe, grid and mode (the lists, in mode 0 the pruned programs, and the
+ * primitives' float32 mirror): it needs that scratch in both modes. */
 int64_t fb_field_scratch_bytes(const fb_geom* g, int32_t n_prims, int32_t n_chain);
 int fb_field_classify_device(const fb_geom* g, const fb_prim* d_prims, int32_t n_prims, const fb_insn* d_chain,
                              int32_t n_chain, int32_t mode, int32_t* d_kind, float* d_cma, int32_t* d_active,
@@ -401,7 +402,8 @@ int fb_clearance_mask_device(const uint8_t* d_occ, const double* d_edt_mm, int64
  * columns ascending, -kond off the diagonal, the diagonal summed in scipy's COO order).  The
  * capacities are the lengths of the caller's u / v / kond (edges), indptr (nodes + 1) and indices /
  * data (entries) buffers: outputs beyond them are not written, and a null pointer is accepted only
- * where its capacity is 0.  At most (2^31 - 1) / 7 cells (status 1 beyond);
+ * where its capacity is 0.  The emit call takes the cells' occupancy from what the count call left in the
+ * scratch (d_occ is required but not read again).  At most (2^31 - 1) / 7 cells (status 1 beyond);
  * fb_lattice_scratch_bytes returns -1 for such shapes. */
 int64_t fb_lattice_scratch_bytes(int nx, int ny, int nz);
 int fb_lattice_count_device(const uint8_t* d_occ, int nx, int ny, int nz, int32_t* d_totals, void* d_scratch,
