@@ -77,9 +77,10 @@ class RecipeQueries:
         import torch
         a = self._accel
         scratch, nscratch = None, 0
+        grid, dims = (a[3].ctypes.data, a[4].ctypes.data) if a else (None, None)
         if a is not None and pts.shape[0] > 0:
-            nbytes = int(self.lib.fb_query_scratch_bytes_h(a[3].ctypes.data, a[4].ctypes.data, pts.shape[0],
-                                                           1 if grad is not None else 0, float(h)))
+            nbytes = int(self.lib.fb_query_scratch_bytes_h(grid, dims, pts.shape[0], 1 if grad is not None else 0,
+                                                           float(h)))
             if nbytes > 0:
                 nscratch = nbytes
                 if alloc is not None:
@@ -88,8 +89,7 @@ class RecipeQueries:
                     scratch = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
                     if isinstance(stream, torch.cuda.Stream):  # freed only after that stream's kernels
                         scratch.record_stream(stream)
-        args = (a[0], a[1], a[2], a[3].ctypes.data, a[4].ctypes.data, *a[5]) if a else (None,) * 5 + (None, None,
-                                                                                                     None, None, 0, 0)
+        args = (a[0], a[1], a[2], grid, dims, *a[5]) if a else (None,) * 9 + (0, 0)
         st = self.lib.fb_query_points_device(self.primf.data_ptr(), self.chain.data_ptr(), self.n_chain, self._walk,
                                              *args, pts.data_ptr(), pts.shape[0], float(h),
                                              value.data_ptr() if value is not None else None,
