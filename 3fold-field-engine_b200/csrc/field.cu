@@ -740,7 +740,7 @@ __device__ __noinline__ void classify_alone(const Geo& G, const BlockAt& A, cons
 
 // Superblocks of 1 or 8 blocks: every block by itself, in a kernel of its own.  Behind the bricks' branch their
 // walk is a call out of line beside the bricks' registers and shared memory (512^3 of 3000 elements in blocks of
-// 16: 1230 us, 1082 here; 64^3 of 2 elements 10.9 and 7.9).  A batch keeps one kernel for all of its recipes: two
+// 16: 1230 us, 1093 here; 64^3 of 2 elements 10.9 and 7.9).  A batch keeps one kernel for all of its recipes: two
 // after one another left the GPU idle at the end of each (20 recipes 3540 -> 3710 us).
 __device__ __forceinline__ void classify_block_alone(const Geo& G, const FbPrim* __restrict__ prims,
                                                      const PrimF* __restrict__ primf, const FbInsn* __restrict__ chain,
